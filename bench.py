@@ -61,7 +61,7 @@ WORKLOADS = {
 }
 # reference latencies read from its published chart (Hygon DCU gfx928), microseconds
 PUBLISHED_US = {"final1": 207, "final2": 367, "final3": 724, "final4": 654, "final5": 593, "final6": 133}
-ALGO_ARG = {"ref": -1, "4x3": 0, "2x3": 1, "fused": 2, "auto": 3, "row": 4}
+ALGO_ARG = {"ref": -1, "4x3": 0, "2x3": 1, "fused": 2, "auto": 3, "row": 4, "direct": 5}
 SERVE_WORKLOADS = {
     "cfg5": "serving: 16 resident 3x3 pad-1 layers (C,K in {64..512}, H=W in {7..112}), N ~ U{1..64}, "
             "Poisson arrivals swept over multiples of the plain per-request capacity, 40 GiB workspace budget",
@@ -324,6 +324,7 @@ def algorithmic_work(name, geo, m_bytes_per_value=None):
       fused2x3          x + U + y;                   FLOPs 2*16*P*C*K
       row4x3            x + U1 (2*18*C*K) + y;       FLOPs 2*18*RT*C*K over
                         RT = N*OH*ceil(OW/4) row tiles
+      direct3x3         x + U9 (2*9*C*K) + y;        FLOPs 2*9*N*OH*OW*C*K
     M is counted at `m_bytes_per_value` bytes per value (3 for the 24-bit
     F(4x3) default, stored in blocks of 64 tiles; 4 for fp32, 2 for fp16).
     Returns (algorithmic bytes, design bytes, FLOPs, formula)."""
@@ -343,6 +344,9 @@ def algorithmic_work(name, geo, m_bytes_per_value=None):
         rt = n * oh * math.ceil(ow / 4)
         u1 = 2.0 * 18 * c * k
         return x_b + u1 + y_b, x_b + u1 + y_b, 2.0 * 18 * rt * c * k, "x + U1 + y"
+    if name == "direct3x3":
+        u9 = 2.0 * 9 * c * k
+        return x_b + u9 + y_b, x_b + u9 + y_b, 2.0 * 9 * n * oh * ow * c * k, "x + U9 + y"
     if name == "input_transform":
         return x_b + v_b, x_b + v_b, 0.0, "x + V"
     if name == "tile_scale":
@@ -369,7 +373,8 @@ def roofline_for(name, wg, geo, ms, pk, pk_kind, m_bytes_per_value=None):
                     "peak_source": f"{pk_kind} HBM copy"})
     E = (geo[5] + 2) ** 2
     out["algorithmic_per_launch"] = f"{byts / 1e6:.1f} MB ({formula})" + (
-        (f", {flops / 1e9:.2f} GFLOP (2*18*RT*C*K)" if name == "row4x3" else f", {flops / 1e9:.2f} GFLOP (2*{E}*P*C*K)")
+        f", {flops / 1e9:.2f} GFLOP (" + {"row4x3": "2*18*RT*C*K", "direct3x3": "2*9*N*OH*OW*C*K"}.get(
+            name, f"2*{E}*P*C*K") + ")"
         if flops else "")
     out["algorithmic_bytes"] = byts
     out["design_bytes"] = design
@@ -384,12 +389,14 @@ def roofline_for(name, wg, geo, ms, pk, pk_kind, m_bytes_per_value=None):
 def step_roofline(geo, algo, wg, ms_step, pk, pk_kind):
     """Whole-step roofline of one call: the bytes no design can avoid (x, the
     transformed filter U, y) and the algorithm's tensor work (its Winograd
-    GEMM FLOPs), against the measured time per step."""
+    or direct GEMM FLOPs), against the measured time per step."""
     n, c, h, w, k, m = geo
     tiles = n * math.ceil(h / m) * math.ceil(w / m)
     E = (m + 2) ** 2
     x_b, y_b = 2.0 * n * c * h * w, 2.0 * n * k * h * w
-    if algo == wg.ALGO_4X3_ROW:
+    if algo == wg.ALGO_DIRECT:
+        u_b, flops = 2.0 * 9 * c * k, 2.0 * 9 * n * h * w * c * k
+    elif algo == wg.ALGO_4X3_ROW:
         u_b, flops = 2.0 * 18 * c * k, 2.0 * 18 * n * h * math.ceil(w / 4) * c * k
     else:
         u_b, flops = 2.0 * E * c * k, 2.0 * E * tiles * c * k
@@ -533,7 +540,7 @@ def our_arm(args):
         ops.append(wg.Conv2d(prob, opts))
     stream = torch.cuda.current_stream(device)
     sptr = stream.cuda_stream
-    algo = ops[0].algo
+    algo = wg.ALGO_DIRECT if ops[0].direct else ops[0].algo   # what the calls run
 
     for i in range(args.warmup):
         ops[i % nsets](sptr)
@@ -1106,7 +1113,7 @@ def suite_arm(args):
             b.record()
             torch.cuda.synchronize()
             us = a.elapsed_time(b) / args.steps * 1e3
-            row[label] = {"algo": wg.ALGO_NAMES[op.algo], "us": us, "tflops": fl / (us * 1e-6) / 1e12}
+            row[label] = {"algo": wg.ALGO_NAMES[wg.ALGO_DIRECT if op.direct else op.algo], "us": us, "tflops": fl / (us * 1e-6) / 1e12}
             op.destroy()
         us = time_cudnn(torch, x, wt, args.steps, args.warmup) * 1e3
         row["cudnn"] = {"us": us, "tflops": fl / (us * 1e-6) / 1e12}

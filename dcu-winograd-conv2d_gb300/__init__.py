@@ -18,9 +18,9 @@ LIB_PATH = os.path.join(HERE, "_build", "libwgconv.so")
 
 # status codes and algorithms (include/conv2d.h)
 OK, ERR_INVALID, ERR_UNSUPPORTED, ERR_NOMEM, ERR_CUDA, ERR_TIMEOUT, ERR_BUSY = range(7)
-ALGO_REFERENCE, ALGO_4X3, ALGO_2X3, ALGO_2X3_FUSED, ALGO_AUTO, ALGO_4X3_ROW = -1, 0, 1, 2, 3, 4
+ALGO_REFERENCE, ALGO_4X3, ALGO_2X3, ALGO_2X3_FUSED, ALGO_AUTO, ALGO_4X3_ROW, ALGO_DIRECT = -1, 0, 1, 2, 3, 4, 5
 ALGO_NAMES = {ALGO_4X3: "F(4x3) non-fused", ALGO_2X3: "F(2x3) non-fused", ALGO_2X3_FUSED: "F(2x3) fused",
-              ALGO_4X3_ROW: "row F(4x3) fused"}
+              ALGO_4X3_ROW: "row F(4x3) fused", ALGO_DIRECT: "direct fused"}
 
 
 class Problem(ctypes.Structure):
@@ -47,7 +47,7 @@ class Options(ctypes.Structure):
 EXPORTS = [
     "getParamsize", "getkernelInfo", "conv2d_fp16", "wg_getParamsize", "wg_getkernelInfo",
     "conv2d_options_default", "getkernelInfo_ex", "conv2d_fp16_ex", "conv2d_fp16_host", "conv2d_fp16_host_steps",
-    "conv2d_refresh_filter", "conv2d_destroy", "conv2d_get_algo", "conv2d_workspace_bytes",
+    "conv2d_refresh_filter", "conv2d_destroy", "conv2d_get_algo", "conv2d_get_direct", "conv2d_workspace_bytes",
     "conv2d_launches_per_call", "conv2d_check_device", "conv2d_last_error", "conv2d_last_error_message",
     "conv2d_status_string", "conv2d_select_reference", "conv2d_copy_to_host", "conv2d_fp16_timed",
     "conv2d_autotune", "conv2d_autotune_clear", "conv2d_fp16_noalloc", "conv2d_noalloc_check_device",
@@ -100,6 +100,7 @@ def lib():
         L.conv2d_refresh_filter.argtypes = [vp, vp]
         L.conv2d_destroy.argtypes = [vp]
         L.conv2d_get_algo.argtypes = [vp]
+        L.conv2d_get_direct.argtypes = [vp]
         L.conv2d_workspace_bytes.argtypes = [vp]
         L.conv2d_workspace_bytes.restype = ctypes.c_longlong
         L.conv2d_launches_per_call.argtypes = [vp]
@@ -207,6 +208,8 @@ class Conv2d:
 
     def kernel_names(self):
         """Kernels launched by one call, in launch order."""
+        if self.direct:
+            return ["direct3x3"]
         if self.algo == ALGO_2X3_FUSED:
             return ["fused2x3"]
         if self.algo == ALGO_4X3_ROW:
@@ -233,6 +236,11 @@ class Conv2d:
     @property
     def algo(self):
         return lib().conv2d_get_algo(self.ptr)
+
+    @property
+    def direct(self):
+        """Whether calls run the direct kernel (by name, or the tuner found it faster)."""
+        return lib().conv2d_get_direct(self.ptr) == 1
 
     @property
     def workspace_bytes(self):

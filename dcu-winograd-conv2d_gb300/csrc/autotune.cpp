@@ -2,14 +2,16 @@
 //
 // The reference picks F(2x3) fused / F(2x3) / F(4x3) with fixed size rules
 // (src/conv2d.cpp:83-114).  Here every candidate (algorithm x GEMM channel
-// tile, plus the row-Winograd F(4x3) kernel this operator adds) is planned on scratch output memory and timed on the device the
-// first time a shape is seen; the winner is cached per shape and, when
+// tile, plus the row-Winograd F(4x3) kernel this operator adds) is planned on
+// scratch output memory and timed on the device the first time a shape is seen; the winner is cached per shape and, when
 // WG_CONV2D_TUNE_FILE names a file, persisted there so later processes make
 // the same choice without measuring.  The reference selection wins unless
 // another candidate is more than 3% faster, so noise between nearly equal
-// candidates cannot flip the choice from run to run.
+// candidates cannot flip the choice from run to run.  The direct kernel is
+// timed as well: where it is faster than the winner, calls run it.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -27,10 +29,22 @@ namespace {
 using Key = std::tuple<unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, unsigned, int, int, int>;
 
 struct Choice {
-    int algo;
+    int algo;      // among the Winograd algorithms
     int bn;
     float ms;
+    bool direct;   // the direct kernel ran faster
 };
+
+// Direct-convolution operations per second the direct kernel holds under the
+// board's power cap: 32 x 256 x 56^2 -> 256 takes 70 us in the first
+// milliseconds, as it is timed here, and 82.5 us (1,435 TFLOP/s) once calls
+// have run back to back for some tenths of a second; the Winograd paths, with
+// 0.25-0.5 of its products, keep their times (101.7 us).  32 x 512 x 28^2 ->
+// 512, 70.5 us here against F(4x3)'s 71.1, would be 80 us in earnest.
+constexpr double kSustainedFlops = 1.43e15;
+
+// In the tune file the algorithm's number carries the direct kernel's flag.
+constexpr int kDirectFlag = 16;
 
 std::mutex g_mu;
 std::map<Key, Choice> g_cache;
@@ -59,7 +73,7 @@ void load_file_locked() {
     float ms;
     while (std::fscanf(fp, "%u %u %u %u %u %u %u %d %d %d %d %d %f", &n, &c, &h, &w, &k, &p, &q, &bf, &f4, &sc, &algo,
                        &bn, &ms) == 13)
-        g_cache[Key(n, c, h, w, k, p, q, bf, f4, sc)] = Choice{algo, bn, ms};
+        g_cache[Key(n, c, h, w, k, p, q, bf, f4, sc)] = Choice{algo & ~kDirectFlag, bn, ms, (algo & kDirectFlag) != 0};
     std::fclose(fp);
 }
 
@@ -70,7 +84,7 @@ void append_file_locked(const Key& kk, const Choice& ch) {
     if (!fp) return;
     std::fprintf(fp, "%u %u %u %u %u %u %u %d %d %d %d %d %.5f\n", std::get<0>(kk), std::get<1>(kk), std::get<2>(kk),
                  std::get<3>(kk), std::get<4>(kk), std::get<5>(kk), std::get<6>(kk), std::get<7>(kk), std::get<8>(kk),
-                 std::get<9>(kk), ch.algo, ch.bn, ch.ms);
+                 std::get<9>(kk), ch.algo | (ch.direct ? kDirectFlag : 0), ch.bn, ch.ms);
     std::fclose(fp);
 }
 
@@ -106,7 +120,8 @@ float time_candidate(const problem_t& pr, conv2d_options_t opt, int algo, int bn
 
 }  // namespace
 
-int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallback, int* algo_out, int* bn_out) {
+int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallback, int* algo_out, int* bn_out,
+                    bool* direct_out) {
     const Key kk = key_of(pr, opt);
     {
         std::lock_guard<std::mutex> lk(g_mu);
@@ -115,6 +130,7 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
         if (it != g_cache.end()) {
             *algo_out = it->second.algo;
             *bn_out = it->second.bn;
+            *direct_out = it->second.direct;
             return CONV2D_OK;
         }
     }
@@ -124,6 +140,7 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
         cudaGetLastError();
         *algo_out = fallback;
         *bn_out = 0;
+        *direct_out = false;
         return CONV2D_ERR_NOMEM;
     }
     cudaStream_t s;
@@ -139,7 +156,7 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
         cands.push_back({a, bn0});
         if (pr.k > 128) cands.push_back({a, bn0 == 256 ? 128 : 256});
     }
-    Choice best{fallback, 0, -1.f};
+    Choice best{fallback, 0, -1.f, false};
     float ref_ms = -1.f;
     int ref_bn = 0;
     for (const Cand& cd : cands) {
@@ -149,12 +166,16 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
             ref_ms = ms;
             ref_bn = cd.bn;
         }
-        if (best.ms < 0.f || ms < best.ms) best = Choice{cd.algo, cd.bn, ms};
+        if (best.ms < 0.f || ms < best.ms) best = Choice{cd.algo, cd.bn, ms, false};
     }
+    const float direct_ms = best.ms < 0.f ? -1.f : time_candidate(pr, opt, CONV2D_ALGO_DIRECT, 0, scratch, s);
     cudaStreamDestroy(s);
     cudaFree(scratch);
-    if (ref_ms > 0.f && best.ms > 0.f && best.ms > ref_ms / 1.03f) best = Choice{fallback, ref_bn, ref_ms};
-    if (best.ms < 0.f) best = Choice{fallback, 0, 0.f};
+    if (ref_ms > 0.f && best.ms > 0.f && best.ms > ref_ms / 1.03f) best = Choice{fallback, ref_bn, ref_ms, false};
+    if (best.ms < 0.f) best = Choice{fallback, 0, 0.f, false};
+    // no margin: its result is the more accurate one
+    const double flops = 18.0 * pr.n * pr.c * pr.k * (pr.h + 2.0 * pr.p - 2) * (pr.w + 2.0 * pr.q - 2);
+    best.direct = direct_ms > 0.f && std::max(static_cast<double>(direct_ms), flops / kSustainedFlops * 1e3) < best.ms;
     {
         std::lock_guard<std::mutex> lk(g_mu);
         if (g_cache.find(kk) == g_cache.end()) {
@@ -164,6 +185,7 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
     }
     *algo_out = best.algo;
     *bn_out = best.bn;
+    *direct_out = best.direct;
     return CONV2D_OK;
 }
 

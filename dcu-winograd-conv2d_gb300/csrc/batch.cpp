@@ -148,6 +148,8 @@ struct Batch {
         Plan& p = *plans[i];
         const void* x_end =
             static_cast<const uint16_t*>(p.prob.in) + static_cast<long long>(p.prob.n) * p.g.c * p.g.h * p.g.w;
+        if (p.run_direct)
+            return launch_direct(p.direct, p.prob.in, p.prob.out, static_cast<int>(p.prob.n), err, s);
         if (p.algo == CONV2D_ALGO_4X3_ROW)
             return launch_row4x3(p.row, p.prob.in, x_end, p.prob.out, static_cast<int>(p.prob.n), err, s);
         return launch_fused2x3(p.fused, p.g, p.prob.in, x_end, p.prob.out, err, s);
@@ -395,7 +397,7 @@ int conv2d_batch_info(const conv2d_batch_t* batch, int index, int* algo, int* ge
     if (!b || index < 0 || index >= static_cast<int>(b->plans.size())) return set_last_error(CONV2D_ERR_INVALID, "bad index");
     const Plan& p = *b->plans[index];
     if (algo) *algo = p.algo;
-    if (gemm_bn) *gemm_bn = p.algo == CONV2D_ALGO_2X3_FUSED ? 32 : p.algo == CONV2D_ALGO_4X3_ROW ? 64 : p.gemm_full.bn;
+    if (gemm_bn) *gemm_bn = p.run_direct ? p.direct.main.bn : p.algo == CONV2D_ALGO_2X3_FUSED ? 32 : p.algo == CONV2D_ALGO_4X3_ROW ? 64 : p.gemm_full.bn;
     return CONV2D_OK;
 }
 

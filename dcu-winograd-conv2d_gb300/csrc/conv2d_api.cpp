@@ -58,6 +58,7 @@ int env_algo(int dflt) {
     if (s == "fused" || s == "2x3_fused") return CONV2D_ALGO_2X3_FUSED;
     if (s == "auto") return CONV2D_ALGO_AUTO;
     if (s == "row" || s == "4x3_row") return CONV2D_ALGO_4X3_ROW;
+    if (s == "direct") return CONV2D_ALGO_DIRECT;
     return dflt;
 }
 
@@ -127,6 +128,12 @@ int default_bn(int K) {
     return w256 <= w128 ? 256 : 128;
 }
 
+// item shape of the direct kernel: gemm_bn where it names one, else from the sizes
+static int direct_tile(const conv2d_options_t& o) {
+    const int bn = o.gemm_bn & 0x1ff;
+    return bn >= 32 && bn <= 256 && bn % 32 == 0 ? o.gemm_bn : 0;
+}
+
 Plan::~Plan() { release(); }
 
 void Plan::release() {
@@ -167,11 +174,14 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
         algo = select_reference64(pr->n, pr->c, pr->h, pr->w, pr->k, pr->r, pr->s, oh, ow);
     if (opt.algo == CONV2D_ALGO_AUTO) {
         int a = algo, bn = 0;
-        autotune_choose(*pr, opt, algo, &a, &bn);
+        autotune_choose(*pr, opt, algo, &a, &bn, &run_direct);
         algo = a;
         if (bn) opt.gemm_bn = bn;
+        // a caller who reads the Winograd-domain workspace back needs it written
+        if (env_int("WG_CONV2D_KEEP_WORKSPACE", 0)) run_direct = false;
     }
-    if (algo < 0 || (algo > 2 && algo != CONV2D_ALGO_4X3_ROW)) return fail(CONV2D_ERR_INVALID, "bad algorithm");
+    if (algo == CONV2D_ALGO_DIRECT) run_direct = true;
+    if (algo < 0 || (algo > 2 && algo != CONV2D_ALGO_4X3_ROW && algo != CONV2D_ALGO_DIRECT)) return fail(CONV2D_ERR_INVALID, "bad algorithm");
 
     op = opt.operand_bf16 ? OpType::BF16 : OpType::F16;
     nhwc = opt.layout_nhwc != 0;
@@ -199,6 +209,18 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
                                     : plan_row4x3(row, g4, nullptr);
         if (opt.io_bf16 || opt.operand_bf16 || opt.tile_scaling || opt.f4_points || pe != cudaSuccess)
             algo = CONV2D_ALGO_4X3_NON_FUSED;
+        cudaGetLastError();
+    }
+    if (run_direct) {
+        // operands in the tensors' own type; where the kernel does not take the
+        // sizes, the selected algorithm runs (F(4x3) non-fused where none is)
+        const Geom g1 = make_geom(pr->n, pr->c, pr->h, pr->w, pr->k, pr->p, pr->q, 2);
+        const int tile = algo == CONV2D_ALGO_DIRECT ? direct_tile(opt) : 0;
+        if ((opt.operand_bf16 && !opt.io_bf16) ||
+            plan_direct(direct, g1, nhwc, opt.io_bf16 != 0, nullptr, tile, num_sms) != cudaSuccess) {
+            run_direct = false;
+            if (algo == CONV2D_ALGO_DIRECT) algo = CONV2D_ALGO_4X3_NON_FUSED;
+        }
         cudaGetLastError();
     }
     const int m = (algo == CONV2D_ALGO_4X3_NON_FUSED || algo == CONV2D_ALGO_4X3_ROW) ? 4 : 2;
@@ -240,7 +262,9 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
 
     // one workspace: U | V | M | scale | device error word (256-byte aligned parts)
     auto al = [](long long b) { return (b + 255) / 256 * 256; };
-    u_bytes = algo == CONV2D_ALGO_4X3_ROW ? row4x3_filter_bytes(row) : static_cast<long long>(E) * g.kp * g.cp * op_bytes;
+    u_bytes = run_direct                    ? direct_filter_bytes(g.k, g.c)
+              : algo == CONV2D_ALGO_4X3_ROW ? row4x3_filter_bytes(row)
+                                            : static_cast<long long>(E) * g.kp * g.cp * op_bytes;
     const long long bU = al(u_bytes);
     long long bV = 0, bM = 0, bS = 0;
     if (!single_kernel()) {
@@ -265,7 +289,18 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
     ce = cudaMemset(err, 0, sizeof(DevErr));
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemset");
 
-    if (algo == CONV2D_ALGO_2X3_FUSED) {
+    if (run_direct) {
+        ce = plan_direct(direct, g, nhwc, opt.io_bf16 != 0, U, algo == CONV2D_ALGO_DIRECT ? direct_tile(opt) : 0, num_sms);
+        if (ce != cudaSuccess) return cuda_fail(ce, "direct plan");
+        launches = 1;
+        {
+            DirectParts parts;
+            info_grid = static_cast<unsigned>(
+                2 * std::min(direct_parts(direct, pr->in, pr->out, static_cast<int>(pr->n), parts), direct.max_pairs));
+        }
+        info_threads = static_cast<unsigned>(direct_threads());
+        info_smem = direct.ring.smem_bytes;
+    } else if (algo == CONV2D_ALGO_2X3_FUSED) {
         ce = plan_fused2x3(fused, op, g, U);
         fused.io_bf16 = opt.io_bf16 != 0;
         if (ce != cudaSuccess) return cuda_fail(ce, "fused plan");
@@ -316,9 +351,9 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
 }
 
 int Plan::filter(cudaStream_t s) {
-    cudaError_t ce = algo == CONV2D_ALGO_4X3_ROW
-                         ? launch_row4x3_filter(row, prob.weight, U, s)
-                         : launch_filter_transform(xf, op, prob.weight, U, g.k, g.c, g.cp, s, opt.io_bf16 != 0);
+    cudaError_t ce = run_direct                    ? launch_direct_filter(prob.weight, U, g.k, g.c, s)
+                     : algo == CONV2D_ALGO_4X3_ROW ? launch_row4x3_filter(row, prob.weight, U, s)
+                                                   : launch_filter_transform(xf, op, prob.weight, U, g.k, g.c, g.cp, s, opt.io_bf16 != 0);
     if (ce != cudaSuccess) return cuda_fail(ce, "filter transform launch");
     filter_ready = true;
     return CONV2D_OK;
@@ -336,6 +371,12 @@ int Plan::run_range(int n0, int nc, const GemmPlan* gp, cudaStream_t s) {
     const Geom gc = make_geom(nc, g.c, g.h, g.w, g.k, g.pad_h, g.pad_w, g.m);
     const uint16_t* xin = static_cast<const uint16_t*>(prob.in) + n0 * in_img;
     uint16_t* yout = static_cast<uint16_t*>(prob.out) + n0 * out_img;
+    if (run_direct) {
+        ce = launch_direct(direct, xin, yout, nc, err, s);
+        if (ce != cudaSuccess) return cuda_fail(ce, "direct convolution launch");
+        mark(s);
+        return CONV2D_OK;
+    }
     if (algo == CONV2D_ALGO_2X3_FUSED) {
         ce = launch_fused2x3(fused, gc, xin, x_end, yout, err, s);
         if (ce != cudaSuccess) return cuda_fail(ce, "fused F(2x3) launch");
@@ -635,6 +676,12 @@ void fill_blob(ParamBlob* pb, Plan* pl) {
     pb->plan = pl;
 }
 
+void replace_plan(void* param, Plan* plan) {
+    Plan* old = plan_of(param);
+    fill_blob(static_cast<ParamBlob*>(param), plan);
+    delete old;
+}
+
 }  // namespace wg
 
 using namespace wg;
@@ -748,6 +795,11 @@ int conv2d_get_algo(const void* param_ptr) {
     return pl ? pl->algo : -1;
 }
 
+int conv2d_get_direct(const void* param_ptr) {
+    Plan* pl = plan_of(param_ptr);
+    return pl ? (pl->run_direct ? 1 : 0) : -1;
+}
+
 long long conv2d_workspace_bytes(const void* param_ptr) {
     Plan* pl = plan_of(param_ptr);
     return pl ? pl->ws_bytes : -1;
@@ -844,7 +896,8 @@ int conv2d_autotune(const problem_t* problem, const conv2d_options_t* opt, int* 
         options_default(&o);
     const unsigned oh = problem->h + 2 * problem->p - 2, ow = problem->w + 2 * problem->q - 2;
     const int ref = select_reference64(problem->n, problem->c, problem->h, problem->w, problem->k, 3, 3, oh, ow);
-    return autotune_choose(*problem, o, ref, algo, gemm_bn);
+    bool direct = false;
+    return autotune_choose(*problem, o, ref, algo, gemm_bn, &direct);
 }
 
 void conv2d_autotune_clear(void) { autotune_clear(); }

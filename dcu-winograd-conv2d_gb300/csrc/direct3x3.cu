@@ -1,0 +1,973 @@
+// Direct 3x3 convolution as an implicit GEMM on the 5th-generation tensor
+// cores, one fused kernel: no Winograd-domain tensor is written.
+//
+// Pixels are numbered in a flattened, zero-padded space: position
+//     z = (n * PH + i) * PW + j      (i, j: padded row and column)
+// with PW = W + max(q, 2q - 2) and PH = H + max(p, 2p - 2), so that the zero
+// columns right of one row are those left of the next, and the zero rows
+// below one image those above the next.  Output (n, oh, ow) sits at
+// z = (n * PH + oh) * PW + ow and its tap (r, s) reads position
+// z + r * PW + s.  A block of consecutive output positions therefore needs
+// one window of consecutive positions, and in the tcgen05 canonical K-major
+// layout (16-byte granules of 8 channels, one per position) each tap is the
+// same window at another start address: nothing is copied per tap.
+//
+// Work item: 256 output positions x bn output channels (bn a multiple of 32,
+// at most 256), computed by a pair of CTAs (cta_group::2, M = 256): each CTA
+// holds the window of its own 128 positions and half of the filter rows.
+// Per 16 input channels:
+//   * producer warps (three groups of four, chunks round robin) read the
+//     window's pixels of 16 channels straight from the caller's tensor --
+//     2-byte loads of 8 planes per granule from NCHW, one 16-byte load from
+//     channels-last -- and write the granules, zeros where padded;
+//   * one TMA box per CTA brings its half of the nine taps' filter rows;
+//   * one thread of the even CTA issues nine MMAs.
+// Accumulators are double-buffered in TMEM (2 x 256 columns), so the epilogue
+// warps store one item while the next is computed.  fp16 or bf16 products are
+// exact and summed in fp32; each output is rounded once.
+//
+// Why a pair and why this tile: per 16 channels an item of 128 positions per
+// CTA x 256 channels takes 1,152 cycles of MMAs, and in that time a CTA reads
+// 9 x (4 + 4) KB of operands from shared memory (576 cycles at 128 bytes),
+// receives 37 KB of filter (288) and writes its window (about 200 with the
+// loads): without the pair the filter side doubles and shared memory, not the
+// tensor cores, sets the time.  Narrow channel tiles are bound there all the
+// same (the window is read nine times for few columns), so they take several
+// blocks of 128 positions per item, which share the filter rows and the
+// window's halo.  Measured, back to back with rotating buffers, against the
+// tuner's choice without this kernel: 32x256x56^2 -> 256 70 us (1,700 TFLOP/s;
+// 82 under the power cap) against 102; 32x256x28^2 -> 256 24.2 against 35;
+// 32x256x14^2 -> 256 13 against 18.7; 1x64x56^2 -> 64 6.8 against 9.5; bf16
+// 32x256x28^2 -> 256 23.8 against 52.7.
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "wg_kernels.h"
+#include "wg_launch.h"
+#include "wg_ptx.cuh"
+
+namespace wg {
+
+namespace {
+
+constexpr int kTaps9 = 9;
+constexpr int kChunkC = 16;                       // input channels per stage
+constexpr int kRows = 128;                        // output positions per CTA
+constexpr int kGroups = 3, kGroupWarps = 4;       // producer groups
+constexpr int kProdWarps = kGroups * kGroupWarps;
+constexpr int kEpiWarps = 4, kEpiHalves = kEpiWarps / 4;
+constexpr int kTmaWarp = kProdWarps + kEpiWarps, kMmaWarpD = kTmaWarp + 1;
+constexpr int kDirectThreads = 32 * (kMmaWarpD + 1);
+constexpr int kMaxRingA = 12, kMaxRingB = 12;
+constexpr int kHeader = 512;                      // barriers
+constexpr int kMaxSmem = 227 * 1024;
+// one CTA per SM (each takes all of TMEM), whatever the rings need
+constexpr int kMinSmem = 116 * 1024;
+
+// Element offset (from image n0) of the input pixel at flattened position z,
+// or -1 where the position is padding or past the last image.
+template <bool NHWC>
+__device__ __forceinline__ int pixel_offset(const DirectDesc& d, int z, int n0) {
+    const int n = static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z)));
+    const int rem = z - n * d.img;
+    const int i = static_cast<int>(fast_div(d.fd_pw, static_cast<uint32_t>(rem)));
+    const int y = i - d.pad_h, x = rem - i * d.pw - d.pad_w;
+    const bool in = n < d.n && static_cast<unsigned>(y) < static_cast<unsigned>(d.h) &&
+                    static_cast<unsigned>(x) < static_cast<unsigned>(d.w);
+    const int pix = y * d.w + x;
+    return in ? (n - n0) * (d.c * d.h * d.w) + (NHWC ? pix * d.c : pix) : -1;
+}
+
+__device__ __forceinline__ uint32_t ldg16(const uint16_t* p) {
+    uint16_t v;
+    asm volatile("ld.global.nc.b16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint32_t ldg32(const uint16_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void ldg128(const uint16_t* p, uint32_t* v) {
+    asm volatile("ld.global.nc.v4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "l"(p));
+}
+
+struct DItem {
+    int tile, nb;
+};
+
+__device__ __forceinline__ DItem locate_direct(const DirectDesc* __restrict__ descs, int ndesc, int t, int& pi) {
+    while (pi + 1 < ndesc && t >= descs[pi + 1].item_begin) ++pi;
+    const DirectDesc& d = descs[pi];
+    const uint32_t local = static_cast<uint32_t>(t - d.item_begin);
+    DItem it;
+    it.tile = static_cast<int>(fast_div(d.fd_nb, local));
+    it.nb = static_cast<int>(local) - it.tile * d.n_blocks;
+    return it;
+}
+
+// ---- producers ----------------------------------------------------------------
+// A group of four warps writes the windows of every kGroups-th chunk.  Its
+// work is a sequence of steps (item, chunk, block of positions), each 16
+// registers of loads per thread; a step's loads are issued before the step
+// ahead of it is stored, so one load latency covers two steps.  Per block and
+// thread:
+//   pairs   two neighbouring pixels of 16 planes (4-byte loads; W even, x
+//           4-byte aligned), 128 pairs; the padding of the window is cleared
+//           by the threads whose positions it is
+//   single  one position of 16 planes (2-byte loads), 128 positions
+//   NHWC    four (position, granule) of 16 bytes, 256 positions
+constexpr int kGroupThreads = 32 * kGroupWarps;
+constexpr int kMaxPadBits = 32;      // pairs: positions per thread the pad mask covers
+
+struct Step {
+    uint32_t r[16];
+    int p;             // pairs, single: position of the first granule; NHWC: of the block's first
+    uint32_t pads;     // pairs: bit i set where position gt + 128 i is padding (last block of a chunk only)
+    uint32_t flags;    // bit 0: first block of the chunk, 1: last, 2: pairs; 4..7: zero the granule
+                       // (single: 4); the window's length above bit 16
+};
+
+// Bytes of one granule's window in shared memory: 4 mod 8 positions, so that
+// the two granules of a channels-last pixel fall in different bank groups.
+__host__ __device__ __forceinline__ int granule_bytes(int win) { return ((win + 7) / 8 * 8 + 4) * 16; }
+
+template <bool NHWC>
+struct Producer {
+    const DirectDesc* __restrict__ descs;
+    int ndesc, total_items, step, grp, gt;
+    uint32_t rank;
+    // load cursor
+    int t, pi, c, chunks, gc0, blk, blocks;
+    int z0, n0, win, channels;
+    int pairs;
+    uint32_t plane;
+    const uint16_t* xi;
+    // the item's first blocks: element offset from xi (-1: nothing to load) and
+    // position; NHWC: the four parts of the first two blocks
+    static constexpr int kKeep = NHWC ? 8 : 4;
+    int off[kKeep];
+    uint32_t pos2[2];   // positions of blocks 0, 1 and 2, 3 as 16-bit halves (-1 as 0xffff)
+    uint32_t pads;
+
+    // pairs: pair number gt + 128 i of the window, decoded from scratch (blocks past kKeep)
+    __device__ __forceinline__ void locate_pair(const DirectDesc& d, int i, int& o, int& p) const {
+        const int g = d_first(d) + 2 * (gt + kGroupThreads * i);
+        const int hw = d.h * d.w, n = static_cast<int>(fast_div(d.fd_hw, static_cast<uint32_t>(g))), m = g - n * hw;
+        const int y = static_cast<int>(fast_div(d.fd_w, static_cast<uint32_t>(m)));
+        p = n * d.img + (y + d.pad_h) * d.pw + (m - y * d.w) + d.pad_w - z0;
+        o = n < d.n && p < win ? (n - n0) * (d.c * hw) + m : -1;
+        if (o < 0) p = win;
+    }
+    // index (over all images, in memory order of one channel) of the first
+    // pixel pair that reaches into the window
+    __device__ __forceinline__ int d_first(const DirectDesc& d) const {
+        const int n = static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z0)));
+        const int rem = z0 - n * d.img;
+        const int i = static_cast<int>(fast_div(d.fd_pw, static_cast<uint32_t>(rem)));
+        const int y = i - d.pad_h, x = rem - i * d.pw - d.pad_w;
+        const int m = y < 0 ? 0 : min(y, d.h) * d.w + (y < d.h ? min(max(x, 0), d.w) : 0);
+        return (n * (d.h * d.w) + m) & ~1;
+    }
+
+    __device__ __forceinline__ void decode(const DirectDesc& d) {
+        if constexpr (NHWC) {
+#pragma unroll
+            for (int i = 0; i < kKeep; ++i) off[i] = pixel_offset<true>(d, z0 + i * 64 + (gt >> 1), n0);
+        } else if (pairs) {
+            // pairs 128 apart: a step of qy rows and rx columns
+            const int hw = d.h * d.w, w = d.w, h = d.h, chw = d.c * hw;
+            const int g = d_first(d) + 2 * gt;
+            int n = static_cast<int>(fast_div(d.fd_hw, static_cast<uint32_t>(g)));
+            const int m = g - n * hw;
+            int y = static_cast<int>(fast_div(d.fd_w, static_cast<uint32_t>(m))), x = m - y * w;
+#pragma unroll
+            for (int i = 0; i < kKeep; ++i) {
+                const int p = n * d.img + (y + d.pad_h) * d.pw + x + d.pad_w - z0;
+                const bool in = n < d.n && p < win;
+                off[i] = in ? (n - n0) * chw + y * w + x : -1;
+                const uint32_t q = static_cast<uint32_t>(in ? p : win) & 0xffffu;
+                pos2[i / 2] = (i & 1) ? pos2[i / 2] | (q << 16) : q;
+                x += d.step_x;
+                y += d.step_y;
+                if (x >= w) x -= w, ++y;
+                while (y >= h && n < d.n) y -= h, ++n;
+            }
+            // positions 128 apart: the window's padding among this thread's
+            int zn = static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z0 + gt)));
+            const int rem = z0 + gt - zn * d.img;
+            int zi = static_cast<int>(fast_div(d.fd_pw, static_cast<uint32_t>(rem))), zj = rem - zi * d.pw;
+            pads = 0;
+            for (int i = 0, p = gt; p < win; ++i, p += kGroupThreads) {
+                const bool in = zn < d.n && static_cast<unsigned>(zi - d.pad_h) < static_cast<unsigned>(h) &&
+                                static_cast<unsigned>(zj - d.pad_w) < static_cast<unsigned>(w);
+                pads |= (in ? 0u : 1u) << i;
+                zj += d.pad_step_j;
+                zi += d.pad_step_i;
+                if (zj >= d.pw) zj -= d.pw, ++zi;
+                while (zi >= d.ph) zi -= d.ph, ++zn;
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < kKeep; ++i) {
+                const uint32_t q = static_cast<uint32_t>(gt + kGroupThreads * i);
+                pos2[i / 2] = (i & 1) ? pos2[i / 2] | (q << 16) : q;
+                off[i] = pixel_offset<false>(d, z0 + static_cast<int>(q), n0);
+            }
+        }
+    }
+
+    // moves to the group's next step; false when there is none
+    __device__ __forceinline__ bool advance() {
+        if (++blk < blocks) return true;
+        blk = 0;
+        c += kGroups;
+        while (c >= chunks) {
+            gc0 += chunks;
+            chunks = 0;
+            t += step;
+            if (t >= total_items) return false;
+            const DItem it = locate_direct(descs, ndesc, t, pi);
+            const DirectDesc& d = descs[pi];
+            chunks = d.c_chunks;
+            c = (grp - gc0 % kGroups + kGroups) % kGroups;
+            if (c >= chunks) continue;
+            z0 = d.pos0 + (2 * it.tile + static_cast<int>(rank)) * d.cta_rows;
+            n0 = min(static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z0))), d.n - 1);
+            win = d.win;
+            channels = d.c;
+            pairs = d.pairs;
+            plane = static_cast<uint32_t>(d.h * d.w);
+            xi = static_cast<const uint16_t*>(d.x) + static_cast<long long>(n0) * channels * plane;
+            blocks = NHWC ? (win + 255) / 256 : pairs ? (win / 2 + kGroupThreads) / kGroupThreads
+                                                     : (win + kGroupThreads - 1) / kGroupThreads;
+            pads = 0;
+            decode(d);
+        }
+        return true;
+    }
+
+    __device__ __forceinline__ void load(Step& s) const {
+        const int left = channels - c * kChunkC;   // channels from this chunk on
+        s.flags = (static_cast<uint32_t>(win) << 16) | (blk == 0 ? 1u : 0u) | (blk == blocks - 1 ? 2u : 0u) | (pairs ? 4u : 0u);
+        s.pads = blk == blocks - 1 ? pads : 0u;
+        if (NHWC) {
+            const int gsel = gt & 1, ch = c * kChunkC + 8 * gsel;
+            s.p = blk * 256 + (gt >> 1);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                int o = blk == 0 ? off[k] : off[4 + k];
+                if (blk > 1) o = pixel_offset<true>(descs[pi], z0 + s.p + 64 * k, n0);
+                if (o < 0 || ch >= channels) {
+                    o = 0;
+                    s.flags |= 16u << k;
+                }
+                ldg128(xi + o + (ch < channels ? ch : 0), s.r + 4 * k);
+            }
+        } else {
+            int o = off[0];
+            o = blk == 1 ? off[1] : o;
+            o = blk == 2 ? off[2] : o;
+            o = blk == 3 ? off[3] : o;
+            const uint32_t pq = blk < 2 ? pos2[0] : pos2[1];
+            int p = static_cast<int16_t>((blk & 1) ? pq >> 16 : pq);
+            if (blk >= kKeep) {
+                if (pairs) {
+                    locate_pair(descs[pi], blk, o, p);
+                } else {
+                    p = gt + kGroupThreads * blk;
+                    o = pixel_offset<false>(descs[pi], z0 + p, n0);
+                }
+            }
+            s.p = p;
+            if (o < 0) s.flags |= 16u;
+            // a warp whose lanes all lie past the window reads one value over and over
+            const bool live = __any_sync(0xffffffffu, p < win);
+            // padding reads the image's first pixel (cleared or not stored later)
+            const uint16_t* src = xi + max(o, 0) + static_cast<unsigned long long>(c * kChunkC) * plane;
+            const uint32_t st = live ? plane : 0u;
+            if (left >= kChunkC) {
+                if (pairs) {
+#pragma unroll
+                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg32(src + static_cast<unsigned long long>(j) * st);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg16(src + static_cast<unsigned long long>(j) * st);
+                }
+            } else {
+                // the last chunk of a C that is not a multiple of 16
+#pragma unroll
+                for (int j = 0; j < kChunkC; ++j) {
+                    const uint16_t* q = src + static_cast<unsigned long long>(min(j, left - 1)) * st;
+                    const uint32_t v = pairs ? ldg32(q) : ldg16(q);
+                    s.r[j] = j < left ? v : 0u;
+                }
+            }
+        }
+    }
+
+    // writes a loaded step's granules into the window stage at A
+    __device__ __forceinline__ void store(const Step& s, unsigned char* A) const {
+        const int s_win = static_cast<int>(s.flags >> 16), s_gran = granule_bytes(s_win);
+        if (NHWC) {
+            unsigned char* dst = A + (gt & 1) * s_gran;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int p = s.p + 64 * k;
+                const bool z = (s.flags >> (4 + k)) & 1u;
+                if (p < s_win)
+                    *reinterpret_cast<uint4*>(dst + p * 16) =
+                        make_uint4(z ? 0u : s.r[4 * k], z ? 0u : s.r[4 * k + 1], z ? 0u : s.r[4 * k + 2], z ? 0u : s.r[4 * k + 3]);
+            }
+        } else if (s.flags & 4u) {
+            // lanes 4-7 of every 8 store their second pixel first: the 8 lanes
+            // of a store phase then write 8 different 16-byte bank groups
+            const uint32_t sel0 = (gt & 4) ? 0x7632u : 0x5410u, sel1 = sel0 ^ 0x2222u;
+            const int p0 = s.p + ((gt >> 2) & 1), p1 = s.p + 1 - ((gt >> 2) & 1);
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+                const uint32_t* r = s.r + 8 * g;
+                unsigned char* dst = A + g * s_gran;
+                if (static_cast<unsigned>(p0) < static_cast<unsigned>(s_win))
+                    *reinterpret_cast<uint4*>(dst + p0 * 16) =
+                        make_uint4(__byte_perm(r[0], r[1], sel0), __byte_perm(r[2], r[3], sel0),
+                                   __byte_perm(r[4], r[5], sel0), __byte_perm(r[6], r[7], sel0));
+                if (static_cast<unsigned>(p1) < static_cast<unsigned>(s_win) && s.p < s_win)
+                    *reinterpret_cast<uint4*>(dst + p1 * 16) =
+                        make_uint4(__byte_perm(r[0], r[1], sel1), __byte_perm(r[2], r[3], sel1),
+                                   __byte_perm(r[4], r[5], sel1), __byte_perm(r[6], r[7], sel1));
+            }
+            for (uint32_t m = s.pads; m; m &= m - 1) {
+                unsigned char* dst = A + (gt + kGroupThreads * (__ffs(m) - 1)) * 16;
+                *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+                *reinterpret_cast<uint4*>(dst + s_gran) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        } else {
+            const bool z = (s.flags & 16u) != 0;
+            if (s.p < s_win)
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    const uint32_t* r = s.r + 8 * g;
+                    *reinterpret_cast<uint4*>(A + g * s_gran + s.p * 16) =
+                        z ? make_uint4(0u, 0u, 0u, 0u)
+                          : make_uint4(__byte_perm(r[0], r[1], 0x5410), __byte_perm(r[2], r[3], 0x5410),
+                                       __byte_perm(r[4], r[5], 0x5410), __byte_perm(r[6], r[7], 0x5410));
+                }
+        }
+    }
+};
+
+template <bool BF16>
+__device__ __forceinline__ uint32_t pack2(uint32_t a, uint32_t b) {
+    if constexpr (BF16) {
+        __nv_bfloat162 v = __floats2bfloat162_rn(__uint_as_float(a), __uint_as_float(b));
+        return *reinterpret_cast<uint32_t*>(&v);
+    } else {
+        __half2 v = __floats2half2_rn(__uint_as_float(a), __uint_as_float(b));
+        return *reinterpret_cast<uint32_t*>(&v);
+    }
+}
+
+// Stores a loaded step once its stage is free; after a chunk's last block
+// hands the stage to the MMAs and moves to the group's next one.
+template <bool NHWC>
+__device__ __forceinline__ bool flush_step(const Producer<NHWC>& pr, const Step& s, unsigned char* astage, int a_bytes,
+                                           int na, int& sa, uint32_t& ph, uint64_t* afull, uint64_t* aempty,
+                                           volatile int* abort_flag, DevErr* err) {
+    if ((s.flags & 1u) && !mbar_wait(&aempty[sa], ph, abort_flag, err, ERR_SITE_EMPTY)) return false;
+    pr.store(s, astage + sa * a_bytes);
+    if (s.flags & 2u) {
+        fence_proxy_async_smem();     // the window is read by the tensor core
+        __syncwarp();
+        if ((pr.gt & 31) == 0) mbar_arrive_cluster(map_to_rank(&afull[sa], 0));
+        sa += kGroups;
+        while (sa >= na) sa -= na, ph ^= 1u;
+    }
+    return true;
+}
+
+template <bool NHWC, bool BF16>
+__device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs, int ndesc, int total_items,
+                                            const DirectRing& ring, DevErr* err) {
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    unsigned char* bstage = smem;                              // filter ring
+    unsigned char* astage = smem + ring.nb * ring.b_bytes;     // window ring
+    uint64_t* bars = reinterpret_cast<uint64_t*>(astage + ring.na * ring.a_bytes);
+    uint64_t* afull = bars;                        // even CTA: windows of both CTAs written
+    uint64_t* aempty = afull + kMaxRingA;          // MMAs done with the window
+    uint64_t* bfull = aempty + kMaxRingA;          // even CTA: filter halves of both CTAs landed
+    uint64_t* bempty = bfull + kMaxRingB;          // MMAs done with the filter rows
+    uint64_t* tfull = bempty + kMaxRingB;          // [2] accumulator ready
+    uint64_t* tempty = tfull + 2;                  // [2] even CTA: accumulator drained in both CTAs
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
+    const int na = ring.na, nb = ring.nb;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kMaxRingA; ++i) {
+            mbar_init(&afull[i], 2 * kGroupWarps);
+            mbar_init(&aempty[i], 1);
+        }
+        for (int i = 0; i < kMaxRingB; ++i) {
+            mbar_init(&bfull[i], 1);
+            mbar_init(&bempty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], 2 * kEpiWarps);
+        }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    pdl_wait();     // input and filter written, earlier readers of the output done
+    pdl_trigger();
+    if (warp == kMmaWarpD) tmem_alloc_pair(tmem_slot, 512);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp < kProdWarps) {
+        Producer<NHWC> pr;
+        pr.descs = descs;
+        pr.ndesc = ndesc;
+        pr.total_items = total_items;
+        pr.step = step;
+        pr.grp = warp / kGroupWarps;
+        pr.gt = static_cast<int>(threadIdx.x) - pr.grp * kGroupThreads;
+        pr.rank = rank;
+        pr.t = first - step;
+        pr.pi = pr.c = pr.chunks = pr.gc0 = pr.blk = pr.blocks = 0;
+        int sa = pr.grp;             // this group's next window stage and its phase
+        uint32_t ph = 1;
+        while (sa >= na) sa -= na, ph ^= 1u;
+        bool ok = true;
+        Step s0, s1;
+        bool more = pr.advance();
+        if (more) pr.load(s0);
+        while (more) {
+            more = pr.advance();
+            if (more) pr.load(s1);
+            ok = flush_step(pr, s0, astage, ring.a_bytes, na, sa, ph, afull, aempty, abort_flag, err);
+            if (!ok || !more) break;
+            more = pr.advance();
+            if (more) pr.load(s0);
+            ok = flush_step(pr, s1, astage, ring.a_bytes, na, sa, ph, afull, aempty, abort_flag, err);
+            if (!ok) break;
+        }
+        // the last commits on this CTA's window barriers must land before it exits
+        if (ok && warp == 0 && lane == 0)
+            for (int k = max(0, pr.gc0 - na); k < pr.gc0; ++k)
+                if (!mbar_wait(&aempty[k % na], (k / na) & 1, abort_flag, err, ERR_SITE_DRAIN)) break;
+    } else if (warp == kTmaWarp) {
+        // ---- filter halves: one box per chunk, counted on the even CTA's barrier
+        if (lane == 0) {
+            int gc = 0, pi = 0, prefetched = -1;
+            bool ok = true;
+            for (int t = first; t < total_items && ok; t += step) {
+                const DItem it = locate_direct(descs, ndesc, t, pi);
+                const DirectDesc& d = descs[pi];
+                if (prefetched != pi) {
+                    tma_prefetch_desc(&d.tmU);
+                    prefetched = pi;
+                }
+                const uint32_t bytes = static_cast<uint32_t>(kTaps9 * 2 * (d.bn / 2) * 16);
+                const int row = (it.nb * d.bn + static_cast<int>(rank) * (d.bn / 2)) / 8;
+                const int chunks = d.c_chunks;
+                for (int c = 0; c < chunks; ++c, ++gc) {
+                    const int sb = gc % nb;
+                    if (!mbar_wait(&bempty[sb], ((gc / nb) & 1) ^ 1, abort_flag, err, ERR_SITE_EMPTY)) {
+                        ok = false;
+                        break;
+                    }
+                    if (rank == 0) mbar_arrive_expect_tx(&bfull[sb], 2 * bytes);
+                    tma_load_4d_pair(bstage + sb * ring.b_bytes, &d.tmU, map_to_rank(&bfull[sb], 0), 0, row, c * 2, 0);
+                }
+            }
+            if (ok)
+                for (int k = max(0, gc - nb); k < gc; ++k)
+                    if (!mbar_wait(&bempty[k % nb], (k / nb) & 1, abort_flag, err, ERR_SITE_DRAIN)) break;
+        }
+    } else if (warp == kMmaWarpD) {
+        // ---- MMAs of the pair, issued by one elected thread of the even CTA.
+        //      The whole warp walks the loop with warp-uniform control flow and
+        //      values, so descriptors stay in uniform registers: with one lane
+        //      in the loop every MMA first moved its operands there
+        if (rank == 0) {
+            int pi = 0, k = 0, sa = 0, sb = 0;
+            uint32_t aph = 0, bph = 0;
+            const int a_step = ring.a_bytes / 16, b_step = ring.b_bytes / 16;
+            const uint64_t a_lo = make_smem_desc(smem_u32(astage), 0, 128, Swz::None);
+            const uint64_t b_lo = make_smem_desc(smem_u32(bstage), 0, 128, Swz::None);
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const bool elected = elect_one();
+            bool ok = true;
+            for (int t = first; t < total_items && ok; t += step, ++k) {
+                locate_direct(descs, ndesc, t, pi);
+                const DirectDesc& d = descs[pi];
+                const int acc = k & 1;
+                if (!mbar_wait_warp(&tempty[acc], ((k >> 1) & 1) ^ 1, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+                tc_fence_after();
+                const uint32_t idesc = make_idesc_f16(2 * kRows, d.bn, BF16);
+                const uint32_t d_tmem = tmem_u + static_cast<uint32_t>(acc * 256);
+                // descriptors of stage 0, tap 0; stages and taps only move the
+                // start address (the low 14 bits, in 16-byte units)
+                const int chunks = d.c_chunks, bn = d.bn, pw = d.pw, mb = d.mb;
+                const uint64_t ad0 = a_lo | (static_cast<uint64_t>(d.gran >> 4) << 16);
+                const uint64_t bd0 = b_lo | (static_cast<uint64_t>(bn >> 1) << 16);
+                for (int c = 0; c < chunks; ++c) {
+                    if (!mbar_wait_warp(&bfull[sb], bph, abort_flag, err, ERR_SITE_FULL) ||
+                        !mbar_wait_warp(&afull[sa], aph, abort_flag, err, ERR_SITE_FULL)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t as = ad0 + static_cast<uint32_t>(sa * a_step);
+                    const uint64_t bs = bd0 + static_cast<uint32_t>(sb * b_step);
+                    if (elected) {
+                        for (int m = 0; m < mb; ++m) {
+                            const uint64_t am = as + static_cast<uint32_t>(m * kRows);
+#pragma unroll
+                            for (int tap = 0; tap < kTaps9; ++tap)
+                                tc_mma_f16_pair(d_tmem + static_cast<uint32_t>(m * bn),
+                                                am + static_cast<uint32_t>((tap / 3) * pw + tap % 3),
+                                                bs + static_cast<uint32_t>(tap * bn), idesc, (c | tap) != 0 ? 1u : 0u);
+                        }
+                        tc_commit_pair(&aempty[sa]);
+                        tc_commit_pair(&bempty[sb]);
+                    }
+                    __syncwarp();
+                    if (++sa == na) sa = 0, aph ^= 1u;
+                    if (++sb == nb) sb = 0, bph ^= 1u;
+                }
+                if (ok && elected) tc_commit_pair(&tfull[acc]);
+                __syncwarp();
+            }
+        }
+    } else {
+        // ---- epilogue: kEpiHalves warps per TMEM lane quarter, taking blocks
+        //      of 16 columns in turn
+        const int quarter = warp & 3, half = (warp - kProdWarps) >> 2;
+        int pi = 0, k = 0;
+        for (int t = first; t < total_items; t += step, ++k) {
+            const DItem it = locate_direct(descs, ndesc, t, pi);
+            const DirectDesc& d = descs[pi];
+            const int acc = k & 1;
+            if (!mbar_wait(&tfull[acc], (k >> 1) & 1, abort_flag, err, ERR_SITE_TMEM_FULL)) break;
+            __syncwarp();
+            tc_fence_after();
+            uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * 256 + half * 16);
+            const int K = d.k, bn = d.bn, mb = d.mb, ow_n = d.ow;
+            const int oplane = d.oh * ow_n;
+            const bool vec = d.vec != 0;
+            const int zb = d.pos0 + (2 * it.tile + static_cast<int>(rank)) * d.cta_rows + quarter * 32 + lane;
+            for (int m = 0; m < mb; ++m) {
+                const int z = zb + m * kRows;
+                const int n = static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z)));
+                const int rem = z - n * d.img;
+                const int oh = static_cast<int>(fast_div(d.fd_pw, static_cast<uint32_t>(rem)));
+                const int ow = rem - oh * d.pw;
+                const bool valid = n < d.n && oh < d.oh && ow < ow_n;
+                const int opix = oh * ow_n + ow;
+                int k0 = it.nb * bn + half * 16;
+                uint16_t* o = static_cast<uint16_t*>(d.y);
+                if constexpr (NHWC)
+                    o += (static_cast<long long>(n) * oplane + opix) * K + k0;
+                else
+                    o += (static_cast<long long>(n) * K + k0) * oplane + opix;
+                for (int b = half; b < bn / 16; b += kEpiHalves, k0 += 16 * kEpiHalves, taddr += 16 * kEpiHalves) {
+                    uint32_t r[16];
+                    tmem_ld_x16(taddr, r);
+                    tc_wait_ld16(r);
+                    if (m == mb - 1 && b + kEpiHalves >= bn / 16) {   // this warp's last read of the accumulators
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(map_to_rank(&tempty[acc], 0));
+                    }
+                    if (valid) {
+                        if constexpr (NHWC) {
+                            if (vec && k0 + 16 <= K) {
+#pragma unroll
+                                for (int j = 0; j < 2; ++j)
+                                    reinterpret_cast<uint4*>(o)[j] = make_uint4(
+                                        pack2<BF16>(r[8 * j], r[8 * j + 1]), pack2<BF16>(r[8 * j + 2], r[8 * j + 3]),
+                                        pack2<BF16>(r[8 * j + 4], r[8 * j + 5]), pack2<BF16>(r[8 * j + 6], r[8 * j + 7]));
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    if (k0 + j < K) o[j] = static_cast<uint16_t>(pack2<BF16>(r[j], 0u));
+                            }
+                        } else {
+                            // a warp's 32 positions of one channel are (nearly) contiguous
+                            uint16_t* q = o;
+                            if (k0 + 16 <= K) {
+#pragma unroll
+                                for (int j = 0; j < 16; j += 2) {
+                                    const uint32_t v = pack2<BF16>(r[j], r[j + 1]);
+                                    q[0] = static_cast<uint16_t>(v);
+                                    q[oplane] = static_cast<uint16_t>(v >> 16);
+                                    q += 2 * static_cast<long long>(oplane);
+                                }
+                            } else {
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) {
+                                    if (k0 + j < K) *q = static_cast<uint16_t>(pack2<BF16>(r[j], 0u));
+                                    q += oplane;
+                                }
+                            }
+                        }
+                    }
+                    o += NHWC ? 16LL * kEpiHalves : 16LL * kEpiHalves * oplane;
+                    __syncwarp();
+                }
+                // (bn / 16 is even: every warp of a quarter takes as many blocks)
+            }
+        }
+    }
+
+    __syncthreads();
+    if (*abort_flag) {
+        // let any copy or MMA still in flight land before the pair retires
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) {
+        }
+    }
+    tc_fence_before();
+    cluster_sync();   // the peer's MMAs, copies and arrivals on this CTA are done
+    tc_fence_after();
+    if (warp == kMmaWarpD) tmem_dealloc_pair(tmem_base, 512);
+}
+
+template <bool NHWC, bool BF16>
+__global__ void __launch_bounds__(kDirectThreads, 1)
+    direct3x3_kernel(const __grid_constant__ DirectParts parts, const __grid_constant__ DirectRing ring, DevErr* err) {
+    direct_body<NHWC, BF16>(parts.d, parts.count, parts.items, ring, err);
+}
+
+// U9[tap][Cp/8][Kp][8]: the KCRS filter as granules of 8 input channels, zero
+// past C and K.  One thread per (output channel, granule).
+__global__ void __launch_bounds__(256) direct_filter_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ U, int K,
+                                                           int C, int CG, int Kp) {
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= CG * Kp) return;
+    const int g = idx / Kp, k = idx - g * Kp;
+    uint16_t v[8][kTaps9];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+        const int c = g * 8 + j;
+        const uint16_t* src = w + (static_cast<long long>(k) * C + c) * kTaps9;
+#pragma unroll
+        for (int t = 0; t < kTaps9; ++t) v[j][t] = (k < K && c < C) ? src[t] : static_cast<uint16_t>(0);
+    }
+#pragma unroll
+    for (int t = 0; t < kTaps9; ++t) {
+        uint4 q;
+        q.x = v[0][t] | (static_cast<uint32_t>(v[1][t]) << 16);
+        q.y = v[2][t] | (static_cast<uint32_t>(v[3][t]) << 16);
+        q.z = v[4][t] | (static_cast<uint32_t>(v[5][t]) << 16);
+        q.w = v[6][t] | (static_cast<uint32_t>(v[7][t]) << 16);
+        *reinterpret_cast<uint4*>(U + ((static_cast<long long>(t) * CG + g) * Kp + k) * 8) = q;
+    }
+}
+
+// The KCRS filter back from U9, one thread per value.
+__global__ void __launch_bounds__(256) direct_unfilter_kernel(const uint16_t* __restrict__ U, uint16_t* __restrict__ w, int K,
+                                                             int C, int CG, int Kp) {
+    const long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (idx >= static_cast<long long>(K) * C * kTaps9) return;
+    const int t = static_cast<int>(idx % kTaps9), c = static_cast<int>(idx / kTaps9 % C);
+    const int k = static_cast<int>(idx / kTaps9 / C);
+    w[idx] = U[((static_cast<long long>(t) * CG + c / 8) * Kp + k) * 8 + (c & 7)];
+}
+
+// Output positions of n images, up to the last one.
+long long positions(const DirectDesc& d, long long n) {
+    return (n - 1) * d.img + static_cast<long long>(d.oh - 1) * d.pw + d.ow;
+}
+
+int window_of(int mb, int pw) { return kRows * mb + 2 * pw + 2; }
+
+int b_stage_bytes(int bn) { return kTaps9 * bn * 16; }
+
+// Ring depths for one window size and channel tile; false when two stages of
+// each do not fit.
+bool size_ring(DirectRing& r, int a_bytes, int b_bytes) {
+    const int room = kMaxSmem - 1024 - kHeader;
+    r.a_bytes = a_bytes;
+    r.b_bytes = b_bytes;
+    // as many chunks ahead on both sides; what is left over goes to the windows
+    for (int nb = std::min(kMaxRingB, room / (a_bytes + b_bytes)); nb >= 2; --nb) {
+        const int na = std::min(kMaxRingA, (room - nb * b_bytes) / a_bytes);
+        if (na >= 2) {
+            r.nb = nb;
+            r.na = na;
+            r.smem_bytes = std::max(kMinSmem, nb * b_bytes + na * a_bytes + kHeader + 1024);
+            return true;
+        }
+    }
+    return false;
+}
+
+// Cycles of one item of mb x 256 positions x bn channels: per chunk the longer
+// of its 9 mb MMAs (each bn / 2 cycles of tensor time for 256 x bn x 16 on a
+// pair, or the shared-memory reads of its operands: 4 KB of window and 16 bn
+// bytes of filter per CTA at 128 bytes per cycle) and the producers' time for
+// the window; plus what an item costs however short.
+double item_cycles(int bn, int mb, int pw, int chunks) {
+    const double mma = 9.0 * mb * std::max(bn / 2.0, 36.0 + bn / 8.0);
+    const double prod = 150.0 + 2.0 * window_of(mb, pw);
+    return chunks * std::max(mma, prod) + 1200.0 + 120.0 * mb * bn / 32;
+}
+
+template <class F, class... Args>
+cudaError_t launch_cluster(F kern, int pairs, int smem, cudaStream_t s, const Args&... args) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs);
+    cfg.blockDim = dim3(kDirectThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// CTA pairs that run at once (one CTA per SM; a cluster stays within a GPC)
+int max_pairs(int num_sms) {
+    auto kern = direct3x3_kernel<false, false>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) return num_sms / 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (num_sms / 2));
+    cfg.blockDim = dim3(kDirectThreads);
+    cfg.dynamicSmemBytes = kMaxSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+        cudaGetLastError();
+        return num_sms / 2;
+    }
+    return std::min(n, num_sms / 2);
+}
+
+}  // namespace
+
+int direct_threads() { return kDirectThreads; }
+
+long long direct_filter_bytes(int K, int C) {
+    return static_cast<long long>(kTaps9) * ((C + 7) / 8 * 8) * ((K + 7) / 8 * 8) * 2;
+}
+
+namespace {
+
+// One way to cut a problem: items of mb x 256 positions x bn channels, and the
+// positions past the last whole round of items in smaller ones.
+struct Split {
+    int bn = 0, mb = 0;
+    long long main_tiles = 0;     // tiles of the main part
+    int tail_bn = 0, tail_mb = 0; // 0: no tail
+    double cycles = 0;
+};
+
+bool tile_fits(int bn, int mb, int pw, DirectRing* ring) {
+    if (bn * mb > 256) return false;
+    const int a = (2 * granule_bytes(window_of(mb, pw)) + 127) / 128 * 128;
+    DirectRing r;
+    if (!size_ring(r, a, b_stage_bytes(bn))) return false;
+    if (ring) *ring = r;
+    return true;
+}
+
+// Least rounds x cycles for `pos` positions over `pairs` pairs.
+Split best_split(long long pos, int K, int pw, int chunks, int pairs, int only_bn, int only_mb, bool tail) {
+    Split best;
+    for (int mb = 1; mb <= 8; mb *= 2) {
+        if (only_mb && mb != only_mb) continue;
+        for (int bn = 32; bn <= 256; bn += 32) {
+            if (only_bn && bn != only_bn) continue;
+            if (!tile_fits(bn, mb, pw, nullptr)) continue;
+            const long long rows = 2LL * kRows * mb;
+            const long long tiles = (pos + rows - 1) / rows, nb = (K + bn - 1) / bn, items = tiles * nb;
+            const double one = item_cycles(bn, mb, pw, chunks);
+            Split s;
+            s.bn = bn;
+            s.mb = mb;
+            s.main_tiles = tiles;
+            s.cycles = static_cast<double>((items + pairs - 1) / pairs) * one;
+            if (best.bn == 0 || s.cycles < best.cycles) best = s;
+            // whole rounds in the main part, the rest in items that take less than one more round
+            const long long rounds = items / pairs, main = rounds * pairs / nb;
+            if (tail && main > 0 && main < tiles) {
+                const Split t = best_split(pos - main * rows, K, pw, chunks, pairs, 0, 0, false);
+                s.main_tiles = main;
+                s.tail_bn = t.bn;
+                s.tail_mb = t.mb;
+                s.cycles = static_cast<double>((main * nb + pairs - 1) / pairs) * one + t.cycles;
+                if (s.cycles < best.cycles) best = s;
+            }
+        }
+    }
+    return best;
+}
+
+cudaError_t encode_filter(DirectDesc& d, const void* U, bool bf16) {
+    const cuuint64_t CG = static_cast<cuuint64_t>((d.c + 7) / 8), Kr = static_cast<cuuint64_t>((d.k + 7) / 8);
+    cuuint64_t dims[4] = {64, Kr, CG, kTaps9};
+    cuuint64_t strides[3] = {128, Kr * 128, CG * Kr * 128};
+    cuuint32_t box[4] = {64, static_cast<cuuint32_t>(d.bn / 16), 2, kTaps9};
+    return encode_tiled(&d.tmU, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
+                        const_cast<void*>(U), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE) == CUDA_SUCCESS
+               ? cudaSuccess
+               : cudaErrorInvalidValue;
+}
+
+// fields of an item shape
+void set_tile(DirectDesc& d, int bn, int mb) {
+    d.bn = bn;
+    d.mb = mb;
+    d.cta_rows = kRows * mb;
+    d.win = window_of(mb, d.pw);
+    d.gran = granule_bytes(d.win);
+    d.n_blocks = (d.k + bn - 1) / bn;
+    d.fd_nb = make_fastdiv(static_cast<uint32_t>(d.n_blocks));
+}
+
+}  // namespace
+
+cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, const void* U, int tile, int num_sms) {
+    DirectDesc d{};
+    if (nhwc && g.c % 8 != 0) return cudaErrorNotSupported;   // a pixel's granule is one 16-byte load
+    d.n = g.n;
+    d.c = g.c;
+    d.h = g.h;
+    d.w = g.w;
+    d.k = g.k;
+    d.pad_h = g.pad_h;
+    d.pad_w = g.pad_w;
+    d.oh = g.oh;
+    d.ow = g.ow;
+    d.pw = g.w + std::max(g.pad_w, 2 * g.pad_w - 2);
+    d.ph = g.h + std::max(g.pad_h, 2 * g.pad_h - 2);
+    const long long img = static_cast<long long>(d.ph) * d.pw;
+    // positions, and the window's element offsets from its first image, in 32 bits
+    if (g.n * img + 4LL * d.pw + 8192 >= (1LL << 31)) return cudaErrorNotSupported;
+    d.img = static_cast<int>(img);
+    d.c_chunks = (g.c + kChunkC - 1) / kChunkC;
+    d.step_y = (2 * kGroupThreads) / g.w;
+    d.step_x = (2 * kGroupThreads) % g.w;
+    d.pad_step_i = kGroupThreads / d.pw;
+    d.pad_step_j = kGroupThreads % d.pw;
+    const long long imgs = std::min<long long>(g.n, (window_of(8, d.pw) + 2048) / img + 2);
+    if (imgs * g.c * g.h * g.w >= (1LL << 31)) return cudaErrorNotSupported;
+    d.fd_img = make_fastdiv(static_cast<uint32_t>(d.img));
+    d.fd_pw = make_fastdiv(static_cast<uint32_t>(d.pw));
+    d.fd_hw = make_fastdiv(static_cast<uint32_t>(static_cast<long long>(g.h) * g.w));
+    d.fd_w = make_fastdiv(static_cast<uint32_t>(g.w));
+    if (dp.max_pairs == 0) dp.max_pairs = max_pairs(num_sms);
+    const int bn = tile & 0x1ff, mb = tile >> 9;
+    const Split s = best_split(positions(d, g.n), g.k, d.pw, d.c_chunks, dp.max_pairs, bn, mb, true);
+    if (s.bn == 0 || !tile_fits(s.bn, s.mb, d.pw, &dp.ring)) return cudaErrorNotSupported;
+    set_tile(d, s.bn, s.mb);
+    dp.main = d;
+    dp.tail = d;
+    dp.has_tail = s.tail_bn != 0;
+    if (dp.has_tail) {
+        set_tile(dp.tail, s.tail_bn, s.tail_mb);
+        DirectRing r;
+        // one ring serves both parts: the larger stages
+        const int a = std::max((2 * d.gran + 127) / 128 * 128, (2 * dp.tail.gran + 127) / 128 * 128);
+        if (size_ring(r, a, std::max(b_stage_bytes(d.bn), b_stage_bytes(dp.tail.bn))))
+            dp.ring = r;
+        else
+            dp.has_tail = false;
+    }
+    dp.main_tiles = static_cast<int>(s.main_tiles);
+    dp.nhwc = nhwc;
+    dp.bf16 = bf16;
+    const long long rows = 2LL * s.mb * kRows;
+    if ((positions(d, g.n) + rows - 1) / rows * ((g.k + 31) / 32) >= (1LL << 30)) return cudaErrorNotSupported;
+    if (!U) return cudaSuccess;
+    cudaError_t e = encode_filter(dp.main, U, bf16);
+    if (e == cudaSuccess && dp.has_tail) e = encode_filter(dp.tail, U, bf16);
+    return e;
+}
+
+cudaError_t launch_direct_unfilter(const void* U, void* weight, int K, int C, cudaStream_t stream) {
+    const int CG = (C + 7) / 8, Kp = (K + 7) / 8 * 8;
+    const long long n = static_cast<long long>(K) * C * kTaps9;
+    direct_unfilter_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
+        static_cast<const uint16_t*>(U), static_cast<uint16_t*>(weight), K, C, CG, Kp);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_direct_filter(const void* weight, void* U, int K, int C, cudaStream_t stream) {
+    const int CG = (C + 7) / 8, Kp = (K + 7) / 8 * 8;
+    const long long n = static_cast<long long>(CG) * Kp;
+    direct_filter_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
+        static_cast<const uint16_t*>(weight), static_cast<uint16_t*>(U), K, C, CG, Kp);
+    return cudaGetLastError();
+}
+
+int direct_parts(const DirectPlan& dp, const void* x, void* y, int n_images, DirectParts& out) {
+    const long long pos = positions(dp.main, n_images);
+    auto part = [&](const DirectDesc& d, long long pos0, long long tiles, int begin) {
+        DirectDesc& o = out.d[out.count++];
+        o = d;
+        o.x = x;
+        o.y = y;
+        o.n = n_images;
+        o.pos0 = static_cast<int>(pos0);
+        o.item_begin = begin;
+        o.items = static_cast<int>(tiles * d.n_blocks);
+        // (the mask of padding positions covers 32 per thread)
+        o.pairs = !dp.nhwc && d.w % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0 && d.win <= kMaxPadBits * kGroupThreads;
+        o.vec = d.k % 8 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+        return begin + o.items;
+    };
+    const long long rows = 2LL * dp.main.cta_rows, tiles = (pos + rows - 1) / rows;
+    out.count = 0;
+    if (!dp.has_tail || tiles <= dp.main_tiles) {
+        out.items = part(dp.main, 0, tiles, 0);
+    } else {
+        const long long done = dp.main_tiles * rows, trows = 2LL * dp.tail.cta_rows;
+        out.items = part(dp.main, 0, dp.main_tiles, 0);
+        out.items = part(dp.tail, done, (pos - done + trows - 1) / trows, out.items);
+    }
+    return out.items;
+}
+
+cudaError_t launch_direct(const DirectPlan& dp, const void* x, void* y, int n_images, DevErr* err, cudaStream_t stream) {
+    DirectParts p;
+    const int pairs = std::min(direct_parts(dp, x, y, n_images, p), dp.max_pairs);
+    if (dp.nhwc)
+        return dp.bf16 ? launch_cluster(direct3x3_kernel<true, true>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
+                       : launch_cluster(direct3x3_kernel<true, false>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
+    return dp.bf16 ? launch_cluster(direct3x3_kernel<false, true>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
+                   : launch_cluster(direct3x3_kernel<false, false>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
+}
+
+}  // namespace wg

@@ -8,10 +8,12 @@
 // transform, operand type and padded sizes, the byte count and an FNV-1a
 // checksum of the payload) followed by U exactly as it lies in device memory:
 // U[E][Cp/8][Kp][8] in the operand type, or for the row F(4x3) kernel
-// U1[18][Cp16/8][Kp64][8] fp16 (its own transform code in the header).
+// U1[18][Cp16/8][Kp64][8] fp16, for the direct kernel U9[9][Cp/8][Kp][8] in the
+// tensors' type (each with its own transform code in the header).
 #include <cstdint>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -44,6 +46,13 @@ uint64_t fnv1a(const unsigned char* p, size_t n) {
     return h;
 }
 
+constexpr int32_t kDirectXform = 32;   // U9[9][Cp/8][Kp][8], the filter itself
+
+bool same_layer(const PlanFileHeader& a, const PlanFileHeader& b) {
+    return a.c == b.c && a.k == b.k && a.xform == b.xform && a.op == b.op && a.e == b.e && a.cp == b.cp && a.kp == b.kp &&
+           a.u_bytes == b.u_bytes;
+}
+
 PlanFileHeader header_of(const Plan& pl) {
     PlanFileHeader h;
     std::memset(&h, 0, sizeof(h));
@@ -56,10 +65,25 @@ PlanFileHeader header_of(const Plan& pl) {
     h.xform = static_cast<int32_t>(pl.xf) + (pl.algo == CONV2D_ALGO_4X3_ROW ? 16 : 0);   // row F(4x3): own layout
     h.op = static_cast<int32_t>(pl.op);
     h.e = static_cast<uint32_t>(pl.g.alpha * pl.g.alpha);
+    if (pl.run_direct) {
+        h.xform = kDirectXform;
+        h.e = 9;
+    }
     h.cp = static_cast<uint32_t>(pl.g.cp);
     h.kp = static_cast<uint32_t>(pl.g.kp);
     h.u_bytes = static_cast<uint64_t>(pl.u_bytes);
     return h;
+}
+
+// The plan of the Winograd algorithm that a tuned plan running the direct
+// kernel stands for: its filter files are that algorithm's, as they are where
+// the direct kernel is not the faster.  Null when it cannot be made.
+std::unique_ptr<Plan> winograd_plan(const Plan& pl) {
+    conv2d_options_t o = pl.opt;
+    o.algo = pl.algo;
+    std::unique_ptr<Plan> np(new Plan());
+    if (np->build(&pl.prob, &o) != CONV2D_OK) return nullptr;
+    return np;
 }
 
 }  // namespace
@@ -77,6 +101,19 @@ int conv2d_plan_save(const void* param, const char* path) {
     if (!pl->filter_ready || pl->opt.filter_policy == 1) {
         const int st = pl->filter(nullptr);
         if (st) return st;
+    }
+    std::unique_ptr<Plan> winograd;
+    if (pl->run_direct && pl->algo != CONV2D_ALGO_DIRECT) {
+        // from the plan's own copy of the filter: the caller's may have changed or be gone
+        void* w = nullptr;
+        if (!(winograd = winograd_plan(*pl)) || cudaMalloc(&w, static_cast<size_t>(pl->prob.k) * pl->prob.c * 18) != cudaSuccess)
+            return set_last_error(CONV2D_ERR_NOMEM, "workspace of the filter transform");
+        winograd->prob.weight = w;
+        const bool ok = launch_direct_unfilter(pl->U, w, pl->g.k, pl->g.c, nullptr) == cudaSuccess &&
+                        winograd->filter(nullptr) == CONV2D_OK && cudaDeviceSynchronize() == cudaSuccess;
+        cudaFree(w);
+        if (!ok) return set_last_error(CONV2D_ERR_CUDA, "filter transform failed");
+        pl = winograd.get();
     }
     PlanFileHeader h = header_of(*pl);
     std::vector<unsigned char> u(h.u_bytes);
@@ -98,13 +135,19 @@ int conv2d_plan_load(const void* param, const char* path) {
     PlanFileHeader h;
     std::vector<unsigned char> u;
     bool ok = std::fread(&h, sizeof(h), 1, f) == 1;
-    const PlanFileHeader want = header_of(*pl);
+    DeviceGuard dg(pl->device);
+    std::unique_ptr<Plan> winograd;
+    if (pl->run_direct && pl->algo != CONV2D_ALGO_DIRECT && !(winograd = winograd_plan(*pl))) {
+        std::fclose(f);
+        return set_last_error(CONV2D_ERR_NOMEM, "workspace of the plan file's algorithm");
+    }
+    Plan* to = winograd ? winograd.get() : pl;   // the plan the file's filter feeds from now on
+    const PlanFileHeader want = header_of(*to);
     if (ok && (std::memcmp(h.magic, kPlanMagic, 8) != 0 || h.version != 1)) {
         std::fclose(f);
         return set_last_error(CONV2D_ERR_INVALID, "not a plan file");
     }
-    if (ok && (h.c != want.c || h.k != want.k || h.xform != want.xform || h.op != want.op || h.e != want.e ||
-               h.cp != want.cp || h.kp != want.kp || h.u_bytes != want.u_bytes)) {
+    if (ok && !same_layer(h, want)) {
         std::fclose(f);
         return set_last_error(CONV2D_ERR_INVALID,
                               "plan file was made for another layer, transform or operand type");
@@ -116,11 +159,11 @@ int conv2d_plan_load(const void* param, const char* path) {
     std::fclose(f);
     if (!ok) return set_last_error(CONV2D_ERR_INVALID, "plan file truncated");
     if (fnv1a(u.data(), u.size()) != h.checksum) return set_last_error(CONV2D_ERR_INVALID, "plan file checksum mismatch");
-    DeviceGuard dg(pl->device);
     // U may still be read by work queued earlier on any stream
-    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpy(pl->U, u.data(), u.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpy(to->U, u.data(), u.size(), cudaMemcpyHostToDevice) != cudaSuccess)
         return set_last_error(CONV2D_ERR_CUDA, "copy of the transformed filter failed");
-    pl->filter_ready = true;
+    to->filter_ready = true;
+    if (winograd) replace_plan(const_cast<void*>(param), winograd.release());
     return CONV2D_OK;
 }
 

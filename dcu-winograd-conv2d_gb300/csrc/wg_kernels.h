@@ -296,6 +296,68 @@ cudaError_t launch_row4x3(const RowPlan& rp, const void* x, const void* x_end, v
 // out (which holds those images)
 cudaError_t launch_row4x3i(const RowPlan& rp, void* out, int n_base, int n_images, DevErr* err, cudaStream_t stream);
 
+// ---- direct 3x3 convolution, one fused kernel (direct3x3.cu) ---------------
+// One problem: the layout of its flattened, zero-padded positions, its
+// channel tile, and its range of the work index.
+struct alignas(64) DirectDesc {
+    CUtensorMap tmU;     // U9, boxes of bn/2 output channels x 16 input channels x 9 taps
+    const void* x;
+    void* y;
+    int n, c, h, w, k;
+    int pad_h, pad_w, oh, ow;
+    int pw, ph, img;     // positions per padded row, padded rows per image, positions per image
+    int bn, n_blocks;    // output channels per item, blocks of them
+    int mb, cta_rows;    // blocks of 128 positions per CTA and item, their positions
+    int c_chunks;        // 16-channel chunks
+    int win;             // positions of one CTA's window
+    int gran;            // bytes of one granule's window in shared memory
+    int vec;             // channels-last: 16-byte output stores
+    int pairs;           // NCHW: input read as pixel pairs
+    int step_y, step_x;          // 256 pixels as rows and columns of the input
+    int pad_step_i, pad_step_j;  // 128 positions as rows and columns of positions
+    int pos0;            // first position of item_begin's item
+    int item_begin, items;
+    FastDiv fd_nb, fd_img, fd_pw, fd_hw, fd_w;
+};
+
+// Shared-memory rings of one launch: window stages and filter stages.
+struct DirectRing {
+    int na, nb, a_bytes, b_bytes, smem_bytes;
+};
+
+// One problem's launch: whole rounds of items over the CTA pairs, and the
+// positions after them in smaller items.
+struct DirectParts {
+    DirectDesc d[2];
+    int count, items;
+};
+
+struct DirectPlan {
+    DirectDesc main, tail;
+    DirectRing ring;
+    int main_tiles;
+    int max_pairs;       // CTA pairs the device runs at once (0: not asked yet)
+    bool has_tail, nhwc, bf16;
+};
+
+// tile: output channels per item (a multiple of 32 up to 256) + 512 x blocks
+// of 128 positions per CTA (1, 2, 4 or 8, with at most 256 channels x blocks);
+// either part 0 = chosen from the sizes.  cudaErrorNotSupported when the
+// window of one CTA does not fit in shared memory (rows beyond about 1,600
+// columns), for sizes beyond 32-bit positions, and for channels-last C not a
+// multiple of 8.  U may be null (a size probe).
+cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, const void* U, int tile, int num_sms);
+// the work items of n_images images starting at x into y; returns their number
+int direct_parts(const DirectPlan& dp, const void* x, void* y, int n_images, DirectParts& out);
+long long direct_filter_bytes(int K, int C);
+int direct_threads();
+// U9[tap][Cp/8][Kp][8] from KCRS weights (16-bit values copied as they are)
+cudaError_t launch_direct_filter(const void* weight, void* U, int K, int C, cudaStream_t stream);
+// and back
+cudaError_t launch_direct_unfilter(const void* U, void* weight, int K, int C, cudaStream_t stream);
+// n_images images starting at x into y
+cudaError_t launch_direct(const DirectPlan& dp, const void* x, void* y, int n_images, DevErr* err, cudaStream_t stream);
+
 // L2 size of the current device in bytes.
 long long l2_cache_bytes();
 

@@ -32,6 +32,10 @@ struct Plan {
     int device = 0;
     int num_sms = 1;
     int algo = 0;
+    // calls run the direct kernel: asked for by name, or measured faster than
+    // `algo`, the tuner's choice among the Winograd algorithms, which the plan
+    // still stands for (reports, filter files)
+    bool run_direct = false;
     Xform xf = Xform::F2;
     OpType op = OpType::F16;
     MType mt = MType::F16;  // storage of the GEMM result M
@@ -49,6 +53,7 @@ struct Plan {
     GemmPlan gemm_full{}, gemm_tail{};
     FusedPlan fused{};
     RowPlan row{};
+    DirectPlan direct{};
     long long u_bytes = 0;   // bytes of the transformed filter U
     bool nhwc = false;   // channels-last input and output
     NhwcInDesc nh_in{};
@@ -77,7 +82,9 @@ struct Plan {
     cudaEvent_t host_ev[3 * kMaxHostChunks + 2] = {};
 
     // one kernel per call, no Winograd-domain workspace
-    bool single_kernel() const { return algo == CONV2D_ALGO_2X3_FUSED || algo == CONV2D_ALGO_4X3_ROW; }
+    bool single_kernel() const {
+        return run_direct || algo == CONV2D_ALGO_2X3_FUSED || algo == CONV2D_ALGO_4X3_ROW;
+    }
     // GEMM result row-major (M[E][P][Kp]) for the NHWC output transform of
     // fp16 / fp32 M; 24-bit M keeps the granule layout in both layouts
     bool m_row() const { return nhwc && mt != MType::F24; }
@@ -128,13 +135,16 @@ int select_reference64(unsigned long long n, unsigned long long c, unsigned long
                        unsigned long long k, unsigned long long r, unsigned long long s, unsigned long long oh,
                        unsigned long long ow);
 Plan* plan_of(const void* param);
+// Puts `plan` in place of the blob's plan, which is deleted.
+void replace_plan(void* param, Plan* plan);
 
 // Records the status and message conv2d_last_error / _message report.
 int set_last_error(int status, const char* msg);
 
 // Per-shape algorithm and GEMM tile choice for CONV2D_ALGO_AUTO
 // (autotune.cpp): measured once per shape, cached, optionally persisted.
-int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallback, int* algo, int* bn);
+// *direct: the direct kernel ran faster than that choice.
+int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallback, int* algo, int* bn, bool* direct);
 void autotune_clear();
 
 }  // namespace wg

@@ -94,8 +94,11 @@ enum {
     CONV2D_ALGO_2X3_NON_FUSED = 1,
     CONV2D_ALGO_2X3_FUSED = 2,
     CONV2D_ALGO_AUTO = 3,        /* per-shape autotuner (measures candidates once per shape) */
-    CONV2D_ALGO_4X3_ROW = 4      /* row-Winograd F(4x3), one fused kernel: 1-D F(4,3) along the
+    CONV2D_ALGO_4X3_ROW = 4,     /* row-Winograd F(4x3), one fused kernel: 1-D F(4,3) along the
                                     width, the 3 filter rows summed directly; fp16 NCHW tensors */
+    CONV2D_ALGO_DIRECT = 5       /* direct convolution, one fused kernel: an implicit GEMM over the
+                                    9 taps with exact products and fp32 sums; every tensor type and
+                                    layout of this interface */
 };
 
 /* Options for getkernelInfo_ex.  conv2d_options_default() gives the values
@@ -107,7 +110,8 @@ enum {
  * kernel) on the device, reading the problem's input and weights and writing
  * a scratch output, and keeps the reference rule's pick unless another is
  * more than 3% faster; the choice is cached per shape (and in
- * WG_CONV2D_TUNE_FILE).  On GB300 the reference rule's fused F(2x3) pick is
+ * WG_CONV2D_TUNE_FILE).  It also times the direct kernel, which calls run
+ * where it is faster than that pick (conv2d_get_direct).  On GB300 the reference rule's fused F(2x3) pick is
  * several times slower than the alternatives for wide K (e.g. 392 against
  * 115 us on 32x256x56^2 -> 256).  algo = CONV2D_ALGO_REFERENCE, or
  * WG_CONV2D_ALGO=ref, applies the reference rule (src/conv2d.cpp:83-114)
@@ -176,9 +180,16 @@ int conv2d_refresh_filter(const void* param_ptr, void* stream);
  * release path: include/common.h:174 never runs).  The blob is unusable after. */
 int conv2d_destroy(void* param_ptr);
 
-/* Selected algorithm (CONV2D_ALGO_4X3_NON_FUSED .. CONV2D_ALGO_2X3_FUSED, or
- * CONV2D_ALGO_4X3_ROW), or -1. */
+/* Selected algorithm (CONV2D_ALGO_4X3_NON_FUSED .. CONV2D_ALGO_2X3_FUSED,
+ * CONV2D_ALGO_4X3_ROW, or CONV2D_ALGO_DIRECT when asked for by name), or -1. */
 int conv2d_get_algo(const void* param_ptr);
+
+/* 1 when conv2d calls of this blob run the direct kernel: asked for as
+ * CONV2D_ALGO_DIRECT, or, under CONV2D_ALGO_AUTO, measured faster than the
+ * selected algorithm (which conv2d_get_algo still reports, and whose filter
+ * files conv2d_plan_save and _load still use; after a load the blob runs that
+ * algorithm, from the file's filter).  0 otherwise, -1 for a bad blob. */
+int conv2d_get_direct(const void* param_ptr);
 
 /* Device workspace bytes held by the blob. */
 long long conv2d_workspace_bytes(const void* param_ptr);
