@@ -7,7 +7,9 @@
 //     transform family, the GEMMs of all problems in one persistent launch
 //     per (channel tile, M type) whose work queue holds every (problem,
 //     element, tile block, channel block) item, the output transforms in one
-//     launch per family -- captured once into a CUDA graph and replayed; or
+//     launch per family, the problems that run the direct kernel in one
+//     launch over all their items -- captured once into a CUDA graph and
+//     replayed; or
 //   * per call: each problem's own launches, one problem after another
 //     (the comparison the grouped run is measured against).
 // Both use the same workspaces, so their results are bit-identical.
@@ -62,6 +64,12 @@ struct Batch {
     std::vector<InGroup> in_groups;
     std::vector<GemmGroup> gemm_groups;
     std::vector<OutGroup> out_groups;
+    // problems that run the direct kernel: one launch over all of them
+    struct DirectGroup {
+        const DirectDesc* descs = nullptr;
+        int n = 0, items = 0, pairs = 0;
+        DirectRing ring{};
+    } direct;
     std::vector<int> fused;      // problems run by their own fused kernel
     std::vector<int> scaled;     // problems whose tile scale is computed per problem
     cudaGraphExec_t graph = nullptr;
@@ -91,11 +99,12 @@ struct Batch {
     struct Unit {
         Xform xf;      // chain: transform and GEMM tile
         int bn;
-        int single;    // or the problem run by its own kernel (>= 0)
+        int single;    // or the problem run by its own kernel (>= 0), or kDirectUnit
         double flops;  // direct-convolution work
         int stream;    // 0: the caller's stream, k: side[k - 1]
     };
     std::vector<Unit> units;
+    static constexpr int kChainUnit = -1, kDirectUnit = -2;
 
     cudaError_t launch_chain(Xform xf, int bn, cudaStream_t s) {
         cudaError_t e = cudaSuccess;
@@ -122,6 +131,8 @@ struct Batch {
     }
 
     cudaError_t launch_unit(const Unit& u, cudaStream_t s) {
+        if (u.single == kDirectUnit)
+            return launch_direct_grouped(direct.descs, direct.n, direct.items, direct.ring, direct.pairs, err, s);
         return u.single >= 0 ? launch_single(u.single, s) : launch_chain(u.xf, u.bn, s);
     }
 
@@ -148,8 +159,6 @@ struct Batch {
         Plan& p = *plans[i];
         const void* x_end =
             static_cast<const uint16_t*>(p.prob.in) + static_cast<long long>(p.prob.n) * p.g.c * p.g.h * p.g.w;
-        if (p.run_direct)
-            return launch_direct(p.direct, p.prob.in, p.prob.out, static_cast<int>(p.prob.n), err, s);
         if (p.algo == CONV2D_ALGO_4X3_ROW)
             return launch_row4x3(p.row, p.prob.in, x_end, p.prob.out, static_cast<int>(p.prob.n), err, s);
         return launch_fused2x3(p.fused, p.g, p.prob.in, x_end, p.prob.out, err, s);
@@ -188,8 +197,15 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     const char* sb = std::getenv("WG_CONV2D_BATCH_SPLIT_BN");
     const bool split_bn = sb && sb[0] == '1';
     std::map<std::tuple<int, int, int, int>, std::vector<int>> gemm_keys;     // (bn, M type, op, xform) -> problems
+    std::vector<DirectProblem> direct_probs;
+    double direct_flops = 0;
     for (int i = 0; i < count; ++i) {
         Plan& p = *b->plans[i];
+        if (p.run_direct) {
+            direct_probs.push_back({p.g, p.prob.in, p.prob.out, p.U});
+            direct_flops += 18.0 * p.prob.n * p.prob.k * p.g.oh * p.g.ow * p.prob.c;
+            continue;
+        }
         if (p.single_kernel()) {
             b->fused.push_back(i);
             continue;
@@ -250,9 +266,18 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
         }
         gemm_r.push_back({kv.first, r});
     }
-    // one device block: error word | GemmDesc[] (64-byte aligned) | InDesc[] | OutDesc[]
+    std::vector<DirectDesc> direct_descs(direct_probs.size());
+    if (!direct_probs.empty()) {
+        b->direct.n = static_cast<int>(direct_probs.size());
+        b->direct.pairs = direct_max_pairs(b->plans[0]->num_sms);
+        if (make_direct_group(direct_probs.data(), b->direct.n, b->direct.pairs, direct_descs.data(), b->direct.ring,
+                              b->direct.items) != cudaSuccess)
+            return batch_fail(CONV2D_ERR_CUDA, "direct kernel descriptors");
+    }
+    // one device block: error word | GemmDesc[] and DirectDesc[] (64-byte aligned) | InDesc[] | OutDesc[]
     auto al = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t oE = 0, oG = 256, oI = oG + al(gemm_descs.size() * sizeof(GemmDesc)),
+    const size_t oE = 0, oG = 256, oD = oG + al(gemm_descs.size() * sizeof(GemmDesc)),
+                 oI = oD + al(direct_descs.size() * sizeof(DirectDesc)),
                  oO = oI + al(in_descs.size() * sizeof(InDesc)), total = oO + al(out_descs.size() * sizeof(OutDesc));
     if (cudaMalloc(&b->dev, total) != cudaSuccess) {
         cudaGetLastError();
@@ -262,6 +287,10 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     b->err = reinterpret_cast<DevErr*>(base + oE);
     cudaMemset(b->err, 0, sizeof(DevErr));
     if (!gemm_descs.empty()) cudaMemcpy(base + oG, gemm_descs.data(), gemm_descs.size() * sizeof(GemmDesc), cudaMemcpyHostToDevice);
+    if (!direct_descs.empty()) {
+        cudaMemcpy(base + oD, direct_descs.data(), direct_descs.size() * sizeof(DirectDesc), cudaMemcpyHostToDevice);
+        b->direct.descs = reinterpret_cast<const DirectDesc*>(base + oD);
+    }
     if (!in_descs.empty()) cudaMemcpy(base + oI, in_descs.data(), in_descs.size() * sizeof(InDesc), cudaMemcpyHostToDevice);
     if (!out_descs.empty()) cudaMemcpy(base + oO, out_descs.data(), out_descs.size() * sizeof(OutDesc), cudaMemcpyHostToDevice);
     int sms = b->plans[0]->num_sms;
@@ -282,7 +311,7 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     int single = 0;   // launches of the problems run by their own kernels
     for (int i : b->fused) single += b->plans[i]->launches;
     b->grouped_launches = static_cast<int>(b->scaled.size() + b->in_groups.size() + b->gemm_groups.size() +
-                                           b->out_groups.size()) + single;
+                                           b->out_groups.size()) + single + (b->direct.n ? 1 : 0);
     if (cudaDeviceSynchronize() != cudaSuccess) return batch_fail(CONV2D_ERR_CUDA, "batch setup failed");
     // work units (chains and single-kernel problems), largest first, each to
     // the stream with the least direct-convolution work so far
@@ -292,9 +321,9 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     };
     for (const Batch::InGroup& g : b->in_groups) {
         bool seen = false;   // one unit per chain, whatever its operand types
-        for (const Batch::Unit& v : b->units) seen = seen || (v.single < 0 && v.xf == g.xf && v.bn == g.bn);
+        for (const Batch::Unit& v : b->units) seen = seen || (v.single == Batch::kChainUnit && v.xf == g.xf && v.bn == g.bn);
         if (seen) continue;
-        Batch::Unit u{g.xf, g.bn, -1, 0.0, 0};
+        Batch::Unit u{g.xf, g.bn, Batch::kChainUnit, 0.0, 0};
         for (int i = 0; i < count; ++i) {
             const Plan& p = *b->plans[i];
             if (!p.single_kernel() && p.xf == g.xf && (g.bn == 0 || p.gemm_full.bn == g.bn)) u.flops += flops(i);
@@ -302,6 +331,7 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
         b->units.push_back(u);
     }
     for (int i : b->fused) b->units.push_back({Xform::F2, 0, i, flops(i), 0});
+    if (b->direct.n) b->units.push_back({Xform::F2, 0, Batch::kDirectUnit, direct_flops, 0});
     std::stable_sort(b->units.begin(), b->units.end(),
                      [](const Batch::Unit& x, const Batch::Unit& y) { return x.flops > y.flops; });
     {

@@ -43,7 +43,8 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <cstring>
+#include <atomic>
+#include <vector>
 
 #include "wg_kernels.h"
 #include "wg_launch.h"
@@ -655,6 +656,13 @@ __global__ void __launch_bounds__(kDirectThreads, 1)
     direct_body<NHWC, BF16>(parts.d, parts.count, parts.items, ring, err);
 }
 
+// Many problems (fp16 NCHW) as one work queue; descs device-resident, sorted by item_begin.
+__global__ void __launch_bounds__(kDirectThreads, 1)
+    direct3x3_grouped(const DirectDesc* __restrict__ descs, int ndesc, int items, const __grid_constant__ DirectRing ring,
+                      DevErr* err) {
+    direct_body<false, false>(descs, ndesc, items, ring, err);
+}
+
 // U9[tap][Cp/8][Kp][8]: the KCRS filter as granules of 8 input channels, zero
 // past C and K.  One thread per (output channel, granule).
 __global__ void __launch_bounds__(256) direct_filter_kernel(const uint16_t* __restrict__ w, uint16_t* __restrict__ U, int K,
@@ -856,10 +864,8 @@ void set_tile(DirectDesc& d, int bn, int mb) {
     d.fd_nb = make_fastdiv(static_cast<uint32_t>(d.n_blocks));
 }
 
-}  // namespace
-
-cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, const void* U, int tile, int num_sms) {
-    DirectDesc d{};
+cudaError_t describe_direct(DirectDesc& d, const Geom& g, bool nhwc) {
+    d = DirectDesc{};
     if (nhwc && g.c % 8 != 0) return cudaErrorNotSupported;   // a pixel's granule is one 16-byte load
     d.n = g.n;
     d.c = g.c;
@@ -870,24 +876,60 @@ cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, con
     d.pad_w = g.pad_w;
     d.oh = g.oh;
     d.ow = g.ow;
-    d.pw = g.w + std::max(g.pad_w, 2 * g.pad_w - 2);
-    d.ph = g.h + std::max(g.pad_h, 2 * g.pad_h - 2);
-    const long long img = static_cast<long long>(d.ph) * d.pw;
-    // positions, and the window's element offsets from its first image, in 32 bits
-    if (g.n * img + 4LL * d.pw + 8192 >= (1LL << 31)) return cudaErrorNotSupported;
+    const long long pw = static_cast<long long>(g.w) + std::max(g.pad_w, 2 * g.pad_w - 2);
+    const long long ph = static_cast<long long>(g.h) + std::max(g.pad_h, 2 * g.pad_h - 2), img = ph * pw;
+    // positions (with what the last items reach past them) and the window's
+    // element offsets from its first image, in 32 bits
+    if (g.n * img + 4 * pw + 8192 >= (1LL << 31)) return cudaErrorNotSupported;
+    d.pw = static_cast<int>(pw);
+    d.ph = static_cast<int>(ph);
     d.img = static_cast<int>(img);
+    const long long imgs = std::min<long long>(g.n, (window_of(8, d.pw) + 2048) / img + 2);
+    if (imgs * g.c * g.h * g.w >= (1LL << 31)) return cudaErrorNotSupported;
+    // items of the smallest tile
+    if ((positions(d, g.n) / (2 * kRows) + 1) * ((g.k + 31) / 32) >= (1LL << 30)) return cudaErrorNotSupported;
     d.c_chunks = (g.c + kChunkC - 1) / kChunkC;
     d.step_y = (2 * kGroupThreads) / g.w;
     d.step_x = (2 * kGroupThreads) % g.w;
     d.pad_step_i = kGroupThreads / d.pw;
     d.pad_step_j = kGroupThreads % d.pw;
-    const long long imgs = std::min<long long>(g.n, (window_of(8, d.pw) + 2048) / img + 2);
-    if (imgs * g.c * g.h * g.w >= (1LL << 31)) return cudaErrorNotSupported;
     d.fd_img = make_fastdiv(static_cast<uint32_t>(d.img));
     d.fd_pw = make_fastdiv(static_cast<uint32_t>(d.pw));
     d.fd_hw = make_fastdiv(static_cast<uint32_t>(static_cast<long long>(g.h) * g.w));
     d.fd_w = make_fastdiv(static_cast<uint32_t>(g.w));
-    if (dp.max_pairs == 0) dp.max_pairs = max_pairs(num_sms);
+    return cudaSuccess;
+}
+
+// the descriptor's tensors, and its items [begin, begin + tiles * n_blocks) from position pos0
+void place(DirectDesc& d, const void* x, void* y, bool nhwc, long long pos0, long long tiles, int begin) {
+    d.x = x;
+    d.y = y;
+    d.pos0 = static_cast<int>(pos0);
+    d.item_begin = begin;
+    d.items = static_cast<int>(tiles * d.n_blocks);
+    // (the mask of padding positions covers 32 per thread)
+    d.pairs = !nhwc && d.w % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0 && d.win <= kMaxPadBits * kGroupThreads;
+    d.vec = d.k % 8 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+}
+
+}  // namespace
+
+int direct_max_pairs(int num_sms) {
+    static std::atomic<int> cached{0};   // one device type per process; the same answer from every thread
+    int n = cached.load();
+    if (n == 0) cached.store(n = max_pairs(num_sms));
+    return n;
+}
+
+bool direct_supported(const Geom& g, bool nhwc) {
+    DirectDesc d;
+    return describe_direct(d, g, nhwc) == cudaSuccess && tile_fits(32, 1, d.pw, nullptr);
+}
+
+cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, const void* U, int tile, int num_sms) {
+    DirectDesc d;
+    if (cudaError_t e = describe_direct(d, g, nhwc); e != cudaSuccess) return e;
+    dp.max_pairs = direct_max_pairs(num_sms);
     const int bn = tile & 0x1ff, mb = tile >> 9;
     const Split s = best_split(positions(d, g.n), g.k, d.pw, d.c_chunks, dp.max_pairs, bn, mb, true);
     if (s.bn == 0 || !tile_fits(s.bn, s.mb, d.pw, &dp.ring)) return cudaErrorNotSupported;
@@ -908,8 +950,6 @@ cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, con
     dp.main_tiles = static_cast<int>(s.main_tiles);
     dp.nhwc = nhwc;
     dp.bf16 = bf16;
-    const long long rows = 2LL * s.mb * kRows;
-    if ((positions(d, g.n) + rows - 1) / rows * ((g.k + 31) / 32) >= (1LL << 30)) return cudaErrorNotSupported;
     if (!U) return cudaSuccess;
     cudaError_t e = encode_filter(dp.main, U, bf16);
     if (e == cudaSuccess && dp.has_tail) e = encode_filter(dp.tail, U, bf16);
@@ -937,15 +977,8 @@ int direct_parts(const DirectPlan& dp, const void* x, void* y, int n_images, Dir
     auto part = [&](const DirectDesc& d, long long pos0, long long tiles, int begin) {
         DirectDesc& o = out.d[out.count++];
         o = d;
-        o.x = x;
-        o.y = y;
         o.n = n_images;
-        o.pos0 = static_cast<int>(pos0);
-        o.item_begin = begin;
-        o.items = static_cast<int>(tiles * d.n_blocks);
-        // (the mask of padding positions covers 32 per thread)
-        o.pairs = !dp.nhwc && d.w % 2 == 0 && reinterpret_cast<uintptr_t>(x) % 4 == 0 && d.win <= kMaxPadBits * kGroupThreads;
-        o.vec = d.k % 8 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+        place(o, x, y, dp.nhwc, pos0, tiles, begin);
         return begin + o.items;
     };
     const long long rows = 2LL * dp.main.cta_rows, tiles = (pos + rows - 1) / rows;
@@ -958,6 +991,81 @@ int direct_parts(const DirectPlan& dp, const void* x, void* y, int n_images, Dir
         out.items = part(dp.tail, done, (pos - done + trows - 1) / trows, out.items);
     }
     return out.items;
+}
+
+// Item shapes for a queue of many problems: throughput decides (items x
+// cycles), not rounds, as the problems fill each other's; but no item longer
+// than a third of the queue's time where a shorter one is to be had.  Longest
+// items first, so that the pairs, which take the items in turn, end together.
+cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDesc* out, DirectRing& ring, int& items) {
+    struct Pick {
+        DirectDesc d;
+        double one;
+        int i;
+    };
+    std::vector<Pick> picks(n);
+    // stages small enough for four of each
+    auto fits = [](int bn, int mb, int pw) {
+        DirectRing r;
+        return tile_fits(bn, mb, pw, &r) && (mb == 1 || r.a_bytes <= 18 * 1024);
+    };
+    auto choose = [&](Pick& k, double longest) {
+        const long long pos = positions(k.d, k.d.n);
+        double best = 0;
+        int bbn = 0, bmb = 0;
+        for (int mb = 1; mb <= 8; mb *= 2)
+            for (int bn = 32; bn <= 256; bn += 32) {
+                if (!fits(bn, mb, k.d.pw)) continue;
+                const double one = item_cycles(bn, mb, k.d.pw, k.d.c_chunks);
+                const long long rows = 2LL * kRows * mb;
+                double t = static_cast<double>((pos + rows - 1) / rows * ((k.d.k + bn - 1) / bn)) * one;
+                if (longest > 0 && one > longest) t *= one / longest;
+                if (bbn == 0 || t < best) {
+                    best = t;
+                    bbn = bn;
+                    bmb = mb;
+                }
+            }
+        if (bbn == 0) return -1.0;
+        set_tile(k.d, bbn, bmb);
+        k.one = item_cycles(bbn, bmb, k.d.pw, k.d.c_chunks);
+        return best;
+    };
+    double total = 0;
+    for (int i = 0; i < n; ++i) {
+        if (cudaError_t e = describe_direct(picks[i].d, p[i].g, false); e != cudaSuccess) return e;
+        picks[i].i = i;
+        const double t = choose(picks[i], 0);
+        if (t < 0) return cudaErrorNotSupported;
+        total += t;
+    }
+    const double longest = total / pairs / 3;
+    int a = 0, b = 0;
+    for (Pick& k : picks) {
+        if (k.one > longest) choose(k, longest);
+        a = std::max(a, (2 * k.d.gran + 127) / 128 * 128);
+        b = std::max(b, b_stage_bytes(k.d.bn));
+    }
+    if (!size_ring(ring, a, b)) return cudaErrorNotSupported;
+    std::stable_sort(picks.begin(), picks.end(), [](const Pick& x, const Pick& y) { return x.one > y.one; });
+    long long begin = 0;
+    for (int i = 0; i < n; ++i) {
+        DirectDesc& d = picks[i].d;
+        const DirectProblem& q = p[picks[i].i];
+        if (cudaError_t e = encode_filter(d, q.U, false); e != cudaSuccess) return e;
+        const long long rows = 2LL * d.cta_rows;
+        place(d, q.x, q.y, false, 0, (positions(d, d.n) + rows - 1) / rows, static_cast<int>(begin));
+        begin += d.items;
+        if (begin >= (1LL << 31)) return cudaErrorNotSupported;
+        out[i] = d;
+    }
+    items = static_cast<int>(begin);
+    return cudaSuccess;
+}
+
+cudaError_t launch_direct_grouped(const DirectDesc* descs, int ndesc, int items, const DirectRing& ring, int pairs, DevErr* err,
+                                  cudaStream_t stream) {
+    return launch_cluster(direct3x3_grouped, std::min(items, pairs), ring.smem_bytes, stream, descs, ndesc, items, ring, err);
 }
 
 cudaError_t launch_direct(const DirectPlan& dp, const void* x, void* y, int n_images, DevErr* err, cudaStream_t stream) {

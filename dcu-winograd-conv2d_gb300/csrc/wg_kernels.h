@@ -336,7 +336,7 @@ struct DirectPlan {
     DirectDesc main, tail;
     DirectRing ring;
     int main_tiles;
-    int max_pairs;       // CTA pairs the device runs at once (0: not asked yet)
+    int max_pairs;       // CTA pairs the device runs at once
     bool has_tail, nhwc, bf16;
 };
 
@@ -349,6 +349,22 @@ struct DirectPlan {
 cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, const void* U, int tile, int num_sms);
 // the work items of n_images images starting at x into y; returns their number
 int direct_parts(const DirectPlan& dp, const void* x, void* y, int n_images, DirectParts& out);
+// One problem (fp16 NCHW) of a queue of many.
+struct DirectProblem {
+    Geom g;
+    const void* x;
+    void* y;
+    const void* U;       // U9
+};
+// Whether the direct kernel takes these sizes.
+bool direct_supported(const Geom& g, bool nhwc);
+// CTA pairs the device runs at once.
+int direct_max_pairs(int num_sms);
+// Descriptors (out[n], sorted by item_begin, to be copied to the device) and
+// ring of one launch over n problems.
+cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDesc* out, DirectRing& ring, int& items);
+cudaError_t launch_direct_grouped(const DirectDesc* descs, int ndesc, int items, const DirectRing& ring, int pairs, DevErr* err,
+                                  cudaStream_t stream);
 long long direct_filter_bytes(int K, int C);
 int direct_threads();
 // U9[tap][Cp/8][Kp][8] from KCRS weights (16-bit values copied as they are)

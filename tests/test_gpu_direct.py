@@ -142,3 +142,40 @@ def test_filter_files(wg, tmp_path, monkeypatch):
                 a.load(own)
     finally:
         wg.lib().conv2d_autotune_clear()
+
+
+def test_one_queue_of_many_problems(wg, tmp_path, monkeypatch):
+    """A batch whose problems all run the direct kernel: one launch, exact on
+    integers, from one pixel to several rounds of items, odd and even rows."""
+    shapes = [(1, 3, 1, 1, 1), (2, 16, 7, 7, 40), (20, 32, 40, 40, 256), (3, 17, 13, 9, 33), (1, 64, 56, 56, 64),
+              (1, 20, 5, 300, 8), (40, 33, 7, 7, 300)]
+    tune = tmp_path / "tune"
+    tune.write_text("".join(f"{n} {c} {h} {w} {k} 1 1 0 0 0 {wg.ALGO_2X3 + 16} 0 0.1\n" for n, c, h, w, k in shapes))
+    monkeypatch.setenv("WG_CONV2D_TUNE_FILE", str(tune))
+    wg.lib().conv2d_autotune_clear()
+    g = torch.Generator().manual_seed(3)
+    try:
+        probs, keep = [], []
+        for n, c, h, w, k in shapes:
+            x = torch.randint(-2, 3, (n, c, h, w), generator=g).double()
+            f = torch.randint(-1, 2, (k, c, 3, 3), generator=g).double()
+            want = torch.nn.functional.conv2d(x, f, padding=1).half()
+            xd, fd = x.half().cuda(), f.half().cuda()
+            y = torch.zeros((n, k, h, w), dtype=torch.float16, device="cuda")
+            probs.append(wg.make_problem(xd.data_ptr(), fd.data_ptr(), y.data_ptr(), n, c, h, w, k))
+            keep.append((xd, fd, y, want))
+        b = wg.Batch(probs, wg.default_options(algo=wg.ALGO_AUTO))
+    finally:
+        wg.lib().conv2d_autotune_clear()
+    assert b.launches(True) == 1 and b.launches(False) == len(shapes)
+    s = torch.cuda.current_stream().cuda_stream
+    for _ in range(3):   # direct launches, then the recorded graph
+        for _, _, y, _ in keep:
+            y.zero_()
+        b.run(s)
+        torch.cuda.synchronize()
+        st, site = b.check_device()
+        assert st == wg.OK, site
+        for i, (_, _, y, want) in enumerate(keep):
+            assert torch.equal(y.cpu(), want), i
+    b.destroy()
