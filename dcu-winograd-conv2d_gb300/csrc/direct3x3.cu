@@ -810,35 +810,46 @@ bool tile_fits(int bn, int mb, int pw, DirectRing* ring) {
     return true;
 }
 
-// Least rounds x cycles for `pos` positions over `pairs` pairs.
-Split best_split(long long pos, int K, int pw, int chunks, int pairs, int only_bn, int only_mb, bool tail) {
+// Cycles of every item shape that fits (0: does not), by log2 mb and bn / 32 - 1.
+struct TileCosts {
+    double one[4][8];
+    TileCosts(int pw, int chunks, int only_bn, int only_mb) {
+        for (int i = 0; i < 4; ++i)
+            for (int j = 0; j < 8; ++j) {
+                const int mb = 1 << i, bn = 32 * (j + 1);
+                const bool out = (only_mb && mb != only_mb) || (only_bn && bn != only_bn) || !tile_fits(bn, mb, pw, nullptr);
+                one[i][j] = out ? 0 : item_cycles(bn, mb, pw, chunks);
+            }
+    }
+};
+
+// Least rounds x cycles for `pos` positions over `pairs` pairs; with `tail`,
+// the positions past the last whole round may take another shape.
+Split best_split(long long pos, int K, int pairs, const TileCosts& cost, const TileCosts* tail) {
     Split best;
-    for (int mb = 1; mb <= 8; mb *= 2) {
-        if (only_mb && mb != only_mb) continue;
-        for (int bn = 32; bn <= 256; bn += 32) {
-            if (only_bn && bn != only_bn) continue;
-            if (!tile_fits(bn, mb, pw, nullptr)) continue;
-            const long long rows = 2LL * kRows * mb;
-            const long long tiles = (pos + rows - 1) / rows, nb = (K + bn - 1) / bn, items = tiles * nb;
-            const double one = item_cycles(bn, mb, pw, chunks);
+    for (int i = 0; i < 4; ++i)
+        for (int j = 0; j < 8; ++j) {
+            const double one = cost.one[i][j];
+            if (one == 0) continue;
             Split s;
-            s.bn = bn;
-            s.mb = mb;
+            s.mb = 1 << i;
+            s.bn = 32 * (j + 1);
+            const long long rows = 2LL * kRows * s.mb;
+            const long long tiles = (pos + rows - 1) / rows, nb = (K + s.bn - 1) / s.bn, items = tiles * nb;
             s.main_tiles = tiles;
             s.cycles = static_cast<double>((items + pairs - 1) / pairs) * one;
             if (best.bn == 0 || s.cycles < best.cycles) best = s;
             // whole rounds in the main part, the rest in items that take less than one more round
-            const long long rounds = items / pairs, main = rounds * pairs / nb;
-            if (tail && main > 0 && main < tiles) {
-                const Split t = best_split(pos - main * rows, K, pw, chunks, pairs, 0, 0, false);
-                s.main_tiles = main;
-                s.tail_bn = t.bn;
-                s.tail_mb = t.mb;
-                s.cycles = static_cast<double>((main * nb + pairs - 1) / pairs) * one + t.cycles;
-                if (s.cycles < best.cycles) best = s;
-            }
+            const long long main = items / pairs * pairs / nb;
+            const double main_cycles = static_cast<double>((main * nb + pairs - 1) / pairs) * one;
+            if (!tail || main <= 0 || main >= tiles || main_cycles >= best.cycles) continue;
+            const Split t = best_split(pos - main * rows, K, pairs, *tail, nullptr);
+            s.main_tiles = main;
+            s.tail_bn = t.bn;
+            s.tail_mb = t.mb;
+            s.cycles = main_cycles + t.cycles;
+            if (s.cycles < best.cycles) best = s;
         }
-    }
     return best;
 }
 
@@ -931,7 +942,8 @@ cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, con
     if (cudaError_t e = describe_direct(d, g, nhwc); e != cudaSuccess) return e;
     dp.max_pairs = direct_max_pairs(num_sms);
     const int bn = tile & 0x1ff, mb = tile >> 9;
-    const Split s = best_split(positions(d, g.n), g.k, d.pw, d.c_chunks, dp.max_pairs, bn, mb, true);
+    const TileCosts any(d.pw, d.c_chunks, 0, 0), asked(d.pw, d.c_chunks, bn, mb);
+    const Split s = best_split(positions(d, g.n), g.k, dp.max_pairs, asked, &any);
     if (s.bn == 0 || !tile_fits(s.bn, s.mb, d.pw, &dp.ring)) return cudaErrorNotSupported;
     set_tile(d, s.bn, s.mb);
     dp.main = d;

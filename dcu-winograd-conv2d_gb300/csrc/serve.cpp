@@ -1,8 +1,8 @@
 // Serving loop: continuous batching of conv2d requests over resident layers.
 //
 // A server owns
-//   * layers: the filter of each is transformed once, for F(2x3) and F(4x3),
-//     and stays on the device;
+//   * layers: the filter of each is laid out once for the direct kernel and
+//     transformed once for F(2x3) and F(4x3), and stays on the device;
 //   * a workspace arena of the configured HBM budget, from which every
 //     admitted request takes its Winograd-domain buffers (V and M) and to
 //     which it returns them when it completes;
@@ -12,7 +12,8 @@
 // `max_batch` requests), and launches the batch as grouped kernels on a free
 // slot: one input-transform launch per transform family, one persistent GEMM
 // launch per (channel tile, M type) over every request's tiles, one
-// output-transform launch per family.  Requests that arrive while other
+// output-transform launch per family, and one launch over the items of every
+// request that runs the direct kernel.  Requests that arrive while other
 // batches are on the GPU are admitted as soon as a slot and workspace free
 // up, and their batch runs concurrently with the ones still in flight.
 // A request's arithmetic does not depend on what else is in its batch, so its
@@ -108,6 +109,7 @@ struct Layer {
     unsigned c, k, h, w, p, q;
     void* U2 = nullptr;  // F(2x3) transformed filter
     void* U4 = nullptr;  // F(4x3)
+    void* U9 = nullptr;  // direct (none in a layer loaded from a file without it)
 };
 
 struct Request {
@@ -117,7 +119,8 @@ struct Request {
     const void* in;
     void* out;
     double t_arrive, t_start = 0, t_done = 0;
-    int m;              // 2 or 4
+    int m;              // 2 or 4: the transform its workspace is sized for
+    bool direct;        // runs the direct kernel
     size_t ws_off = 0, ws_bytes = 0;
     bool done = false;
 };
@@ -136,7 +139,7 @@ struct Slot {
     bool busy = false;
 };
 
-constexpr size_t kDescBytesPerRequest = sizeof(GemmDesc) + sizeof(InDesc) + sizeof(OutDesc) + 256;
+constexpr size_t kDescBytesPerRequest = sizeof(GemmDesc) + sizeof(InDesc) + sizeof(OutDesc) + sizeof(DirectDesc) + 256;
 
 }  // namespace
 
@@ -218,6 +221,16 @@ struct Server {
         return (std::min(L.c, L.k) >= 128 && L.h >= 14 && L.w >= 14) ? 4 : 2;
     }
 
+    // The direct kernel holds about 1,430 TFLOP/s of direct-convolution work
+    // under the power cap whatever the channels; F(4x3), whose traffic per
+    // product falls as they grow, passes it from about 512 x 512 channels on
+    // (32 x 28^2: 70.9 against 80 us; at 256 x 256 101.6 against 82.5 on 56^2).
+    bool choose_direct(const Layer& L, unsigned n) const {
+        if (cfg.algo != CONV2D_ALGO_AUTO || !L.U9) return false;
+        if (std::min(L.c, L.k) >= 512 && L.h >= 14 && L.w >= 14) return false;
+        return direct_supported(make_geom(static_cast<int>(n), L.c, L.h, L.w, L.k, L.p, L.q, 2), false);
+    }
+
     // launch one batch (requests already admitted: workspace assigned)
     int launch(Slot& slot) {
         std::vector<InDesc> in2, in4;
@@ -226,9 +239,14 @@ struct Server {
         long long blk_in2 = 0, blk_in4 = 0, blk_out2 = 0, blk_out4 = 0;
         int smem2 = 0, smem4 = 0;
         char* arena = static_cast<char*>(arena_base);
+        std::vector<DirectProblem> direct;
         for (long long id : slot.reqs) {
             Request& r = reqs[id];
             const Layer& L = layers[r.layer];
+            if (r.direct) {
+                direct.push_back({make_geom(r.n, L.c, L.h, L.w, L.k, L.p, L.q, 2), r.in, r.out, L.U9});
+                continue;
+            }
             const Geom g = make_geom(r.n, L.c, L.h, L.w, L.k, L.p, L.q, r.m);
             const int E = g.alpha * g.alpha;
             char* V = arena + r.ws_off;
@@ -281,6 +299,16 @@ struct Server {
             gg.push_back({kv.first.first, kv.first.second, off, static_cast<int>(kv.second.size()), t});
             off += kv.second.size() * sizeof(GemmDesc);
         }
+        std::vector<DirectDesc> dd(direct.size());
+        DirectRing ring{};
+        int direct_items = 0;
+        const int pairs = direct.empty() ? 0 : direct_max_pairs(num_sms);
+        if (!direct.empty() && make_direct_group(direct.data(), static_cast<int>(direct.size()), pairs, dd.data(), ring,
+                                                 direct_items) != cudaSuccess)
+            return set_last_error(CONV2D_ERR_CUDA, "direct kernel descriptors");
+        const size_t o_direct = off;
+        std::memcpy(h + off, dd.data(), dd.size() * sizeof(DirectDesc));
+        off += dd.size() * sizeof(DirectDesc);
         const size_t o_in2 = off;
         std::memcpy(h + off, in2.data(), in2.size() * sizeof(InDesc));
         off += in2.size() * sizeof(InDesc);
@@ -299,14 +327,17 @@ struct Server {
         if (cudaMemcpyAsync(d, h, off, cudaMemcpyHostToDevice, s) != cudaSuccess)
             return set_last_error(CONV2D_ERR_CUDA, "descriptor copy failed");
         cudaError_t e = cudaSuccess;
-        // with requests of both transforms, the F(2x3) chain goes to stream2
-        // (forked after the descriptor copy, joined before `done`) and runs
-        // beside the F(4x3) chain
-        const bool both = !in2.empty() && !in4.empty();
+        // with requests of several kinds, the F(4x3) chain (or, without one, the
+        // direct launch) stays on the slot's stream and the others go to stream2
+        // (forked after the descriptor copy, joined before `done`) beside it
+        const bool both = (in2.empty() ? 0 : 1) + (in4.empty() ? 0 : 1) + (dd.empty() ? 0 : 1) > 1;
         cudaStream_t s2 = both ? slot.stream2 : s;
         if (both) {
             if ((e = cudaEventRecord(slot.fork, s)) == cudaSuccess) e = cudaStreamWaitEvent(s2, slot.fork, 0);
         }
+        if (!dd.empty() && e == cudaSuccess)
+            e = launch_direct_grouped(reinterpret_cast<const DirectDesc*>(d + o_direct), static_cast<int>(dd.size()),
+                                      direct_items, ring, pairs, err, in4.empty() ? s : s2);
         if (!in2.empty() && e == cudaSuccess)
             e = launch_input_transform_grouped(Xform::F2, OpType::F16, reinterpret_cast<const InDesc*>(d + o_in2),
                                                static_cast<int>(in2.size()), blk_in2, smem2, false, err, s2);
@@ -342,6 +373,13 @@ struct Server {
         const Layer& L = layers[r.layer];
         const Geom g = make_geom(r.n, L.c, L.h, L.w, L.k, L.p, L.q, r.m);
         const int E = g.alpha * g.alpha;
+        cudaError_t e = cudaSuccess;
+        if (r.direct) {
+            DirectPlan dp{};
+            e = plan_direct(dp, g, false, false, L.U9, 0, num_sms);
+            if (e == cudaSuccess) e = launch_direct(dp, r.in, r.out, static_cast<int>(r.n), err, plain_stream);
+            return finish_plain(r, e);
+        }
         // requests run in stream order: all of them use the arena's start
         char* V = static_cast<char*>(arena_base);
         char* Mw = V + (static_cast<size_t>(E) * round_rows(g.P) * g.cp * 2 + 255) / 256 * 256;
@@ -351,9 +389,14 @@ struct Server {
                       default_bn(static_cast<int>(L.k)), num_sms) != cudaSuccess)
             return set_last_error(CONV2D_ERR_CUDA, "tensor map encoding failed");
         const void* x_end = static_cast<const uint16_t*>(r.in) + static_cast<long long>(r.n) * L.c * L.h * L.w;
-        cudaError_t e = launch_input_transform(xf, OpType::F16, g, r.in, x_end, V, nullptr, err, plain_stream);
+        e = launch_input_transform(xf, OpType::F16, g, r.in, x_end, V, nullptr, err, plain_stream);
         if (e == cudaSuccess) e = launch_gemm(gp, err, plain_stream);
         if (e == cudaSuccess) e = launch_output_transform(xf, mtype_for(r.m), g, Mw, r.out, nullptr, err, plain_stream);
+        return finish_plain(r, e);
+    }
+
+    // the event that marks a plain request's completion (e: status of its launches)
+    int finish_plain(Request& r, cudaError_t e) {
         cudaEvent_t ev = nullptr;
         if (e == cudaSuccess) {
             if (event_pool.empty()) {
@@ -537,11 +580,13 @@ int conv2d_server_add_layer(conv2d_server_t* server, unsigned c, unsigned k, uns
     const int cp = (c + 7) / 8 * 8, kp = (k + 7) / 8 * 8;
     const size_t b2 = static_cast<size_t>(16) * kp * cp * 2, b4 = static_cast<size_t>(36) * kp * cp * 2;
     void* blk = nullptr;
-    if (cudaMalloc(&blk, b2 + b4) != cudaSuccess) return set_last_error(CONV2D_ERR_NOMEM, "filter allocation failed");
+    if (cudaMalloc(&blk, b2 + b4 + direct_filter_bytes(k, c)) != cudaSuccess) return set_last_error(CONV2D_ERR_NOMEM, "filter allocation failed");
     sv->u_blocks.push_back(blk);
     L.U2 = blk;
     L.U4 = static_cast<char*>(blk) + b2;
-    if (launch_filter_transform(Xform::F2, OpType::F16, weight, L.U2, k, c, cp, nullptr) != cudaSuccess ||
+    L.U9 = static_cast<char*>(blk) + b2 + b4;
+    if (launch_direct_filter(weight, L.U9, k, c, nullptr) != cudaSuccess ||
+        launch_filter_transform(Xform::F2, OpType::F16, weight, L.U2, k, c, cp, nullptr) != cudaSuccess ||
         launch_filter_transform(Xform::F4, OpType::F16, weight, L.U4, k, c, cp, nullptr) != cudaSuccess ||
         cudaDeviceSynchronize() != cudaSuccess)
         return set_last_error(CONV2D_ERR_CUDA, "filter transform failed");
@@ -566,6 +611,7 @@ int conv2d_server_submit(conv2d_server_t* server, int layer, unsigned n, const v
     r.out = out;
     r.t_arrive = now_us();
     r.m = sv->choose_m(L);
+    r.direct = sv->choose_direct(L, n);
     const Geom g = make_geom(n, L.c, L.h, L.w, L.k, L.p, L.q, r.m);
     if (Server::ws_bytes_for(g) > sv->arena.capacity())
         return set_last_error(CONV2D_ERR_BUSY, "request workspace exceeds the server's HBM budget");
@@ -677,14 +723,22 @@ int conv2d_server_stats(conv2d_server_t* server, conv2d_server_stats_t* st) {
 // magic "WGCSRVL1", version, layer count; per layer its geometry, the byte
 // counts of its F(2x3) and F(4x3) filters and an FNV-1a checksum of both;
 // then the filters as they lie in device memory (U[E][Cp/8][Kp][8], fp16).
+// After them, in files that have it, magic "WGCSRVD1" and per layer the byte
+// count of its direct-kernel filter (0: none) and a checksum, then those
+// filters (U9[9][Cp/8][Kp][8]); layers of a file without it run F(2x3) or F(4x3).
 
 namespace {
 
 constexpr char kServerMagic[8] = {'W', 'G', 'C', 'S', 'R', 'V', 'L', '1'};
+constexpr char kDirectMagic[8] = {'W', 'G', 'C', 'S', 'R', 'V', 'D', '1'};
 
 struct LayerRecord {
     uint32_t c, k, h, w, p, q;
     uint64_t b2, b4, checksum;
+};
+
+struct DirectRecord {
+    uint64_t b9, checksum;
 };
 
 uint64_t fnv1a64(const unsigned char* p, size_t n, uint64_t h = 1469598103934665603ull) {
@@ -706,7 +760,8 @@ int conv2d_server_save_layers(conv2d_server_t* server, const char* path) {
         layers = sv->layers;
     }
     std::vector<LayerRecord> recs;
-    std::vector<std::vector<unsigned char>> data;
+    std::vector<std::vector<unsigned char>> data, data9;
+    std::vector<DirectRecord> recs9;
     for (const Layer& L : layers) {
         const uint64_t cp = (L.c + 7) / 8 * 8, kp = (L.k + 7) / 8 * 8;
         LayerRecord r{L.c, L.k, L.h, L.w, L.p, L.q, 16 * kp * cp * 2, 36 * kp * cp * 2, 0};
@@ -717,6 +772,13 @@ int conv2d_server_save_layers(conv2d_server_t* server, const char* path) {
         r.checksum = fnv1a64(buf.data(), buf.size());
         recs.push_back(r);
         data.push_back(std::move(buf));
+        DirectRecord r9{L.U9 ? static_cast<uint64_t>(direct_filter_bytes(L.k, L.c)) : 0, 0};
+        std::vector<unsigned char> buf9(r9.b9);
+        if (r9.b9 && cudaMemcpy(buf9.data(), L.U9, r9.b9, cudaMemcpyDeviceToHost) != cudaSuccess)
+            return set_last_error(CONV2D_ERR_CUDA, "copy of a resident filter failed");
+        r9.checksum = fnv1a64(buf9.data(), buf9.size());
+        recs9.push_back(r9);
+        data9.push_back(std::move(buf9));
     }
     FILE* f = std::fopen(path, "wb");
     if (!f) return set_last_error(CONV2D_ERR_INVALID, "cannot open the layer file for writing");
@@ -725,6 +787,9 @@ int conv2d_server_save_layers(conv2d_server_t* server, const char* path) {
               std::fwrite(&count, 4, 1, f) == 1 &&
               (recs.empty() || std::fwrite(recs.data(), sizeof(LayerRecord), recs.size(), f) == recs.size());
     for (const auto& d : data) ok = ok && std::fwrite(d.data(), 1, d.size(), f) == d.size();
+    ok = ok && std::fwrite(kDirectMagic, 8, 1, f) == 1 &&
+         (recs9.empty() || std::fwrite(recs9.data(), sizeof(DirectRecord), recs9.size(), f) == recs9.size());
+    for (const auto& d : data9) ok = ok && std::fwrite(d.data(), 1, d.size(), f) == d.size();
     if (std::fclose(f) != 0 || !ok) return set_last_error(CONV2D_ERR_INVALID, "layer file write failed");
     return CONV2D_OK;
 }
@@ -754,20 +819,39 @@ int conv2d_server_load_layers(conv2d_server_t* server, const char* path, int* fi
         ok = std::fread(buf.data(), 1, buf.size(), f) == buf.size() && fnv1a64(buf.data(), buf.size()) == r.checksum;
         data.push_back(std::move(buf));
     }
+    std::vector<DirectRecord> recs9(n, DirectRecord{0, 0});
+    std::vector<std::vector<unsigned char>> data9(n);
+    if (ok) {
+        const size_t got = std::fread(magic, 1, 8, f);
+        if (got != 0) {
+            ok = got == 8 && std::memcmp(magic, kDirectMagic, 8) == 0 &&
+                 (n == 0 || std::fread(recs9.data(), sizeof(DirectRecord), n, f) == n);
+            for (uint32_t i = 0; ok && i < n; ++i) {
+                ok = recs9[i].b9 == 0 || recs9[i].b9 == static_cast<uint64_t>(direct_filter_bytes(recs[i].k, recs[i].c));
+                if (!ok) break;
+                data9[i].resize(recs9[i].b9);
+                ok = std::fread(data9[i].data(), 1, data9[i].size(), f) == data9[i].size() &&
+                     fnv1a64(data9[i].data(), data9[i].size()) == recs9[i].checksum;
+            }
+        }
+    }
     std::fclose(f);
     if (!ok) return set_last_error(CONV2D_ERR_INVALID, "not a valid layer file (magic, version, sizes or checksum)");
     int first = -1;
     for (uint32_t i = 0; i < n; ++i) {
         const LayerRecord& r = recs[i];
         void* blk = nullptr;
-        if (cudaMalloc(&blk, r.b2 + r.b4) != cudaSuccess) return set_last_error(CONV2D_ERR_NOMEM, "filter allocation failed");
-        if (cudaMemcpy(blk, data[i].data(), r.b2 + r.b4, cudaMemcpyHostToDevice) != cudaSuccess) {
+        if (cudaMalloc(&blk, r.b2 + r.b4 + recs9[i].b9) != cudaSuccess) return set_last_error(CONV2D_ERR_NOMEM, "filter allocation failed");
+        if (cudaMemcpy(blk, data[i].data(), r.b2 + r.b4, cudaMemcpyHostToDevice) != cudaSuccess ||
+            (recs9[i].b9 && cudaMemcpy(static_cast<char*>(blk) + r.b2 + r.b4, data9[i].data(), recs9[i].b9,
+                                       cudaMemcpyHostToDevice) != cudaSuccess)) {
             cudaFree(blk);
             return set_last_error(CONV2D_ERR_CUDA, "copy of a resident filter failed");
         }
         Layer L{r.c, r.k, r.h, r.w, r.p, r.q};
         L.U2 = blk;
         L.U4 = static_cast<char*>(blk) + r.b2;
+        if (recs9[i].b9) L.U9 = static_cast<char*>(blk) + r.b2 + r.b4;
         std::lock_guard<std::mutex> lk(sv->mu);
         sv->u_blocks.push_back(blk);
         sv->layers.push_back(L);

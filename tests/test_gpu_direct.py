@@ -179,3 +179,41 @@ def test_one_queue_of_many_problems(wg, tmp_path, monkeypatch):
         for i, (_, _, y, want) in enumerate(keep):
             assert torch.equal(y.cpu(), want), i
     b.destroy()
+
+
+def test_served_layers_of_an_older_file(wg, tmp_path):
+    """A layer file without the direct kernel's filters (they follow the
+    others) still loads, and its layers run the Winograd transform; a file cut
+    inside them is refused."""
+    c, k, h = 64, 96, 14
+    g = torch.Generator().manual_seed(8)
+    wt = (torch.randn((k, c, 3, 3), generator=g) / 24).half().cuda()
+    x = (torch.rand((3, c, h, h), generator=g) * 2 - 1).half().cuda()
+
+    def run(server, layer):
+        y = torch.zeros((3, k, h, h), dtype=torch.float16, device="cuda")
+        torch.cuda.synchronize()
+        server.submit(layer, 3, x.data_ptr(), y.data_ptr())
+        server.wait_all()
+        return y.cpu()
+
+    a = wg.Server(hbm_budget_bytes=1 << 28)
+    a.add_layer(c, k, h, h, wt.data_ptr())
+    path = tmp_path / "layers"
+    a.save_layers(str(path))
+    ya = run(a, 0)
+    f2 = wg.Server(hbm_budget_bytes=1 << 28, algo=wg.ALGO_2X3)
+    f2.add_layer(c, k, h, h, wt.data_ptr())
+    y2 = run(f2, 0)
+    raw = path.read_bytes()
+    cut = raw.rindex(b"WGCSRVD1")
+    older, broken = tmp_path / "older", tmp_path / "broken"
+    older.write_bytes(raw[:cut])
+    broken.write_bytes(raw[:-2])
+    b = wg.Server(hbm_budget_bytes=1 << 28)
+    assert torch.equal(run(b, b.load_layers(str(path))[0]), ya)
+    assert torch.equal(run(b, b.load_layers(str(older))[0]), y2)
+    with pytest.raises(wg.Conv2dError):
+        b.load_layers(str(broken))
+    for server in (a, f2, b):
+        server.destroy()
