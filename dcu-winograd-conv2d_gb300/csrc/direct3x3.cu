@@ -245,8 +245,9 @@ struct Producer {
             pairs = d.pairs;
             plane = static_cast<uint32_t>(d.h * d.w);
             xi = static_cast<const uint16_t*>(d.x) + static_cast<long long>(n0) * channels * plane;
-            blocks = NHWC ? (win + 255) / 256 : pairs ? (win / 2 + kGroupThreads) / kGroupThreads
-                                                     : (win + kGroupThreads - 1) / kGroupThreads;
+            // blocks that reach into the window, for this warp's part of them
+            blocks = NHWC ? (win + 255) / 256
+                          : max(((pairs ? win / 2 + 1 : win) - (gt & ~31) + kGroupThreads - 1) / kGroupThreads, 1);
             pads = 0;
             decode(d);
         }
@@ -287,24 +288,21 @@ struct Producer {
             }
             s.p = p;
             if (o < 0) s.flags |= 16u;
-            // a warp whose lanes all lie past the window reads one value over and over
-            const bool live = __any_sync(0xffffffffu, p < win);
             // padding reads the image's first pixel (cleared or not stored later)
             const uint16_t* src = xi + max(o, 0) + static_cast<unsigned long long>(c * kChunkC) * plane;
-            const uint32_t st = live ? plane : 0u;
             if (left >= kChunkC) {
                 if (pairs) {
 #pragma unroll
-                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg32(src + static_cast<unsigned long long>(j) * st);
+                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg32(src + static_cast<unsigned long long>(j) * plane);
                 } else {
 #pragma unroll
-                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg16(src + static_cast<unsigned long long>(j) * st);
+                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg16(src + static_cast<unsigned long long>(j) * plane);
                 }
             } else {
                 // the last chunk of a C that is not a multiple of 16
 #pragma unroll
                 for (int j = 0; j < kChunkC; ++j) {
-                    const uint16_t* q = src + static_cast<unsigned long long>(min(j, left - 1)) * st;
+                    const uint16_t* q = src + static_cast<unsigned long long>(min(j, left - 1)) * plane;
                     const uint32_t v = pairs ? ldg32(q) : ldg16(q);
                     s.r[j] = j < left ? v : 0u;
                 }
@@ -611,20 +609,19 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
                             }
                         } else {
                             // a warp's 32 positions of one channel are (nearly) contiguous
-                            uint16_t* q = o;
+                            const uint32_t op = static_cast<uint32_t>(oplane);
                             if (k0 + 16 <= K) {
 #pragma unroll
                                 for (int j = 0; j < 16; j += 2) {
                                     const uint32_t v = pack2<BF16>(r[j], r[j + 1]);
-                                    q[0] = static_cast<uint16_t>(v);
-                                    q[oplane] = static_cast<uint16_t>(v >> 16);
-                                    q += 2 * static_cast<long long>(oplane);
+                                    o[static_cast<unsigned long long>(j) * op] = static_cast<uint16_t>(v);
+                                    o[static_cast<unsigned long long>(j + 1) * op] = static_cast<uint16_t>(v >> 16);
                                 }
                             } else {
 #pragma unroll
                                 for (int j = 0; j < 16; ++j) {
-                                    if (k0 + j < K) *q = static_cast<uint16_t>(pack2<BF16>(r[j], 0u));
-                                    q += oplane;
+                                    if (k0 + j < K)
+                                        o[static_cast<unsigned long long>(j) * op] = static_cast<uint16_t>(pack2<BF16>(r[j], 0u));
                                 }
                             }
                         }
