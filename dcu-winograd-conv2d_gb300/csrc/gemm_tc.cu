@@ -311,64 +311,72 @@ __device__ __forceinline__ void gemm_body(const GemmDesc* __restrict__ descs, in
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            int stage = 0;
-            uint32_t phase = 0;
-            int acc = 0;
-            uint32_t acc_phase = 0;
-            int pi = 0;
-            int bkey = -1;
-            uint32_t bphase = 0;
-            for (long long t = t_lo; t < t_hi; t += t_step) {
-                const Item it = locate_item<RESB>(descs, ndesc, t, pi);
-                const int k_blocks = descs[pi].k_blocks;
-                if (!mbar_wait(&tempty[acc], acc_phase ^ 1u, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
-                if constexpr (RESB) {
-                    const int key = it.e * descs[0].n_blocks + it.nb;
-                    if (key != bkey) {
-                        if (!mbar_wait(bfull, bphase, abort_flag, err, ERR_SITE_FULL)) break;
-                        bphase ^= 1u;
-                        bkey = key;
-                    }
+        // The whole warp walks the loop with warp-uniform control flow and
+        // values and one elected lane issues: the descriptors then stay in
+        // uniform registers, where an MMA takes its operands from (issued from
+        // a one-lane loop every MMA first moved them there)
+        int stage = 0;
+        uint32_t phase = 0;
+        int acc = 0;
+        uint32_t acc_phase = 0;
+        int pi = 0;
+        int bkey = -1;
+        uint32_t bphase = 0;
+        const bool elected = elect_one();
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t ad0 = make_smem_desc(smem_u32(sA), kBM * 16, 128, Swz::None);
+        const uint64_t bd0 = make_smem_desc(smem_u32(sB), BN * 16, 128, Swz::None);
+        for (long long t = t_lo; t < t_hi; t += t_step) {
+            const Item it = locate_item<RESB>(descs, ndesc, t, pi);
+            const int k_blocks = descs[pi].k_blocks;
+            if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1u, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+            if constexpr (RESB) {
+                const int key = it.e * descs[0].n_blocks + it.nb;
+                if (key != bkey) {
+                    if (!mbar_wait_warp(bfull, bphase, abort_flag, err, ERR_SITE_FULL)) break;
+                    bphase ^= 1u;
+                    bkey = key;
+                }
+            }
+            tc_fence_after();
+            const uint32_t d_tmem = tmem_u + static_cast<uint32_t>(acc * BN);
+            bool ok = true;
+            for (int kb = 0; kb < k_blocks; ++kb) {
+                if (!mbar_wait_warp(&full[stage], phase, abort_flag, err, ERR_SITE_FULL)) {
+                    ok = false;
+                    break;
                 }
                 tc_fence_after();
-                const uint32_t d_tmem = tmem_base + static_cast<uint32_t>(acc * BN);
-                bool ok = true;
-                for (int kb = 0; kb < k_blocks; ++kb) {
-                    if (!mbar_wait(&full[stage], phase, abort_flag, err, ERR_SITE_FULL)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_base = smem_u32(sA + stage * kTileABytes);
-                    const uint32_t b_base = smem_u32(sB + (RESB ? kb : stage) * Cfg::kTileB);
+                const uint64_t ad = ad0 + static_cast<uint32_t>(stage * (kTileABytes / 16));
+                const uint64_t bd = bd0 + static_cast<uint32_t>((RESB ? kb : stage) * (Cfg::kTileB / 16));
+                if (elected) {
                     // K = 16 per MMA = 2 granules: core matrices at +0 and +LBO
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k) {
-                        const uint64_t ad = make_smem_desc(a_base + k * (2 * kBM * 16), kBM * 16, 128, Swz::None);
-                        const uint64_t bd = make_smem_desc(b_base + k * (2 * BN * 16), BN * 16, 128, Swz::None);
-                        tc_mma_f16(d_tmem, ad, bd, kIdesc, (kb | k) != 0 ? 1u : 0u);
-                    }
+                    for (int k = 0; k < kBK / 16; ++k)
+                        tc_mma_f16(d_tmem, ad + static_cast<uint32_t>(k * 2 * kBM), bd + static_cast<uint32_t>(k * 2 * BN),
+                                   kIdesc, (kb | k) != 0 ? 1u : 0u);
                     tc_commit(&empty[stage]);
-                    if (++stage == S) {
-                        stage = 0;
-                        phase ^= 1u;
-                    }
                 }
-                if (!ok) break;
-                tc_commit(&tfull[acc]);
-                if constexpr (RESB) {
-                    // the next item reads another U block: free this one when
-                    // the MMAs issued so far are done
-                    if (t + 1 < t_hi) {
-                        const Item nx = locate_resb(descs[0], t + 1);
-                        if (nx.e * descs[0].n_blocks + nx.nb != bkey) tc_commit(bempty);
-                    }
+                __syncwarp();
+                if (++stage == S) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
-                if (++acc == 2) {
-                    acc = 0;
-                    acc_phase ^= 1u;
+            }
+            if (!ok) break;
+            if (elected) tc_commit(&tfull[acc]);
+            if constexpr (RESB) {
+                // the next item reads another U block: free this one when
+                // the MMAs issued so far are done
+                if (t + 1 < t_hi) {
+                    const Item nx = locate_resb(descs[0], t + 1);
+                    if (nx.e * descs[0].n_blocks + nx.nb != bkey && elected) tc_commit(bempty);
                 }
+            }
+            __syncwarp();
+            if (++acc == 2) {
+                acc = 0;
+                acc_phase ^= 1u;
             }
         }
     } else if (warp - 2 < 4 * kEpiHalves) {
