@@ -45,13 +45,14 @@ struct Batch {
     };
     struct GemmGroup {
         int bn;
+        int shape;   // gemm_shape
         MType mt;
         OpType op;
         Xform xf;
         const GemmDesc* descs;
         int n;
         long long tiles;
-        int grid;
+        int num_sms;
     };
     struct OutGroup {
         Xform xf;
@@ -121,7 +122,7 @@ struct Batch {
                 return e;
         for (const GemmGroup& g : gemm_groups)
             if (g.xf == xf && (bn == 0 || g.bn == bn) &&
-                (e = launch_gemm_grouped(g.descs, g.n, g.tiles, g.op, g.mt, g.bn, g.grid, err, s)) != cudaSuccess)
+                (e = launch_gemm_grouped(g.descs, g.n, g.tiles, g.op, g.mt, g.shape, g.num_sms, err, s)) != cudaSuccess)
                 return e;
         for (const OutGroup& g : out_groups)
             if (g.xf == xf && g.bn == bn &&
@@ -196,7 +197,7 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     std::map<std::tuple<int, int, int>, std::vector<int>> in_keys, out_keys;  // (xform, op | M type, bn) -> problems
     const char* sb = std::getenv("WG_CONV2D_BATCH_SPLIT_BN");
     const bool split_bn = sb && sb[0] == '1';
-    std::map<std::tuple<int, int, int, int>, std::vector<int>> gemm_keys;     // (bn, M type, op, xform) -> problems
+    std::map<std::tuple<int, int, int, int>, std::vector<int>> gemm_keys;     // (shape, M type, op, xform) -> problems
     std::vector<DirectProblem> direct_probs;
     double direct_flops = 0;
     for (int i = 0; i < count; ++i) {
@@ -216,7 +217,7 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
         const int cbn = split_bn ? p.gemm_full.bn : 0;
         in_keys[{static_cast<int>(p.xf), static_cast<int>(p.op), cbn}].push_back(i);
         out_keys[{static_cast<int>(p.xf), static_cast<int>(p.mt), cbn}].push_back(i);
-        gemm_keys[{p.gemm_full.bn, static_cast<int>(p.mt), static_cast<int>(p.op), static_cast<int>(p.xf)}].push_back(i);
+        gemm_keys[{gemm_shape(p.g.P, p.gemm_full.bn, false), static_cast<int>(p.mt), static_cast<int>(p.op), static_cast<int>(p.xf)}].push_back(i);
     }
     std::vector<InDesc> in_descs;
     std::vector<OutDesc> out_descs;
@@ -259,7 +260,13 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     for (auto& kv : gemm_keys) {
         Range r{gemm_descs.size(), kv.second.size(), 0, 0, false};
         for (int i : kv.second) {
-            GemmDesc d = b->plans[i]->gemm_full.desc;
+            const Plan& p = *b->plans[i];
+            GemmDesc d;
+            if (make_gemm_desc(d, p.op, p.g.alpha * p.g.alpha, p.g.P, p.g.k, p.g.kp, p.g.cp, p.V, p.U, p.Mw, p.mt,
+                               std::get<0>(kv.first)) != cudaSuccess)
+                return batch_fail(CONV2D_ERR_CUDA, "GEMM descriptors (tensor maps)");
+            d.keep_m = p.gemm_full.desc.keep_m;
+            d.discard_v = p.gemm_full.desc.discard_v;
             d.tile_begin = r.total;
             r.total += d.tiles;
             gemm_descs.push_back(d);
@@ -299,11 +306,10 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
                                 std::get<2>(kr.first), reinterpret_cast<const InDesc*>(base + oI) + kr.second.first,
                                 static_cast<int>(kr.second.n), kr.second.total, kr.second.extra, kr.second.scaled});
     for (auto& kr : gemm_r)
-        b->gemm_groups.push_back({std::get<0>(kr.first), static_cast<MType>(std::get<1>(kr.first)),
+        b->gemm_groups.push_back({std::get<0>(kr.first) & ~kGemmPairs, std::get<0>(kr.first), static_cast<MType>(std::get<1>(kr.first)),
                                   static_cast<OpType>(std::get<2>(kr.first)), static_cast<Xform>(std::get<3>(kr.first)),
                                   reinterpret_cast<const GemmDesc*>(base + oG) + kr.second.first,
-                                  static_cast<int>(kr.second.n), kr.second.total,
-                                  static_cast<int>(std::min<long long>(kr.second.total, sms))});
+                                  static_cast<int>(kr.second.n), kr.second.total, sms});
     for (auto& kr : out_r)
         b->out_groups.push_back({static_cast<Xform>(std::get<0>(kr.first)), static_cast<MType>(std::get<1>(kr.first)),
                                  std::get<2>(kr.first), reinterpret_cast<const OutDesc*>(base + oO) + kr.second.first,

@@ -738,22 +738,7 @@ double item_cycles(int bn, int mb, int pw, int chunks) {
 template <class F, class... Args>
 cudaError_t launch_cluster(F kern, int pairs, int smem, cudaStream_t s, const Args&... args) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(kDirectThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
+    return e == cudaSuccess ? launch_pairs(kern, pairs, kDirectThreads, smem, s, args...) : e;
 }
 
 // CTA pairs that run at once (one CTA per SM; a cluster stays within a GPC)

@@ -479,6 +479,259 @@ __device__ __forceinline__ void gemm_body(const GemmDesc* __restrict__ descs, in
     }
 }
 
+// ---- CTA pairs -------------------------------------------------------------------
+// The same GEMM by pairs of CTAs (cta_group::2, M = 256): each CTA loads its
+// own 128 tiles of V and half of the BN output channels of U, so a 64-channel
+// k-block moves 16 KB + BN * 64 bytes into each SM instead of 16 KB + BN * 128.
+// What the SMs take in from L2 beside the M stores bounds this GEMM where U is
+// not resident, not its MMAs.  Stages, TMEM double buffering and the epilogue
+// are those of the single-CTA kernel.  GEMM time, single CTAs -> pairs, F(4x3):
+// 32x512x28^2 -> 512 38.5 -> 34.4 us (262 instead of 393 KB per item of 128
+// tiles and CTA), 16x512x56^2 -> 512 63.1 -> 59.0, 2x640x64^2 -> 640 24.1 (BN
+// 128) -> 22.1 (BN 256); F(2x3) 2x1280x16^2 -> 1280 17.0 -> 16.0.
+template <int BN>
+struct PairCfg {
+    static constexpr int kTileB = BN / 2 * kBK * 2;
+    static constexpr int kStageBytes = kTileABytes + kTileB;
+    static constexpr int kStages = std::min(8, 200 * 1024 / kStageBytes);
+    static constexpr int kSmem = kStages * kStageBytes + 1024 + 256;
+};
+
+template <int BN, bool BF16, class MT>
+__device__ __forceinline__ void gemm_pair_body(const GemmDesc* __restrict__ descs, int ndesc, long long total_tiles,
+                                               DevErr* err) {
+    using Cfg = PairCfg<BN>;
+    constexpr int S = Cfg::kStages;
+    constexpr uint32_t kIdesc = make_idesc_f16(2 * kBM, BN, BF16);
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    unsigned char* sA = smem;
+    unsigned char* sB = smem + S * kTileABytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * Cfg::kStageBytes);   // even CTA: both CTAs' tiles landed
+    uint64_t* empty = full + S;                                                  // MMAs done with the stage
+    uint64_t* tfull = empty + S;                                                 // accumulators ready
+    uint64_t* tempty = tfull + 2;                                                // even CTA: drained in both CTAs
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
+    const long long first = blockIdx.x >> 1, step = gridDim.x >> 1;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < S; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&tfull[i], 1);
+            mbar_init(&tempty[i], 2 * 8);
+        }
+        *abort_flag = 0;
+        fence_barrier_init();
+    }
+    pdl_wait();     // V written, earlier readers of M done
+    pdl_trigger();
+    if (warp == 1) tmem_alloc_pair(tmem_slot, 512);
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            const uint64_t drop = l2_evict_first(), keep_as_is = l2_evict_unchanged();
+            int stage = 0, pi = 0, prefetched = -1;
+            uint32_t phase = 0;
+            bool ok = true;
+            long long used = 0;
+            for (long long t = first; t < total_tiles && ok; t += step) {
+                const Item it = locate(descs, ndesc, t, pi);
+                const GemmDesc& d = descs[pi];
+                if (prefetched != pi) {
+                    tma_prefetch_desc(&d.tmA);
+                    tma_prefetch_desc(&d.tmB);
+                    prefetched = pi;
+                }
+                const int k_blocks = d.k_blocks;
+                const int row_a = (it.mb * 2 + static_cast<int>(rank)) * (kBM / 8);
+                const int row_b = it.nb * (BN / 8) + static_cast<int>(rank) * (BN / 16);
+                const uint64_t pol = it.nb == d.n_blocks - 1 ? drop : keep_as_is;   // V: dropped by its last reader
+                for (int kb = 0; kb < k_blocks; ++kb, ++used) {
+                    if (!mbar_wait(&empty[stage], phase ^ 1u, abort_flag, err, ERR_SITE_EMPTY)) {
+                        ok = false;
+                        break;
+                    }
+                    if (rank == 0) mbar_arrive_expect_tx(&full[stage], 2 * Cfg::kStageBytes);
+                    const uint32_t bar = map_to_rank(&full[stage], 0);
+                    tma_load_4d_pair_hint(sA + stage * kTileABytes, &d.tmA, bar, 0, row_a, kb * 8, it.e, pol);
+                    tma_load_4d_pair(sB + stage * Cfg::kTileB, &d.tmB, bar, 0, row_b, kb * 8, it.e);
+                    if (++stage == S) {
+                        stage = 0;
+                        phase ^= 1u;
+                    }
+                }
+            }
+            // the last commits on this CTA's barriers must land before it exits
+            for (long long u = used > S ? used - S : 0; ok && u < used; ++u)
+                ok = mbar_wait(&empty[u % S], static_cast<uint32_t>(u / S) & 1u, abort_flag, err, ERR_SITE_DRAIN);
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {   // one elected lane of a warp-uniform loop (see gemm_body)
+            int stage = 0, acc = 0, pi = 0;
+            uint32_t phase = 0, acc_phase = 0;
+            const bool elected = elect_one();
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint64_t ad0 = make_smem_desc(smem_u32(sA), kBM * 16, 128, Swz::None);
+            const uint64_t bd0 = make_smem_desc(smem_u32(sB), BN / 2 * 16, 128, Swz::None);
+            bool ok = true;
+            for (long long t = first; t < total_tiles && ok; t += step) {
+                locate(descs, ndesc, t, pi);
+                const int k_blocks = descs[pi].k_blocks;
+                if (!mbar_wait_warp(&tempty[acc], acc_phase ^ 1u, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+                tc_fence_after();
+                const uint32_t d_tmem = tmem_u + static_cast<uint32_t>(acc * 256);
+                for (int kb = 0; kb < k_blocks; ++kb) {
+                    if (!mbar_wait_warp(&full[stage], phase, abort_flag, err, ERR_SITE_FULL)) {
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint64_t ad = ad0 + static_cast<uint32_t>(stage * (kTileABytes / 16));
+                    const uint64_t bd = bd0 + static_cast<uint32_t>(stage * (Cfg::kTileB / 16));
+                    if (elected) {
+#pragma unroll
+                        for (int k = 0; k < kBK / 16; ++k)
+                            tc_mma_f16_pair(d_tmem, ad + static_cast<uint32_t>(k * 2 * kBM), bd + static_cast<uint32_t>(k * BN),
+                                            kIdesc, (kb | k) != 0 ? 1u : 0u);
+                        tc_commit_pair(&empty[stage]);
+                    }
+                    __syncwarp();
+                    if (++stage == S) {
+                        stage = 0;
+                        phase ^= 1u;
+                    }
+                }
+                if (ok && elected) tc_commit_pair(&tfull[acc]);
+                __syncwarp();
+                if (++acc == 2) {
+                    acc = 0;
+                    acc_phase ^= 1u;
+                }
+            }
+        }
+    } else {
+        const int quarter = warp & 3, half = (warp - 2) >> 2;
+        const int row = quarter * 32 + lane;
+        const uint64_t m_pol = descs[0].keep_m ? l2_evict_last() : l2_evict_first();
+        int acc = 0, pi = 0;
+        uint32_t acc_phase = 0;
+        for (long long t = first; t < total_tiles; t += step) {
+            const Item it = locate(descs, ndesc, t, pi);
+            const GemmDesc& d = descs[pi];
+            MT* Mw = static_cast<MT*>(d.Mw);
+            const long long P = d.P, m_lo = d.m_lo;
+            const int kg_count = d.kg_count, E = d.E;
+            if (!mbar_wait(&tfull[acc], acc_phase, abort_flag, err, ERR_SITE_TMEM_FULL)) break;
+            __syncwarp();
+            tc_fence_after();
+            const int tile0 = (it.mb * 2 + static_cast<int>(rank)) * kBM;
+            const long long p = static_cast<long long>(tile0) + row;
+            const int col0 = half * (BN / 2);
+            const uint32_t taddr =
+                tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(acc * 256 + col0);
+            constexpr int kChunks = BN / 64;
+            uint32_t r[2][32];
+            tmem_ld_x32(taddr, r[0]);
+            tc_wait_ld(r[0]);
+#pragma unroll
+            for (int ch = 0; ch < kChunks; ++ch) {
+                if (ch + 1 < kChunks) tmem_ld_x32(taddr + (ch + 1) * 32, r[(ch + 1) & 1]);
+                if (p < P) {
+                    const int k0 = it.nb * BN + col0 + ch * 32;
+                    if constexpr (std::is_same<MT, M24>::value)
+                        store32_m24(reinterpret_cast<unsigned char*>(Mw), r[ch & 1], p, k0, kg_count, it.e, E, m_lo, m_pol);
+                    else
+                        store32<MT>(Mw, r[ch & 1], P, p, k0, kg_count, it.e, m_pol);
+                }
+                __syncwarp();
+                if (ch + 1 < kChunks) tc_wait_ld(r[(ch + 1) & 1]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_rank(&tempty[acc], 0));
+            if (d.discard_v && tile0 < d.v_pp) {
+                // as in gemm_body: this CTA's rows of V have no other reader
+                const int et = (warp - 2) * 32 + lane;
+                const int lpg = min(kBM, d.v_pp - tile0) / 8;
+                const unsigned char* vb = static_cast<const unsigned char*>(d.V) +
+                                          ((static_cast<long long>(it.e) * d.v_cg) * d.v_pp + tile0) * 16;
+                for (int i = et; i < d.v_cg * lpg; i += 256) {
+                    const int g = i / lpg, l = i - g * lpg;
+                    discard_l2_line(vb + static_cast<long long>(g) * d.v_pp * 16 + l * 128);
+                }
+            }
+            if (++acc == 2) {
+                acc = 0;
+                acc_phase ^= 1u;
+            }
+        }
+    }
+
+    __syncthreads();
+    if (*abort_flag) {
+        const unsigned long long t0 = globaltimer_ns();
+        while (globaltimer_ns() - t0 < 2000000ull) {
+        }
+    }
+    tc_fence_before();
+    cluster_sync();   // the peer's MMAs, copies and arrivals on this CTA are done
+    tc_fence_after();
+    if (warp == 1) tmem_dealloc_pair(tmem_base, 512);
+}
+
+template <int BN, bool BF16, class MT>
+__global__ void __launch_bounds__(kGemmThreads, 1) wino_gemm_pair_kernel(const __grid_constant__ GemmDesc d, DevErr* err) {
+    gemm_pair_body<BN, BF16, MT>(&d, 1, d.tiles, err);
+}
+
+template <int BN, bool BF16, class MT>
+__global__ void __launch_bounds__(kGemmThreads, 1)
+    wino_gemm_pair_grouped(const GemmDesc* __restrict__ descs, int ndesc, long long total_tiles, DevErr* err) {
+    gemm_pair_body<BN, BF16, MT>(descs, ndesc, total_tiles, err);
+}
+
+template <int BN, bool BF16, class MT>
+cudaError_t gemm_pair_launch(bool single, const GemmDesc* d, int ndesc, long long total, int pairs, DevErr* err,
+                             cudaStream_t s) {
+    constexpr int smem = PairCfg<BN>::kSmem;
+    static_assert(smem > 116 * 1024, "one CTA per SM: each takes all of TMEM");
+    if (single) {
+        auto kern = wino_gemm_pair_kernel<BN, BF16, MT>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        return e == cudaSuccess ? launch_pairs(kern, pairs, kGemmThreads, smem, s, *d, err) : e;
+    }
+    auto kern = wino_gemm_pair_grouped<BN, BF16, MT>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return e == cudaSuccess ? launch_pairs(kern, pairs, kGemmThreads, smem, s, d, ndesc, total, err) : e;
+}
+
+template <int BN>
+cudaError_t dispatch_pair(bool bf, MType mt, bool single, const GemmDesc* d, int ndesc, long long total, int pairs,
+                          DevErr* err, cudaStream_t s) {
+    switch (mt) {
+        case MType::F32:
+            return bf ? gemm_pair_launch<BN, true, float>(single, d, ndesc, total, pairs, err, s)
+                      : gemm_pair_launch<BN, false, float>(single, d, ndesc, total, pairs, err, s);
+        case MType::F16:
+            return bf ? gemm_pair_launch<BN, true, __half>(single, d, ndesc, total, pairs, err, s)
+                      : gemm_pair_launch<BN, false, __half>(single, d, ndesc, total, pairs, err, s);
+        case MType::F24:
+            return bf ? cudaErrorNotSupported : gemm_pair_launch<BN, false, M24>(single, d, ndesc, total, pairs, err, s);
+    }
+    return cudaErrorInvalidValue;
+}
+
 template <int BN, bool BF16, class MT, bool RESB>
 __global__ void __launch_bounds__(kGemmThreads, 1) wino_gemm_kernel(const __grid_constant__ GemmDesc d, DevErr* err) {
     gemm_body<BN, BF16, MT, RESB>(&d, 1, d.tiles, err);
@@ -539,9 +792,15 @@ cudaError_t dispatch_types(bool bf, MType mt, bool single, const GemmDesc* d, in
     return cudaErrorInvalidValue;
 }
 
-cudaError_t dispatch(int bn, bool bf, MType mt, bool single, const GemmDesc* d, int ndesc, long long total, int grid,
+cudaError_t dispatch(int shape, bool bf, MType mt, bool single, const GemmDesc* d, int ndesc, long long total, int grid,
                      DevErr* err, cudaStream_t s) {
-    switch (bn) {
+    if (shape & kGemmPairs) {
+        const int pairs = static_cast<int>(std::min<long long>(total, direct_max_pairs(grid)));
+        return (shape & ~kGemmPairs) == 128 ? dispatch_pair<128>(bf, mt, single, d, ndesc, total, pairs, err, s)
+                                            : dispatch_pair<256>(bf, mt, single, d, ndesc, total, pairs, err, s);
+    }
+    grid = static_cast<int>(std::min<long long>(total, grid));
+    switch (shape) {
         case 32: return dispatch_types<32>(bf, mt, single, d, ndesc, total, grid, err, s);
         case 64: return dispatch_types<64>(bf, mt, single, d, ndesc, total, grid, err, s);
         case 128: return dispatch_types<128>(bf, mt, single, d, ndesc, total, grid, err, s);
@@ -579,7 +838,10 @@ int gemm_smem_bytes(int bn) {
 }
 
 cudaError_t make_gemm_desc(GemmDesc& d, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
-                           const void* U, void* Mw, MType mt, int bn, bool m_row) {
+                           const void* U, void* Mw, MType mt, int shape, bool m_row) {
+    const int bn = shape & ~kGemmPairs;
+    const bool pair = (shape & kGemmPairs) != 0;
+    if (pair && (bn < 128 || m_row)) return cudaErrorInvalidValue;
     if (bn != 32 && bn != 64 && bn != 128 && bn != 256) return cudaErrorInvalidValue;
     if (P <= 0 || P > 0x7fffffffLL || Cp % 8 != 0 || Kp % 8 != 0) return cudaErrorInvalidValue;
     if (mt == MType::F24 && (m_row || op != OpType::F16)) return cudaErrorNotSupported;
@@ -595,7 +857,10 @@ cudaError_t make_gemm_desc(GemmDesc& d, OpType op, int E, long long P, int K, in
     d.v_pp = static_cast<int>(round_rows(P));
     d.discard_v = 0;
     d.resb = 0;      // plan_gemm decides for single launches; grouped ones hand out items round robin
-    d.m_blocks = static_cast<int>((P + kBM - 1) / kBM);
+    d.pair = pair ? 1 : 0;
+    d.bn = bn;
+    const int bm = pair ? 2 * kBM : kBM;
+    d.m_blocks = static_cast<int>((P + bm - 1) / bm);
     d.n_blocks = (K + bn - 1) / bn;
     d.k_blocks = (Cp + kBK - 1) / kBK;
     d.E = E;
@@ -623,7 +888,7 @@ cudaError_t make_gemm_desc(GemmDesc& d, OpType op, int E, long long P, int K, in
     {
         cuuint64_t dims[4] = {64, Kr, CG, static_cast<cuuint64_t>(E)};
         cuuint64_t strides[3] = {128, Kr * 128, CG * Kr * 128};
-        cuuint32_t box[4] = {64, static_cast<cuuint32_t>(bn / 8), 8, 1};
+        cuuint32_t box[4] = {64, static_cast<cuuint32_t>(pair ? bn / 16 : bn / 8), 8, 1};
         if (encode_tiled(&d.tmB, dt, 4, const_cast<void*>(U), dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE) !=
             CUDA_SUCCESS)
             return cudaErrorInvalidValue;
@@ -631,10 +896,24 @@ cudaError_t make_gemm_desc(GemmDesc& d, OpType op, int E, long long P, int K, in
     return cudaSuccess;
 }
 
+// Pairs where a tile has channels for two (from 128 on) and there are tiles
+// for both CTAs; the row-major M of the channels-last path stays with the
+// single-CTA kernel.
+int gemm_shape(long long P, int bn, bool m_row) { return bn >= 128 && !m_row && P > kBM ? bn | kGemmPairs : bn; }
+
 cudaError_t plan_gemm(GemmPlan& gp, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
                       const void* U, void* Mw, MType mt, int bn, int num_sms, bool m_row) {
-    cudaError_t e = make_gemm_desc(gp.desc, op, E, P, K, Kp, Cp, V, U, Mw, mt, bn, m_row);
+    // U block of one (element, channel block) within the resident budget: it
+    // stays in shared memory over consecutive tile blocks instead of being
+    // reloaded from L2 for every work item (32 x 256 x 56^2 -> 256: 226 of
+    // the 339 MB of operand loads); WG_CONV2D_GEMM_RESIDENT_U=0 turns it off
+    const char* res = std::getenv("WG_CONV2D_GEMM_RESIDENT_U");
+    const long long m_blocks = (P + kBM - 1) / kBM, n_blocks = (K + bn - 1) / bn, k_blocks = (Cp + kBK - 1) / kBK;
+    const bool resb = !(res && res[0] == '0') && k_blocks * bn * kBK * 2 <= kResBBytes && E * m_blocks * n_blocks >= num_sms;
+    gp.shape = resb ? bn : gemm_shape(P, bn, m_row);
+    cudaError_t e = make_gemm_desc(gp.desc, op, E, P, K, Kp, Cp, V, U, Mw, mt, gp.shape, m_row);
     if (e != cudaSuccess) return e;
+    gp.desc.resb = resb ? 1 : 0;
     // M of this launch within the L2 size: kept there for the output transform
     // that reads it next (32 x 512 x 28^2 -> 512 F(4x3): 87 MB in 24 bits); larger M is streamed out
     gp.desc.keep_m = m_bytes(mt, E, P, Kp) <= l2_cache_bytes();
@@ -642,29 +921,27 @@ cudaError_t plan_gemm(GemmPlan& gp, OpType op, int E, long long P, int K, int Kp
     // WG_CONV2D_KEEP_WORKSPACE=1 keeps it (to read the workspace back)
     const char* keep_ws = std::getenv("WG_CONV2D_KEEP_WORKSPACE");
     gp.desc.discard_v = gp.desc.n_blocks == 1 && !(keep_ws && std::atoi(keep_ws) != 0);
-    // U block of one (element, channel block) within the resident budget: it
-    // stays in shared memory over consecutive tile blocks instead of being
-    // reloaded from L2 for every work item (32 x 256 x 56^2 -> 256: 226 of
-    // the 339 MB of operand loads); WG_CONV2D_GEMM_RESIDENT_U=0 turns it off
-    const char* res = std::getenv("WG_CONV2D_GEMM_RESIDENT_U");
-    gp.desc.resb = !(res && res[0] == '0') &&
-                   static_cast<long long>(gp.desc.k_blocks) * bn * kBK * 2 <= kResBBytes &&
-                   gp.desc.tiles >= num_sms;
     gp.op = op;
     gp.bn = bn;
     gp.mt = mt;
-    gp.grid = static_cast<int>(std::min<long long>(gp.desc.tiles, num_sms));
-    gp.smem_bytes = gemm_smem_bytes(bn);
+    gp.num_sms = num_sms;
+    if (gp.desc.pair) {
+        gp.grid = 2 * static_cast<int>(std::min<long long>(gp.desc.tiles, direct_max_pairs(num_sms)));
+        gp.smem_bytes = bn == 128 ? PairCfg<128>::kSmem : PairCfg<256>::kSmem;
+    } else {
+        gp.grid = static_cast<int>(std::min<long long>(gp.desc.tiles, num_sms));
+        gp.smem_bytes = gemm_smem_bytes(bn);
+    }
     return cudaSuccess;
 }
 
 cudaError_t launch_gemm(const GemmPlan& gp, DevErr* err, cudaStream_t stream) {
-    return dispatch(gp.bn, gp.op == OpType::BF16, gp.mt, true, &gp.desc, 1, gp.desc.tiles, gp.grid, err, stream);
+    return dispatch(gp.shape, gp.op == OpType::BF16, gp.mt, true, &gp.desc, 1, gp.desc.tiles, gp.num_sms, err, stream);
 }
 
-cudaError_t launch_gemm_grouped(const GemmDesc* descs, int ndesc, long long total_tiles, OpType op, MType mt, int bn,
-                                int grid, DevErr* err, cudaStream_t stream) {
-    return dispatch(bn, op == OpType::BF16, mt, false, descs, ndesc, total_tiles, grid, err, stream);
+cudaError_t launch_gemm_grouped(const GemmDesc* descs, int ndesc, long long total_tiles, OpType op, MType mt, int shape,
+                                int num_sms, DevErr* err, cudaStream_t stream) {
+    return dispatch(shape, op == OpType::BF16, mt, false, descs, ndesc, total_tiles, num_sms, err, stream);
 }
 
 }  // namespace wg

@@ -235,7 +235,7 @@ struct Server {
     int launch(Slot& slot) {
         std::vector<InDesc> in2, in4;
         std::vector<OutDesc> out2, out4;
-        std::map<std::pair<int, int>, std::vector<GemmDesc>> gemm;  // (bn, m) -> descs
+        std::map<std::pair<int, int>, std::vector<GemmDesc>> gemm;  // (shape, m) -> descs
         long long blk_in2 = 0, blk_in4 = 0, blk_out2 = 0, blk_out4 = 0;
         int smem2 = 0, smem4 = 0;
         char* arena = static_cast<char*>(arena_base);
@@ -256,7 +256,7 @@ struct Server {
             InDesc di = make_in_desc(g, r.in, x_end, V, nullptr, &smem);
             OutDesc dout = make_out_desc(g, mtype_for(r.m), Mw, r.out, nullptr);
             GemmDesc dg;
-            const int bn = default_bn(static_cast<int>(L.k));
+            const int bn = gemm_shape(g.P, default_bn(static_cast<int>(L.k), gemm_shape(g.P, 256, false) != 256), false);
             if (make_gemm_desc(dg, OpType::F16, E, g.P, L.k, g.kp, g.cp, V, r.m == 4 ? L.U4 : L.U2, Mw, mtype_for(r.m), bn) !=
                 cudaSuccess)
                 return set_last_error(CONV2D_ERR_CUDA, "tensor map encoding failed");
@@ -344,7 +344,7 @@ struct Server {
         for (const GG& g : gg)
             if (g.m == 2 && e == cudaSuccess)
                 e = launch_gemm_grouped(reinterpret_cast<const GemmDesc*>(d + g.off), g.n, g.tiles, OpType::F16, mtype_for(g.m),
-                                        g.bn, static_cast<int>(std::min<long long>(g.tiles, num_sms)), err, s2);
+                                        g.bn, num_sms, err, s2);
         if (!out2.empty() && e == cudaSuccess)
             e = launch_output_transform_grouped(Xform::F2, MType::F16, reinterpret_cast<const OutDesc*>(d + o_out2),
                                                 static_cast<int>(out2.size()), blk_out2, err, s2);
@@ -354,7 +354,7 @@ struct Server {
         for (const GG& g : gg)
             if (g.m == 4 && e == cudaSuccess)
                 e = launch_gemm_grouped(reinterpret_cast<const GemmDesc*>(d + g.off), g.n, g.tiles, OpType::F16, mtype_for(g.m),
-                                        g.bn, static_cast<int>(std::min<long long>(g.tiles, num_sms)), err, s);
+                                        g.bn, num_sms, err, s);
         if (!out4.empty() && e == cudaSuccess)
             e = launch_output_transform_grouped(Xform::F4, MType::F24, reinterpret_cast<const OutDesc*>(d + o_out4),
                                                 static_cast<int>(out4.size()), blk_out4, err, s);
@@ -386,7 +386,7 @@ struct Server {
         const Xform xf = r.m == 4 ? Xform::F4 : Xform::F2;
         GemmPlan gp;
         if (plan_gemm(gp, OpType::F16, E, g.P, L.k, g.kp, g.cp, V, r.m == 4 ? L.U4 : L.U2, Mw, mtype_for(r.m),
-                      default_bn(static_cast<int>(L.k)), num_sms) != cudaSuccess)
+                      default_bn(static_cast<int>(L.k), gemm_shape(g.P, 256, false) != 256), num_sms) != cudaSuccess)
             return set_last_error(CONV2D_ERR_CUDA, "tensor map encoding failed");
         const void* x_end = static_cast<const uint16_t*>(r.in) + static_cast<long long>(r.n) * L.c * L.h * L.w;
         e = launch_input_transform(xf, OpType::F16, g, r.in, x_end, V, nullptr, err, plain_stream);

@@ -186,6 +186,8 @@ struct alignas(64) GemmDesc {
     // dirty lines are never written back to HBM
     const void* V;
     int v_cg, v_pp, discard_v;
+    int pair;            // made for CTA pairs: m_blocks are blocks of 256 tiles, tmB boxes of bn/2 channels
+    int bn;
     int resb;            // single launches: U block resident in shared memory, contiguous item ranges per CTA
     long long tile_begin;
     long long tiles;     // E * m_blocks * n_blocks (below 2^31)
@@ -195,22 +197,27 @@ struct alignas(64) GemmDesc {
 struct GemmPlan {
     GemmDesc desc;
     int bn;              // 32, 64, 128 or 256
-    int grid;
+    int shape;           // bn, and how it is run (gemm_shape)
+    int grid, num_sms;
     int smem_bytes;
     MType mt;
     OpType op;
 };
 
+// How a GEMM's tiles are run: output channels per tile, and whether by CTA
+// pairs (kGemmPairs).
+constexpr int kGemmPairs = 1024;
+int gemm_shape(long long P, int bn, bool m_row);
 // Builds the tensor maps; V, U, M must stay at these addresses.
 cudaError_t make_gemm_desc(GemmDesc& d, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
-                           const void* U, void* Mw, MType mt, int bn, bool m_row = false);
+                           const void* U, void* Mw, MType mt, int shape, bool m_row = false);
 cudaError_t plan_gemm(GemmPlan& gp, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
                       const void* U, void* Mw, MType mt, int bn, int num_sms, bool m_row = false);
 cudaError_t launch_gemm(const GemmPlan& gp, DevErr* err, cudaStream_t stream);
-// Many problems (same BN, operand and M types) in one persistent launch; descs
-// device-resident (64-byte aligned), sorted by tile_begin.
-cudaError_t launch_gemm_grouped(const GemmDesc* descs, int ndesc, long long total_tiles, OpType op, MType mt, int bn,
-                                int grid, DevErr* err, cudaStream_t stream);
+// Many problems (same shape, operand and M types) in one persistent launch;
+// descs device-resident (64-byte aligned), sorted by tile_begin.
+cudaError_t launch_gemm_grouped(const GemmDesc* descs, int ndesc, long long total_tiles, OpType op, MType mt, int shape,
+                                int num_sms, DevErr* err, cudaStream_t stream);
 int gemm_smem_bytes(int bn);
 
 // ---- NHWC (channels-last) input and output transforms ---------------------
