@@ -310,7 +310,7 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
         if (ce != cudaSuccess) return cuda_fail(ce, "fused plan");
         launches = 1;
         info_grid = static_cast<unsigned>(fused.m_blocks * fused.n_blocks);
-        info_threads = 320;
+        info_threads = 352;
         info_smem = fused.smem_bytes;
     } else if (algo == CONV2D_ALGO_4X3_ROW) {
         if (nhwc) {

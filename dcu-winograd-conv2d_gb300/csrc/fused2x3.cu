@@ -13,9 +13,9 @@
 //     write the 16 Winograd-domain tiles into shared memory in the tcgen05
 //     canonical K-major layout;
 //   * the transformed filter U (made once per weight set) arrives by one 4-D
-//     TMA per chunk;
+//     TMA per chunk, issued by warp 10;
 //   * warp 8 issues the 16 tcgen05.mma (M=128, N=32, K=16) per chunk from one
-//     thread, accumulating all 16 elements in the 512 TMEM columns;
+//     elected lane, accumulating all 16 elements in the 512 TMEM columns;
 //   * warp 9 issues the staging copies (so no producer warp diverges to
 //     wait for the others);
 //   * after the last chunk warps 0-7 read TMEM, apply A^T m A and write the
@@ -46,7 +46,7 @@ constexpr int kStageBytes = kABytes + kBBytes;           // 80 KB
 constexpr int kStages = 2;
 constexpr int kMaxSeg = 16;                              // images one CTA's tiles may span
 constexpr int kProducers = 256;
-constexpr int kThreads = kProducers + 64;  // + MMA warp + staging-loader warp
+constexpr int kThreads = kProducers + 96;  // + MMA, staging-loader and filter-TMA warps
 // + 256 bytes after the staging buffers: loads of padding columns (pad <= 64)
 // past the last staged row stay inside the CTA's shared memory
 constexpr int kSmemFixed = kStages * kStageBytes + 1024 /*align*/ + 512 /*barriers, segment table, zero block*/ + 256;
@@ -211,53 +211,55 @@ __global__ void __launch_bounds__(kThreads, 1)
                 issue_stage(gc + nbuf, lane);
             }
         }
-    } else if (warp == 8) {
+    } else if (warp == 10) {
+        // filter tiles: one 4-D TMA per chunk, as soon as the MMAs of the chunk
+        // two before it are done with the stage
         if (lane == 0) {
             tma_prefetch_desc(&tmU);
-            auto issue_tma = [&](int gc) {
+            for (int gc = 0; gc < total_chunks; ++gc) {
+                const int s = gc & 1;
+                if (gc >= 2 && !mbar_wait(&empty[s], ((gc >> 1) & 1) ^ 1, abort_flag, err, ERR_SITE_EMPTY)) break;
                 const int k = gc / c_chunks, c = gc - k * c_chunks;
                 const int n_blk = (blockIdx.x + k * gridDim.x) % n_blocks;
-                const int s = gc & 1;
                 mbar_arrive_expect_tx(&full[s], kBBytes);
                 tma_load_4d(smem + s * kStageBytes + kABytes, &tmU, &full[s], 0, n_blk * (kOcPerCta / 8), c * 2, 0);
-            };
-            if (total_chunks > 0) issue_tma(0);
-            if (total_chunks > 1) issue_tma(1);
-            bool ok = true;
-            for (int k = 0; k < my_items && ok; ++k) {
-                // the previous item's accumulators must be drained first
-                if (!mbar_wait(tempty, (k & 1) ^ 1, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
-                tc_fence_after();
-                for (int c = 0; c < c_chunks; ++c) {
-                    const int gc = k * c_chunks + c;
-                    const int s = gc & 1;
-                    if (!mbar_wait(&full[s], (gc >> 1) & 1, abort_flag, err, ERR_SITE_FULL)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_base = smem_u32(smem + s * kStageBytes);
-                    const uint32_t b_base = a_base + kABytes;
-#pragma unroll
-                    for (int e = 0; e < kElems; ++e) {
-                        const uint64_t ad = make_smem_desc(a_base + e * (kTilesPerCta * 16), kAHalf, 128, Swz::None);
-                        const uint64_t bd =
-                            make_smem_desc(b_base + e * (2 * kOcPerCta * 16), kOcPerCta * 16, 128, Swz::None);
-                        tc_mma_f16(tmem_base + e * kOcPerCta, ad, bd, kIdesc, c > 0 ? 1u : 0u);
-                    }
-                    tc_commit(&empty[s]);
-                    if (gc + 2 < total_chunks) {
-                        // the filter tile of chunk gc+2 reuses this stage: issue it
-                        // as soon as these MMAs retire, a whole chunk ahead of its use
-                        if (!mbar_wait(&empty[s], (gc >> 1) & 1, abort_flag, err, ERR_SITE_EMPTY)) {
-                            ok = false;
-                            break;
-                        }
-                        issue_tma(gc + 2);
-                    }
-                }
-                if (ok && !*abort_flag) tc_commit(tfull);
             }
+        }
+    } else if (warp == 8) {
+        // one elected lane of a warp-uniform loop issues the MMAs, so their
+        // descriptors stay in uniform registers
+        const bool elected = elect_one();
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t ad0 = make_smem_desc(smem_u32(smem), kAHalf, 128, Swz::None);
+        const uint64_t bd0 = make_smem_desc(smem_u32(smem) + kABytes, kOcPerCta * 16, 128, Swz::None);
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true;
+        for (int k = 0; k < my_items && ok; ++k) {
+            // the previous item's accumulators must be drained first
+            if (!mbar_wait_warp(tempty, (k & 1) ^ 1, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+            tc_fence_after();
+            for (int c = 0; c < c_chunks; ++c) {
+                if (!mbar_wait_warp(&full[s], ph, abort_flag, err, ERR_SITE_FULL)) {
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
+                const uint64_t as = ad0 + static_cast<uint32_t>(s * (kStageBytes / 16));
+                const uint64_t bs = bd0 + static_cast<uint32_t>(s * (kStageBytes / 16));
+                if (elected) {
+#pragma unroll
+                    for (int e = 0; e < kElems; ++e)
+                        tc_mma_f16(tmem_u + e * kOcPerCta, as + static_cast<uint32_t>(e * kTilesPerCta),
+                                   bs + static_cast<uint32_t>(e * 2 * kOcPerCta), kIdesc, c > 0 ? 1u : 0u);
+                    tc_commit(&empty[s]);
+                }
+                __syncwarp();
+                s ^= 1;
+                if (s == 0) ph ^= 1u;
+            }
+            if (ok && elected) tc_commit(tfull);
+            __syncwarp();
         }
     } else {
         // ---- producers: one tile and 8 channels of every chunk per thread,

@@ -214,40 +214,47 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
     } else if (warp == kMmaWarp) {
-        // one thread issues the MMAs and never waits on their completion
-        if (lane == 0) {
-            bool ok = true;
-            for (int k = 0; k < my_items && ok; ++k) {
-                if (!mbar_wait(tempty, (k & 1) ^ 1, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+        // one elected lane of a warp-uniform loop issues the MMAs (so their
+        // descriptors stay in uniform registers) and never waits on their completion
+        const bool elected = elect_one();
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t ad0 = make_smem_desc(smem_u32(astage), static_cast<uint32_t>(a_gran), 128, Swz::None);
+        const uint64_t bd0 = make_smem_desc(smem_u32(bstage), kBN * 16, 128, Swz::None);
+        const int a_step = a_bytes / 16, a_elem = 2 * a_gran / 16;
+        int sa = 0, sb = 0;
+        uint32_t aph = 0, bph = 0;
+        bool ok = true;
+        for (int k = 0; k < my_items && ok; ++k) {
+            if (!mbar_wait_warp(tempty, (k & 1) ^ 1, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+            tc_fence_after();
+            for (int c = 0; c < c_chunks; ++c) {
+                if (!mbar_wait_warp(&afull[sa], aph, abort_flag, err, ERR_SITE_FULL) ||
+                    !mbar_wait_warp(&bfull[sb], bph, abort_flag, err, ERR_SITE_FULL)) {
+                    ok = false;
+                    break;
+                }
                 tc_fence_after();
-                for (int c = 0; c < c_chunks; ++c) {
-                    const int gc = k * c_chunks + c;
-                    const int sa = gc & 1, sb = gc % nbs;
-                    if (!mbar_wait(&afull[sa], (gc >> 1) & 1, abort_flag, err, ERR_SITE_FULL) ||
-                        !mbar_wait(&bfull[sb], (gc / nbs) & 1, abort_flag, err, ERR_SITE_FULL)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_base = smem_u32(astage + sa * a_bytes);
-                    const uint32_t b_base = smem_u32(bstage + sb * kBBytes);
+                const uint64_t as = ad0 + static_cast<uint32_t>(sa * a_step);
+                const uint64_t bs = bd0 + static_cast<uint32_t>(sb * (kBBytes / 16));
+                if (elected) {
 #pragma unroll
                     for (int e = 0; e < kE; ++e) {
+                        // filter row r reads the transformed rows shifted by r rows of tiles
 #pragma unroll
-                        for (int r = 0; r < kTaps; ++r) {
-                            // filter row r reads the transformed rows shifted by r rows of tiles
-                            const uint64_t ad =
-                                make_smem_desc(a_base + e * (2 * a_gran) + r * tiles_w * 16, a_gran, 128, Swz::None);
-                            const uint64_t bd = make_smem_desc(b_base + (e * kTaps + r) * (2 * kBN * 16), kBN * 16, 128,
-                                                               Swz::None);
-                            tc_mma_f16(tmem_base + e * kBN, ad, bd, kIdesc, (c > 0 || r > 0) ? 1u : 0u);
-                        }
+                        for (int r = 0; r < kTaps; ++r)
+                            tc_mma_f16(tmem_u + e * kBN, as + static_cast<uint32_t>(e * a_elem + r * tiles_w),
+                                       bs + static_cast<uint32_t>((e * kTaps + r) * (2 * kBN)), kIdesc,
+                                       (c > 0 || r > 0) ? 1u : 0u);
                     }
                     tc_commit(&aempty[sa]);
                     tc_commit(&bempty[sb]);
                 }
-                if (ok && !*abort_flag) tc_commit(tfull);
+                __syncwarp();
+                if (++sa == kAStages) sa = 0, aph ^= 1u;
+                if (++sb == nbs) sb = 0, bph ^= 1u;
             }
+            if (ok && elected) tc_commit(tfull);
+            __syncwarp();
         }
     } else {
         // ---- producers: V of (R+2) x tiles_w tiles x 16 channels per chunk.
@@ -550,38 +557,47 @@ __global__ void __launch_bounds__(kThreadsI, 1)
             }
         }
     } else if (warp == kMmaWarpI) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int k = 0; k < my_items && ok; ++k) {
-                if (!mbar_wait(tempty, (k & 1) ^ 1, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+        // one elected lane of a warp-uniform loop issues the MMAs (so their
+        // descriptors stay in uniform registers) and never waits on their completion
+        const bool elected = elect_one();
+        const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+        const uint64_t ad0 = make_smem_desc(smem_u32(astage), static_cast<uint32_t>(a_gran), 128, Swz::None);
+        const uint64_t bd0 = make_smem_desc(smem_u32(bstage), kBN * 16, 128, Swz::None);
+        const int a_step = a_bytes / 16, a_elem = 2 * a_gran / 16;
+        int sa = 0, sb = 0;
+        uint32_t aph = 0, bph = 0;
+        bool ok = true;
+        for (int k = 0; k < my_items && ok; ++k) {
+            if (!mbar_wait_warp(tempty, (k & 1) ^ 1, abort_flag, err, ERR_SITE_TMEM_EMPTY)) break;
+            tc_fence_after();
+            for (int c = 0; c < c_chunks; ++c) {
+                if (!mbar_wait_warp(&afull[sa], aph, abort_flag, err, ERR_SITE_FULL) ||
+                    !mbar_wait_warp(&bfull[sb], bph, abort_flag, err, ERR_SITE_FULL)) {
+                    ok = false;
+                    break;
+                }
                 tc_fence_after();
-                for (int c = 0; c < c_chunks; ++c) {
-                    const int gc = k * c_chunks + c;
-                    const int sa = gc % nas, sb = gc % nbs;
-                    if (!mbar_wait(&afull[sa], (gc / nas) & 1, abort_flag, err, ERR_SITE_FULL) ||
-                        !mbar_wait(&bfull[sb], (gc / nbs) & 1, abort_flag, err, ERR_SITE_FULL)) {
-                        ok = false;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t a_base = smem_u32(astage + sa * a_bytes);
-                    const uint32_t b_base = smem_u32(bstage + sb * kBBytes);
+                const uint64_t as = ad0 + static_cast<uint32_t>(sa * a_step);
+                const uint64_t bs = bd0 + static_cast<uint32_t>(sb * (kBBytes / 16));
+                if (elected) {
 #pragma unroll
                     for (int e = 0; e < kE; ++e) {
+                        // filter row r reads the transformed rows shifted by r rows of tiles
 #pragma unroll
-                        for (int r = 0; r < kTaps; ++r) {
-                            const uint64_t ad =
-                                make_smem_desc(a_base + e * (2 * a_gran) + r * tiles_w * 16, a_gran, 128, Swz::None);
-                            const uint64_t bd = make_smem_desc(b_base + (e * kTaps + r) * (2 * kBN * 16), kBN * 16, 128,
-                                                               Swz::None);
-                            tc_mma_f16(tmem_base + e * kBN, ad, bd, kIdesc, (c > 0 || r > 0) ? 1u : 0u);
-                        }
+                        for (int r = 0; r < kTaps; ++r)
+                            tc_mma_f16(tmem_u + e * kBN, as + static_cast<uint32_t>(e * a_elem + r * tiles_w),
+                                       bs + static_cast<uint32_t>((e * kTaps + r) * (2 * kBN)), kIdesc,
+                                       (c > 0 || r > 0) ? 1u : 0u);
                     }
                     tc_commit(&aempty[sa]);
                     tc_commit(&bempty[sb]);
                 }
-                if (ok && !*abort_flag) tc_commit(tfull);
+                __syncwarp();
+                if (++sa == nas) sa = 0, aph ^= 1u;
+                if (++sb == nbs) sb = 0, bph ^= 1u;
             }
+            if (ok && elected) tc_commit(tfull);
+            __syncwarp();
         }
     } else {
         // ---- producers: task = (row of tiles rho, tile tw, granule g) in
