@@ -113,25 +113,28 @@ __device__ __forceinline__ DItem locate_direct(const DirectDesc* __restrict__ de
 }
 
 // ---- producers ----------------------------------------------------------------
-// A group of four warps writes the windows of every kGroups-th chunk.  Its
-// work is a sequence of steps (item, chunk, block of positions), each 16
-// registers of loads per thread; a step's loads are issued before the step
-// ahead of it is stored, so one load latency covers two steps.  Per block and
-// thread:
+// A group of four warps writes the windows of every kGroups-th chunk (NHWC:
+// pair of chunks).  Its work is a sequence of steps (item, chunk, block of
+// positions), each 16 registers of loads per thread; a step's loads are issued
+// before the step ahead of it is stored, so one load latency covers two steps
+// whether or not a stage is free.  Per block and thread:
 //   pairs   two neighbouring pixels of 16 planes (4-byte loads; W even, x
 //           4-byte aligned), 128 pairs; the padding of the window is cleared
 //           by the threads whose positions it is
 //   single  one position of 16 planes (2-byte loads), 128 positions
-//   NHWC    four (position, granule) of 16 bytes, 256 positions
+//   NHWC    four positions of one of the pair's four granules (16-byte loads),
+//           128 positions: a pixel's 64 bytes are half a line, one chunk's 32
+//           would make twice the requests to L2
 constexpr int kGroupThreads = 32 * kGroupWarps;
 constexpr int kMaxPadBits = 32;      // pairs: positions per thread the pad mask covers
 
 struct Step {
     uint32_t r[16];
     int p;             // pairs, single: position of the first granule; NHWC: of the block's first
-    uint32_t pads;     // pairs: bit i set where position gt + 128 i is padding (last block of a chunk only)
-    uint32_t flags;    // bit 0: first block of the chunk, 1: last, 2: pairs; 4..7: zero the granule
-                       // (single: 4); the window's length above bit 16
+    uint32_t pads;     // pairs: bit i set where position gt + 128 i is padding (last block of a chunk only);
+                       // NHWC: the first of the two chunks, counted over the CTA's items
+    uint32_t flags;    // bit 0: first block of the chunk, 1: last, 2: pairs (NHWC: there is a second
+                       // chunk), 4..7: zero the granule (single: 4); the window's length above bit 16
 };
 
 // Bytes of one granule's window in shared memory: 4 mod 8 positions, so that
@@ -143,18 +146,19 @@ struct Producer {
     const DirectDesc* __restrict__ descs;
     int ndesc, total_items, step, grp, gt;
     uint32_t rank;
-    // load cursor
-    int t, pi, c, chunks, gc0, blk, blocks;
+    // load cursor; NHWC: c counts pairs of chunks (gu0: those of earlier items)
+    int t, pi, c, chunks, gc0, blk, blocks, gu0;
     int z0, n0, win, channels;
     int pairs;
     uint32_t plane;
     const uint16_t* xi;
     // the item's first blocks: element offset from xi (-1: nothing to load) and
-    // position; NHWC: the four parts of the first two blocks
-    static constexpr int kKeep = NHWC ? 8 : 4;
+    // position; NHWC: the first positions, 32 apart
+    static constexpr int kKeep = NHWC ? 12 : 4;
     int off[kKeep];
     uint32_t pos2[2];   // positions of blocks 0, 1 and 2, 3 as 16-bit halves (-1 as 0xffff)
     uint32_t pads;
+    int far_n, far_ij, wn, wi, wj;   // NHWC: image, padded row and column of the first position past the kept ones; walk()
 
     // pairs: pair number gt + 128 i of the window, decoded from scratch (blocks past kKeep)
     __device__ __forceinline__ void locate_pair(const DirectDesc& d, int i, int& o, int& p) const {
@@ -179,7 +183,13 @@ struct Producer {
     __device__ __forceinline__ void decode(const DirectDesc& d) {
         if constexpr (NHWC) {
 #pragma unroll
-            for (int i = 0; i < kKeep; ++i) off[i] = pixel_offset<true>(d, z0 + i * 64 + (gt >> 1), n0);
+            for (int i = 0; i < kKeep; ++i) off[i] = pixel_offset<true>(d, z0 + i * 32 + (gt >> 2), n0);
+            if (win > 32 * kKeep) {
+                const int z = z0 + 32 * kKeep + (gt >> 2);
+                far_n = static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z)));
+                const int rem = z - far_n * d.img, i = static_cast<int>(fast_div(d.fd_pw, static_cast<uint32_t>(rem)));
+                far_ij = (i << 16) | (rem - i * d.pw);
+            }
         } else if (pairs) {
             // pairs 128 apart: a step of qy rows and rx columns
             const int hw = d.h * d.w, w = d.w, h = d.h, chw = d.c * hw;
@@ -223,12 +233,32 @@ struct Producer {
         }
     }
 
+    // NHWC: the pixel offset of the next position past the kept blocks, 32 on
+    // from the one before (`restart`: of the first)
+    __device__ __forceinline__ int walk(bool restart) {
+        const DirectDesc& d = descs[pi];
+        if (restart) wn = far_n, wi = far_ij >> 16, wj = far_ij & 0xffff;
+        const int y = wi - d.pad_h, x = wj - d.pad_w;
+        const bool in = wn < d.n && static_cast<unsigned>(y) < static_cast<unsigned>(d.h) &&
+                        static_cast<unsigned>(x) < static_cast<unsigned>(d.w);
+        const int o = in ? ((wn - n0) * d.h * d.w + y * d.w + x) * d.c : -1;
+        wj += d.walk_j;
+        wi += d.walk_i;
+        if (wj >= d.pw) wj -= d.pw, ++wi;
+        while (wi >= d.ph) wi -= d.ph, ++wn;
+        return o;
+    }
+
+    // the current item's chunks, or pairs of them
+    __device__ __forceinline__ int units() const { return NHWC ? (chunks + 1) / 2 : chunks; }
+
     // moves to the group's next step; false when there is none
     __device__ __forceinline__ bool advance() {
         if (++blk < blocks) return true;
         blk = 0;
         c += kGroups;
-        while (c >= chunks) {
+        while (c >= units()) {
+            gu0 += units();
             gc0 += chunks;
             chunks = 0;
             t += step;
@@ -236,8 +266,8 @@ struct Producer {
             const DItem it = locate_direct(descs, ndesc, t, pi);
             const DirectDesc& d = descs[pi];
             chunks = d.c_chunks;
-            c = (grp - gc0 % kGroups + kGroups) % kGroups;
-            if (c >= chunks) continue;
+            c = (grp - (NHWC ? gu0 : gc0) % kGroups + kGroups) % kGroups;
+            if (c >= units()) continue;
             z0 = d.pos0 + (2 * it.tile + static_cast<int>(rank)) * d.cta_rows;
             n0 = min(static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z0))), d.n - 1);
             win = d.win;
@@ -246,7 +276,7 @@ struct Producer {
             plane = static_cast<uint32_t>(d.h * d.w);
             xi = static_cast<const uint16_t*>(d.x) + static_cast<long long>(n0) * channels * plane;
             // blocks that reach into the window, for this warp's part of them
-            blocks = NHWC ? (win + 255) / 256
+            blocks = NHWC ? (win + 127) / 128
                           : max(((pairs ? win / 2 + 1 : win) - (gt & ~31) + kGroupThreads - 1) / kGroupThreads, 1);
             pads = 0;
             decode(d);
@@ -254,58 +284,62 @@ struct Producer {
         return true;
     }
 
-    __device__ __forceinline__ void load(Step& s) const {
-        const int left = channels - c * kChunkC;   // channels from this chunk on
-        s.flags = (static_cast<uint32_t>(win) << 16) | (blk == 0 ? 1u : 0u) | (blk == blocks - 1 ? 2u : 0u) | (pairs ? 4u : 0u);
-        s.pads = blk == blocks - 1 ? pads : 0u;
-        if (NHWC) {
-            const int gsel = gt & 1, ch = c * kChunkC + 8 * gsel;
-            s.p = blk * 256 + (gt >> 1);
+    __device__ __forceinline__ void load(Step& s) {
+        s.flags = (static_cast<uint32_t>(win) << 16) | (blk == 0 ? 1u : 0u) | (blk == blocks - 1 ? 2u : 0u);
+        if constexpr (NHWC) {
+            const int ch = c * 2 * kChunkC + 8 * (gt & 3);
+            const bool cin = ch < channels;
+            if (2 * c + 1 < chunks) s.flags |= 4u;
+            s.pads = static_cast<uint32_t>(gc0 + 2 * c);
+            s.p = blk * 128 + (gt >> 2);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                int o = blk == 0 ? off[k] : off[4 + k];
-                if (blk > 1) o = pixel_offset<true>(descs[pi], z0 + s.p + 64 * k, n0);
-                if (o < 0 || ch >= channels) {
+                int o = blk == 0 ? off[k] : blk == 1 ? off[4 + k] : off[8 + k];
+                if (blk > 2) o = walk(blk == 3 && k == 0);
+                if (o < 0 || !cin) {
                     o = 0;
                     s.flags |= 16u << k;
                 }
-                ldg128(xi + o + (ch < channels ? ch : 0), s.r + 4 * k);
+                ldg128(xi + o + (cin ? ch : 0), s.r + 4 * k);
+            }
+            return;
+        }
+        if (pairs) s.flags |= 4u;
+        s.pads = blk == blocks - 1 ? pads : 0u;
+        const int left = channels - c * kChunkC;   // channels from this chunk on
+        int o = off[0];
+        o = blk == 1 ? off[1] : o;
+        o = blk == 2 ? off[2] : o;
+        o = blk == 3 ? off[3] : o;
+        const uint32_t pq = blk < 2 ? pos2[0] : pos2[1];
+        int p = static_cast<int16_t>((blk & 1) ? pq >> 16 : pq);
+        if (blk >= kKeep) {
+            if (pairs) {
+                locate_pair(descs[pi], blk, o, p);
+            } else {
+                p = gt + kGroupThreads * blk;
+                o = pixel_offset<false>(descs[pi], z0 + p, n0);
+            }
+        }
+        s.p = p;
+        if (o < 0) s.flags |= 16u;
+        // padding reads the image's first pixel (cleared or not stored later)
+        const uint16_t* src = xi + max(o, 0) + static_cast<unsigned long long>(c * kChunkC) * plane;
+        if (left >= kChunkC) {
+            if (pairs) {
+#pragma unroll
+                for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg32(src + static_cast<unsigned long long>(j) * plane);
+            } else {
+#pragma unroll
+                for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg16(src + static_cast<unsigned long long>(j) * plane);
             }
         } else {
-            int o = off[0];
-            o = blk == 1 ? off[1] : o;
-            o = blk == 2 ? off[2] : o;
-            o = blk == 3 ? off[3] : o;
-            const uint32_t pq = blk < 2 ? pos2[0] : pos2[1];
-            int p = static_cast<int16_t>((blk & 1) ? pq >> 16 : pq);
-            if (blk >= kKeep) {
-                if (pairs) {
-                    locate_pair(descs[pi], blk, o, p);
-                } else {
-                    p = gt + kGroupThreads * blk;
-                    o = pixel_offset<false>(descs[pi], z0 + p, n0);
-                }
-            }
-            s.p = p;
-            if (o < 0) s.flags |= 16u;
-            // padding reads the image's first pixel (cleared or not stored later)
-            const uint16_t* src = xi + max(o, 0) + static_cast<unsigned long long>(c * kChunkC) * plane;
-            if (left >= kChunkC) {
-                if (pairs) {
+            // the last chunk of a C that is not a multiple of 16
 #pragma unroll
-                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg32(src + static_cast<unsigned long long>(j) * plane);
-                } else {
-#pragma unroll
-                    for (int j = 0; j < kChunkC; ++j) s.r[j] = ldg16(src + static_cast<unsigned long long>(j) * plane);
-                }
-            } else {
-                // the last chunk of a C that is not a multiple of 16
-#pragma unroll
-                for (int j = 0; j < kChunkC; ++j) {
-                    const uint16_t* q = src + static_cast<unsigned long long>(min(j, left - 1)) * plane;
-                    const uint32_t v = pairs ? ldg32(q) : ldg16(q);
-                    s.r[j] = j < left ? v : 0u;
-                }
+            for (int j = 0; j < kChunkC; ++j) {
+                const uint16_t* q = src + static_cast<unsigned long long>(min(j, left - 1)) * plane;
+                const uint32_t v = pairs ? ldg32(q) : ldg16(q);
+                s.r[j] = j < left ? v : 0u;
             }
         }
     }
@@ -313,17 +347,7 @@ struct Producer {
     // writes a loaded step's granules into the window stage at A
     __device__ __forceinline__ void store(const Step& s, unsigned char* A) const {
         const int s_win = static_cast<int>(s.flags >> 16), s_gran = granule_bytes(s_win);
-        if (NHWC) {
-            unsigned char* dst = A + (gt & 1) * s_gran;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int p = s.p + 64 * k;
-                const bool z = (s.flags >> (4 + k)) & 1u;
-                if (p < s_win)
-                    *reinterpret_cast<uint4*>(dst + p * 16) =
-                        make_uint4(z ? 0u : s.r[4 * k], z ? 0u : s.r[4 * k + 1], z ? 0u : s.r[4 * k + 2], z ? 0u : s.r[4 * k + 3]);
-            }
-        } else if (s.flags & 4u) {
+        if (s.flags & 4u) {
             // lanes 4-7 of every 8 store their second pixel first: the 8 lanes
             // of a store phase then write 8 different 16-byte bank groups
             const uint32_t sel0 = (gt & 4) ? 0x7632u : 0x5410u, sel1 = sel0 ^ 0x2222u;
@@ -372,10 +396,44 @@ __device__ __forceinline__ uint32_t pack2(uint32_t a, uint32_t b) {
     }
 }
 
+// NHWC: stores a loaded step once its two stages (st, st2) are free, and hands
+// them over after its last block.
+__device__ __forceinline__ bool flush_step2(const Producer<true>& pr, const Step& s, unsigned char* astage, int a_bytes,
+                                            int na, int& st, int& st2, uint64_t* afull, uint64_t* aempty,
+                                            volatile int* abort_flag, DevErr* err) {
+    const bool two = (s.flags & 4u) != 0;
+    if (s.flags & 1u) {
+        const int use = static_cast<int>(s.pads) / na;
+        st = static_cast<int>(s.pads) - use * na;
+        st2 = st + 1 == na ? 0 : st + 1;
+        const uint32_t ph = (use & 1) ^ 1, ph2 = st2 == 0 ? ph ^ 1u : ph;
+        if (!mbar_wait(&aempty[st], ph, abort_flag, err, ERR_SITE_EMPTY)) return false;
+        if (two && !mbar_wait(&aempty[st2], ph2, abort_flag, err, ERR_SITE_EMPTY)) return false;
+    }
+    const int win = static_cast<int>(s.flags >> 16), sub = pr.gt & 3;
+    unsigned char* dst = astage + (sub < 2 ? st : st2) * a_bytes + (sub & 1) * granule_bytes(win);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int p = s.p + 32 * k;
+        const bool z = (s.flags >> (4 + k)) & 1u;
+        if (p < win && (two || sub < 2))
+            *reinterpret_cast<uint4*>(dst + p * 16) =
+                make_uint4(z ? 0u : s.r[4 * k], z ? 0u : s.r[4 * k + 1], z ? 0u : s.r[4 * k + 2], z ? 0u : s.r[4 * k + 3]);
+    }
+    if (s.flags & 2u) {
+        fence_proxy_async_smem();     // the windows are read by the tensor core
+        __syncwarp();
+        if ((pr.gt & 31) == 0) {
+            mbar_arrive_cluster(map_to_rank(&afull[st], 0));
+            if (two) mbar_arrive_cluster(map_to_rank(&afull[st2], 0));
+        }
+    }
+    return true;
+}
+
 // Stores a loaded step once its stage is free; after a chunk's last block
 // hands the stage to the MMAs and moves to the group's next one.
-template <bool NHWC>
-__device__ __forceinline__ bool flush_step(const Producer<NHWC>& pr, const Step& s, unsigned char* astage, int a_bytes,
+__device__ __forceinline__ bool flush_step(const Producer<false>& pr, const Step& s, unsigned char* astage, int a_bytes,
                                            int na, int& sa, uint32_t& ph, uint64_t* afull, uint64_t* aempty,
                                            volatile int* abort_flag, DevErr* err) {
     if ((s.flags & 1u) && !mbar_wait(&aempty[sa], ph, abort_flag, err, ERR_SITE_EMPTY)) return false;
@@ -390,7 +448,11 @@ __device__ __forceinline__ bool flush_step(const Producer<NHWC>& pr, const Step&
     return true;
 }
 
-template <bool NHWC, bool BF16>
+// LATE: the kernel ahead on the stream is waited for only where its data is
+// first touched, so that the set-up (barriers, TMEM, the first item's decoding)
+// overlaps its end.  Not with descriptors in global memory, which that kernel
+// or copy may have written.
+template <bool NHWC, bool BF16, bool LATE>
 __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs, int ndesc, int total_items,
                                             const DirectRing& ring, DevErr* err) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -428,14 +490,18 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
         *abort_flag = 0;
         fence_barrier_init();
     }
-    pdl_wait();     // input and filter written, earlier readers of the output done
-    pdl_trigger();
+    if constexpr (!LATE) pdl_wait();
     if (warp == kMmaWarpD) tmem_alloc_pair(tmem_slot, 512);
     tc_fence_before();
     __syncthreads();
     cluster_sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // input and filter written, earlier readers of the output done
+    auto start = [&] {
+        if constexpr (LATE) pdl_wait();
+        pdl_trigger();
+    };
 
     if (warp < kProdWarps) {
         Producer<NHWC> pr;
@@ -447,22 +513,30 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
         pr.gt = static_cast<int>(threadIdx.x) - pr.grp * kGroupThreads;
         pr.rank = rank;
         pr.t = first - step;
-        pr.pi = pr.c = pr.chunks = pr.gc0 = pr.blk = pr.blocks = 0;
+        pr.pi = pr.c = pr.chunks = pr.gc0 = pr.gu0 = pr.blk = pr.blocks = 0;
         int sa = pr.grp;             // this group's next window stage and its phase
         uint32_t ph = 1;
         while (sa >= na) sa -= na, ph ^= 1u;
+        int st = 0, st2 = 0;
+        auto flush = [&](const Step& s) {
+            if constexpr (NHWC)
+                return flush_step2(pr, s, astage, ring.a_bytes, na, st, st2, afull, aempty, abort_flag, err);
+            else
+                return flush_step(pr, s, astage, ring.a_bytes, na, sa, ph, afull, aempty, abort_flag, err);
+        };
         bool ok = true;
         Step s0, s1;
         bool more = pr.advance();
+        start();
         if (more) pr.load(s0);
         while (more) {
             more = pr.advance();
             if (more) pr.load(s1);
-            ok = flush_step(pr, s0, astage, ring.a_bytes, na, sa, ph, afull, aempty, abort_flag, err);
+            ok = flush(s0);
             if (!ok || !more) break;
             more = pr.advance();
             if (more) pr.load(s0);
-            ok = flush_step(pr, s1, astage, ring.a_bytes, na, sa, ph, afull, aempty, abort_flag, err);
+            ok = flush(s1);
             if (!ok) break;
         }
         // the last commits on this CTA's window barriers must land before it exits
@@ -471,6 +545,7 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
                 if (!mbar_wait(&aempty[k % na], (k / na) & 1, abort_flag, err, ERR_SITE_DRAIN)) break;
     } else if (warp == kTmaWarp) {
         // ---- filter halves: one box per chunk, counted on the even CTA's barrier
+        start();
         if (lane == 0) {
             int gc = 0, pi = 0, prefetched = -1;
             bool ok = true;
@@ -503,6 +578,7 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
         //      The whole warp walks the loop with warp-uniform control flow and
         //      values, so descriptors stay in uniform registers: with one lane
         //      in the loop every MMA first moved its operands there
+        start();
         if (rank == 0) {
             int pi = 0, k = 0, sa = 0, sb = 0;
             uint32_t aph = 0, bph = 0;
@@ -557,6 +633,7 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
     } else {
         // ---- epilogue: kEpiHalves warps per TMEM lane quarter, taking blocks
         //      of 16 columns in turn
+        start();
         const int quarter = warp & 3, half = (warp - kProdWarps) >> 2;
         int pi = 0, k = 0;
         for (int t = first; t < total_items; t += step, ++k) {
@@ -650,14 +727,14 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
 template <bool NHWC, bool BF16>
 __global__ void __launch_bounds__(kDirectThreads, 1)
     direct3x3_kernel(const __grid_constant__ DirectParts parts, const __grid_constant__ DirectRing ring, DevErr* err) {
-    direct_body<NHWC, BF16>(parts.d, parts.count, parts.items, ring, err);
+    direct_body<NHWC, BF16, true>(parts.d, parts.count, parts.items, ring, err);
 }
 
 // Many problems (fp16 NCHW) as one work queue; descs device-resident, sorted by item_begin.
 __global__ void __launch_bounds__(kDirectThreads, 1)
     direct3x3_grouped(const DirectDesc* __restrict__ descs, int ndesc, int items, const __grid_constant__ DirectRing ring,
                       DevErr* err) {
-    direct_body<false, false>(descs, ndesc, items, ring, err);
+    direct_body<false, false, false>(descs, ndesc, items, ring, err);
 }
 
 // U9[tap][Cp/8][Kp][8]: the KCRS filter as granules of 8 input channels, zero
@@ -702,6 +779,10 @@ long long positions(const DirectDesc& d, long long n) {
 }
 
 int window_of(int mb, int pw) { return kRows * mb + 2 * pw + 2; }
+
+// One window stage: two granules; 32 more than a multiple of 128, so that the
+// four granules of a channels-last pixel, in two stages, fall in different banks.
+int window_bytes(int win) { return (2 * granule_bytes(win) + 127) / 128 * 128 + 32; }
 
 int b_stage_bytes(int bn) { return kTaps9 * bn * 16; }
 
@@ -785,7 +866,7 @@ struct Split {
 
 bool tile_fits(int bn, int mb, int pw, DirectRing* ring) {
     if (bn * mb > 256) return false;
-    const int a = (2 * granule_bytes(window_of(mb, pw)) + 127) / 128 * 128;
+    const int a = window_bytes(window_of(mb, pw));
     DirectRing r;
     if (!size_ring(r, a, b_stage_bytes(bn))) return false;
     if (ring) *ring = r;
@@ -886,6 +967,10 @@ cudaError_t describe_direct(DirectDesc& d, const Geom& g, bool nhwc) {
     d.step_x = (2 * kGroupThreads) % g.w;
     d.pad_step_i = kGroupThreads / d.pw;
     d.pad_step_j = kGroupThreads % d.pw;
+    d.walk_i = 32 / d.pw;
+    d.walk_j = 32 % d.pw;
+    // rows and columns of positions in 16 bits each
+    if (nhwc && (d.ph > 0x7fff || d.pw > 0xffff)) return cudaErrorNotSupported;
     d.fd_img = make_fastdiv(static_cast<uint32_t>(d.img));
     d.fd_pw = make_fastdiv(static_cast<uint32_t>(d.pw));
     d.fd_hw = make_fastdiv(static_cast<uint32_t>(static_cast<long long>(g.h) * g.w));
@@ -935,7 +1020,7 @@ cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, con
         set_tile(dp.tail, s.tail_bn, s.tail_mb);
         DirectRing r;
         // one ring serves both parts: the larger stages
-        const int a = std::max((2 * d.gran + 127) / 128 * 128, (2 * dp.tail.gran + 127) / 128 * 128);
+        const int a = std::max(window_bytes(d.win), window_bytes(dp.tail.win));
         if (size_ring(r, a, std::max(b_stage_bytes(d.bn), b_stage_bytes(dp.tail.bn))))
             dp.ring = r;
         else
@@ -1037,7 +1122,7 @@ cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDe
     int a = 0, b = 0;
     for (Pick& k : picks) {
         if (k.one > longest) choose(k, longest);
-        a = std::max(a, (2 * k.d.gran + 127) / 128 * 128);
+        a = std::max(a, window_bytes(k.d.win));
         b = std::max(b, b_stage_bytes(k.d.bn));
     }
     if (!size_ring(ring, a, b)) return cudaErrorNotSupported;

@@ -322,6 +322,7 @@ struct alignas(64) DirectDesc {
     int pairs;           // NCHW: input read as pixel pairs
     int step_y, step_x;          // 256 pixels as rows and columns of the input
     int pad_step_i, pad_step_j;  // 128 positions as rows and columns of positions
+    int walk_i, walk_j;          // 32 positions likewise
     int pos0;            // first position of item_begin's item
     int item_begin, items;
     FastDiv fd_nb, fd_img, fd_pw, fd_hw, fd_w;
