@@ -151,7 +151,7 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
     std::vector<Cand> cands;
     cands.push_back({CONV2D_ALGO_2X3_FUSED, 0});
     cands.push_back({CONV2D_ALGO_4X3_ROW, 0});
-    const int bn0 = default_bn(static_cast<int>(pr.k), true);
+    const int bn0 = default_bn(static_cast<int>(pr.k));
     for (int a : {CONV2D_ALGO_2X3_NON_FUSED, CONV2D_ALGO_4X3_NON_FUSED}) {
         cands.push_back({a, bn0});
         if (pr.k > 128) cands.push_back({a, bn0 == 256 ? 128 : 256});

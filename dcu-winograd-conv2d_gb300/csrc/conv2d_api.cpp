@@ -118,18 +118,14 @@ int options_default(conv2d_options_t* o) {
     return CONV2D_OK;
 }
 
-int default_bn(int K, bool pairs) {
+int default_bn(int K) {
     if (K <= 32) return 32;
     if (K <= 64) return 64;
     if (K <= 128) return 128;
-    // CTA pairs take in 33 KB per k-block for 256 channels and 25 KB for 128,
-    // which pays for the padding of any K (2x1920x32^2 -> 640: GEMM 23.2
-    // against 26.3 us, 2x640x64^2 -> 640 22.1 against 23.2)
-    if (pairs) return 256;
-    // prefer the tile with the least padding waste; ties go to the wider tile
-    const int w256 = ((K + 255) / 256) * 256 - K;
-    const int w128 = ((K + 127) / 128) * 128 - K;
-    return w256 <= w128 ? 256 : 128;
+    // by pairs a k-block of 256 channels brings 33 KB into each SM and one of
+    // 128 25 KB, which pays for the padding of any K (2x1920x32^2 -> 640: GEMM
+    // 23.2 against 26.3 us)
+    return 256;
 }
 
 // item shape of the direct kernel: gemm_bn where it names one, else from the sizes
@@ -334,7 +330,7 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
                             "NHWC needs C a multiple of 8 and rows within one TMA box (about 250 columns)");
             if (ce != cudaSuccess) return cuda_fail(ce, "NHWC tensor map");
         }
-        const int bn = opt.gemm_bn ? opt.gemm_bn : default_bn(g.k, gemm_shape(Pc, 256, m_row()) != 256);
+        const int bn = opt.gemm_bn;
         ce = plan_gemm(gemm_full, op, E, Pc, g.k, g.kp, g.cp, V, U, Mw, mt, bn, num_sms, m_row());
         if (ce != cudaSuccess) return cuda_fail(ce, "GEMM plan (tensor maps)");
         n_chunks = (static_cast<int>(pr->n) + chunk_n - 1) / chunk_n;

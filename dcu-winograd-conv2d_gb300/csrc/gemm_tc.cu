@@ -901,16 +901,68 @@ cudaError_t make_gemm_desc(GemmDesc& d, OpType op, int E, long long P, int K, in
 // single-CTA kernel.
 int gemm_shape(long long P, int bn, bool m_row) { return bn >= 128 && !m_row && P > kBM ? bn | kGemmPairs : bn; }
 
-cudaError_t plan_gemm(GemmPlan& gp, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
-                      const void* U, void* Mw, MType mt, int bn, int num_sms, bool m_row) {
-    // U block of one (element, channel block) within the resident budget: it
-    // stays in shared memory over consecutive tile blocks instead of being
-    // reloaded from L2 for every work item (32 x 256 x 56^2 -> 256: 226 of
-    // the 339 MB of operand loads); WG_CONV2D_GEMM_RESIDENT_U=0 turns it off
+namespace {
+
+// Whether the U block of one (element, channel block) stays in shared memory
+// over consecutive tile blocks instead of being reloaded from L2 for every
+// work item (32 x 256 x 56^2 -> 256: 226 of the 339 MB of operand loads): it
+// has to fit the budget, and the items to fill the SMs;
+// WG_CONV2D_GEMM_RESIDENT_U=0 turns it off.
+bool resident_u(int E, long long P, int K, int Cp, int bn, int num_sms) {
     const char* res = std::getenv("WG_CONV2D_GEMM_RESIDENT_U");
     const long long m_blocks = (P + kBM - 1) / kBM, n_blocks = (K + bn - 1) / bn, k_blocks = (Cp + kBK - 1) / kBK;
-    const bool resb = !(res && res[0] == '0') && k_blocks * bn * kBK * 2 <= kResBBytes && E * m_blocks * n_blocks >= num_sms;
-    gp.shape = resb ? bn : gemm_shape(P, bn, m_row);
+    return !(res && res[0] == '0') && k_blocks * bn * kBK * 2 <= kResBBytes && E * m_blocks * n_blocks >= num_sms;
+}
+
+// Cycles of a single-problem launch: rounds of items, each the bytes it moves
+// into an SM (V and U blocks, 45 a cycle) and out of it (M, 40), and what an
+// item costs however short.  Fitted to this kernel's times: 32x512x28^2 -> 512
+// by BN 256 single CTAs 38.5 us, pairs 34.4, BN 128 resident 46.7; 2x640x64^2
+// -> 640 by BN 128 24.2, BN 256 pairs 22.1; 3x300x25x40 -> 150, one round
+// either way, 8.3 single and 9.8 by pairs.
+double gemm_cycles(int E, long long P, int K, int Cp, MType mt, int bn, bool pair, int num_sms) {
+    const long long bm = pair ? 2 * kBM : kBM, slots = pair ? direct_max_pairs(num_sms) : num_sms;
+    const long long items = E * ((P + bm - 1) / bm) * ((K + bn - 1) / bn), k_blocks = (Cp + kBK - 1) / kBK;
+    const bool resident = !pair && resident_u(E, P, K, Cp, bn, num_sms);
+    const double in = k_blocks * (kTileABytes + (resident ? 0.0 : kBK * 2.0 * (pair ? bn / 2 : bn)));
+    const double out = kBM * static_cast<double>(std::min(bn, K)) * (mt == MType::F16 ? 2 : mt == MType::F24 ? 3 : 4);
+    return static_cast<double>((items + slots - 1) / slots) * (in / 45 + out / 40 + (pair || resident ? 2500 : 1300));
+}
+
+}  // namespace
+
+// The tile for a single-problem launch, of `bn` channels or (0) of any width:
+// the fewest cycles.  On 2x640x64^2 -> 640 (BN 128 / 256 by single CTAs, 128 /
+// 256 by pairs) that is 256 by pairs, GEMM 22.1 us against 24.2 for 128 by
+// single CTAs; on 4x100x30^2 -> 200, 72 items against 36, 128 by pairs.
+int gemm_pick(int E, long long P, int K, int Cp, MType mt, int bn, bool m_row, int num_sms) {
+    // one block of tiles: few CTAs, whose time the kernels around them hide in
+    // part, so that the model says little (16x512x7^2 -> 512, F(4x3): BN 128
+    // 8.8 us by itself against 9.8 for 256, but 21.7 against 19.0 per call);
+    // the width with the least padding, the wider of two
+    if (!bn && K > 128 && P <= kBM) bn = (K + 255) / 256 * 256 <= (K + 127) / 128 * 128 ? 256 : 128;
+    const int least = bn ? bn : K <= 32 ? 32 : K <= 64 ? 64 : 128, most = bn ? bn : K <= 128 ? least : 256;
+    int best = 0;
+    double best_cycles = 0;
+    for (int b = least; b <= most; b *= 2)
+        for (int shape : {b, gemm_shape(P, b, m_row)}) {
+            // one round of single-CTA items is bound by latency, which pairs add to
+            // (40x512x7^2 -> 512 F(4x3): 12.9 us single, 14.0 by pairs)
+            if ((shape & kGemmPairs) && E * ((P + kBM - 1) / kBM) * ((K + b - 1) / b) <= num_sms) continue;
+            const double t = gemm_cycles(E, P, K, Cp, mt, b, (shape & kGemmPairs) != 0, num_sms);
+            if (best == 0 || t < best_cycles) {
+                best = shape;
+                best_cycles = t;
+            }
+        }
+    return best;
+}
+
+cudaError_t plan_gemm(GemmPlan& gp, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
+                      const void* U, void* Mw, MType mt, int bn, int num_sms, bool m_row) {
+    gp.shape = gemm_pick(E, P, K, Cp, mt, bn, m_row, num_sms);
+    bn = gp.shape & ~kGemmPairs;
+    const bool resb = gp.shape == bn && resident_u(E, P, K, Cp, bn, num_sms);
     cudaError_t e = make_gemm_desc(gp.desc, op, E, P, K, Kp, Cp, V, U, Mw, mt, gp.shape, m_row);
     if (e != cudaSuccess) return e;
     gp.desc.resb = resb ? 1 : 0;

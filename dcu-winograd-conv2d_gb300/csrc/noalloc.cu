@@ -115,8 +115,7 @@ extern "C" int conv2d_fp16_noalloc(const problem_t* problem, void* stream) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     GemmPlan gp;
-    const int bn = default_bn(g.k, gemm_shape(g.P, 256, false) != 256);
-    if (plan_gemm(gp, OpType::F16, 16, g.P, g.k, g.kp, g.cp, V, U, Mw, MType::F16, bn, sms > 0 ? sms : 1) != cudaSuccess)
+    if (plan_gemm(gp, OpType::F16, 16, g.P, g.k, g.kp, g.cp, V, U, Mw, MType::F16, 0, sms > 0 ? sms : 1) != cudaSuccess)
         return noalloc_fail(CONV2D_ERR_CUDA, "tensor map encoding failed");
     // the error word starts every call at zero; U, V and M are rewritten in
     // full (padding included) by the kernels below

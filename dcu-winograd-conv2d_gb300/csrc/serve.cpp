@@ -256,7 +256,7 @@ struct Server {
             InDesc di = make_in_desc(g, r.in, x_end, V, nullptr, &smem);
             OutDesc dout = make_out_desc(g, mtype_for(r.m), Mw, r.out, nullptr);
             GemmDesc dg;
-            const int bn = gemm_shape(g.P, default_bn(static_cast<int>(L.k), gemm_shape(g.P, 256, false) != 256), false);
+            const int bn = gemm_shape(g.P, default_bn(static_cast<int>(L.k)), false);
             if (make_gemm_desc(dg, OpType::F16, E, g.P, L.k, g.kp, g.cp, V, r.m == 4 ? L.U4 : L.U2, Mw, mtype_for(r.m), bn) !=
                 cudaSuccess)
                 return set_last_error(CONV2D_ERR_CUDA, "tensor map encoding failed");
@@ -386,7 +386,7 @@ struct Server {
         const Xform xf = r.m == 4 ? Xform::F4 : Xform::F2;
         GemmPlan gp;
         if (plan_gemm(gp, OpType::F16, E, g.P, L.k, g.kp, g.cp, V, r.m == 4 ? L.U4 : L.U2, Mw, mtype_for(r.m),
-                      default_bn(static_cast<int>(L.k), gemm_shape(g.P, 256, false) != 256), num_sms) != cudaSuccess)
+                      0, num_sms) != cudaSuccess)
             return set_last_error(CONV2D_ERR_CUDA, "tensor map encoding failed");
         const void* x_end = static_cast<const uint16_t*>(r.in) + static_cast<long long>(r.n) * L.c * L.h * L.w;
         e = launch_input_transform(xf, OpType::F16, g, r.in, x_end, V, nullptr, err, plain_stream);

@@ -207,10 +207,11 @@ struct GemmPlan {
 // How a GEMM's tiles are run: output channels per tile, and whether by CTA
 // pairs (kGemmPairs).
 constexpr int kGemmPairs = 1024;
-int gemm_shape(long long P, int bn, bool m_row);
+int gemm_shape(long long P, int bn, bool m_row);   // of `bn` channels in a launch of many problems
 // Builds the tensor maps; V, U, M must stay at these addresses.
 cudaError_t make_gemm_desc(GemmDesc& d, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
                            const void* U, void* Mw, MType mt, int shape, bool m_row = false);
+// bn 0: chosen from the sizes
 cudaError_t plan_gemm(GemmPlan& gp, OpType op, int E, long long P, int K, int Kp, int Cp, const void* V,
                       const void* U, void* Mw, MType mt, int bn, int num_sms, bool m_row = false);
 cudaError_t launch_gemm(const GemmPlan& gp, DevErr* err, cudaStream_t stream);

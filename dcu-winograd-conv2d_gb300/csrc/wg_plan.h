@@ -130,8 +130,8 @@ class DeviceGuard {
 
 int validate_problem(const problem_t* pr);
 int options_default(conv2d_options_t* o);
-// GEMM output-channel tile; pairs: run by CTA pairs (gemm_shape)
-int default_bn(int K, bool pairs);
+// GEMM output-channel tile in a launch of many problems
+int default_bn(int K);
 int select_reference64(unsigned long long n, unsigned long long c, unsigned long long h, unsigned long long w,
                        unsigned long long k, unsigned long long r, unsigned long long s, unsigned long long oh,
                        unsigned long long ow);
