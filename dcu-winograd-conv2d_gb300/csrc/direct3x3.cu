@@ -816,10 +816,10 @@ double item_cycles(int bn, int mb, int pw, int chunks) {
     return chunks * std::max(mma, prod) + 1200.0 + 120.0 * mb * bn / 32;
 }
 
-template <class F, class... Args>
-cudaError_t launch_cluster(F kern, int pairs, int smem, cudaStream_t s, const Args&... args) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem);
-    return e == cudaSuccess ? launch_pairs(kern, pairs, kDirectThreads, smem, s, args...) : e;
+template <auto Kernel, class... Args>
+cudaError_t launch_cluster(int pairs, int smem, cudaStream_t s, const Args&... args) {
+    const cudaError_t e = allow_smem<Kernel>(kMaxSmem);
+    return e == cudaSuccess ? launch_pairs(Kernel, pairs, kDirectThreads, smem, s, args...) : e;
 }
 
 // CTA pairs that run at once (one CTA per SM; a cluster stays within a GPC)
@@ -1144,17 +1144,17 @@ cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDe
 
 cudaError_t launch_direct_grouped(const DirectDesc* descs, int ndesc, int items, const DirectRing& ring, int pairs, DevErr* err,
                                   cudaStream_t stream) {
-    return launch_cluster(direct3x3_grouped, std::min(items, pairs), ring.smem_bytes, stream, descs, ndesc, items, ring, err);
+    return launch_cluster<direct3x3_grouped>(std::min(items, pairs), ring.smem_bytes, stream, descs, ndesc, items, ring, err);
 }
 
 cudaError_t launch_direct(const DirectPlan& dp, const void* x, void* y, int n_images, DevErr* err, cudaStream_t stream) {
     DirectParts p;
     const int pairs = std::min(direct_parts(dp, x, y, n_images, p), dp.max_pairs);
     if (dp.nhwc)
-        return dp.bf16 ? launch_cluster(direct3x3_kernel<true, true>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
-                       : launch_cluster(direct3x3_kernel<true, false>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
-    return dp.bf16 ? launch_cluster(direct3x3_kernel<false, true>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
-                   : launch_cluster(direct3x3_kernel<false, false>, pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
+        return dp.bf16 ? launch_cluster<direct3x3_kernel<true, true>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
+                       : launch_cluster<direct3x3_kernel<true, false>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
+    return dp.bf16 ? launch_cluster<direct3x3_kernel<false, true>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
+                   : launch_cluster<direct3x3_kernel<false, false>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
 }
 
 }  // namespace wg

@@ -707,12 +707,12 @@ cudaError_t gemm_pair_launch(bool single, const GemmDesc* d, int ndesc, long lon
     constexpr int smem = PairCfg<BN>::kSmem;
     static_assert(smem > 116 * 1024, "one CTA per SM: each takes all of TMEM");
     if (single) {
-        auto kern = wino_gemm_pair_kernel<BN, BF16, MT>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        constexpr auto kern = wino_gemm_pair_kernel<BN, BF16, MT>;
+        cudaError_t e = allow_smem<kern>(smem);
         return e == cudaSuccess ? launch_pairs(kern, pairs, kGemmThreads, smem, s, *d, err) : e;
     }
-    auto kern = wino_gemm_pair_grouped<BN, BF16, MT>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr auto kern = wino_gemm_pair_grouped<BN, BF16, MT>;
+    cudaError_t e = allow_smem<kern>(smem);
     return e == cudaSuccess ? launch_pairs(kern, pairs, kGemmThreads, smem, s, d, ndesc, total, err) : e;
 }
 
@@ -746,8 +746,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 template <int BN, bool BF16, class MT, bool RESB>
 cudaError_t gemm_launch_r(const GemmDesc& d, int grid, DevErr* err, cudaStream_t s) {
     using Cfg = GemmCfg<BN, RESB>;
-    auto kern = wino_gemm_kernel<BN, BF16, MT, RESB>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemRow);
+    constexpr auto kern = wino_gemm_kernel<BN, BF16, MT, RESB>;
+    cudaError_t e = allow_smem<kern>(Cfg::kSmemRow);
     if (e != cudaSuccess) return e;
     return launch_pdl(kern, dim3(grid), dim3(kGemmThreads), d.m_row ? Cfg::kSmemRow : Cfg::kSmem, s, d, err);
 }
@@ -760,9 +760,9 @@ cudaError_t gemm_launch(const GemmDesc& d, int grid, DevErr* err, cudaStream_t s
 template <int BN, bool BF16, class MT>
 cudaError_t gemm_grouped_launch(const GemmDesc* descs, int ndesc, long long total, int grid, DevErr* err,
                                 cudaStream_t s) {
-    auto kern = wino_gemm_grouped<BN, BF16, MT>;
+    constexpr auto kern = wino_gemm_grouped<BN, BF16, MT>;
     // grouped problems write granule-layout M
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN>::kSmemRow);
+    cudaError_t e = allow_smem<kern>(GemmCfg<BN>::kSmemRow);
     if (e != cudaSuccess) return e;
     return launch_pdl(kern, dim3(grid), dim3(kGemmThreads), GemmCfg<BN>::kSmem, s, descs, ndesc, total, err);
 }

@@ -908,12 +908,12 @@ cudaError_t launch_row4x3i(const RowPlan& rp, void* out, int n_base, int n_image
         sms = 148;
     const dim3 grid(static_cast<unsigned>(std::min<long long>(items, sms)));
     if (rp.out_nhwc) {
-        cudaError_t e = cudaFuncSetAttribute(row4x3i_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, rp.smem_bytes);
+        cudaError_t e = allow_smem<row4x3i_kernel<true>>(rp.smem_bytes);
         if (e != cudaSuccess) return e;
         return launch_pdl(row4x3i_kernel<true>, grid, dim3(kThreadsI), rp.smem_bytes, s, rp.tmX, rp.tmU,
                           static_cast<__half*>(out), gg, n_base, n_images, err);
     }
-    cudaError_t e = cudaFuncSetAttribute(row4x3i_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, rp.smem_bytes);
+    cudaError_t e = allow_smem<row4x3i_kernel<false>>(rp.smem_bytes);
     if (e != cudaSuccess) return e;
     return launch_pdl(row4x3i_kernel<false>, grid, dim3(kThreadsI), rp.smem_bytes, s, rp.tmX, rp.tmU,
                       static_cast<__half*>(out), gg, n_base, n_images, err);
@@ -949,7 +949,7 @@ cudaError_t launch_row4x3(const RowPlan& rp, const void* x, const void* x_end, v
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
         sms <= 0)
         sms = 148;
-    cudaError_t e = cudaFuncSetAttribute(row4x3_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rp.smem_bytes);
+    cudaError_t e = allow_smem<row4x3_kernel>(rp.smem_bytes);
     if (e != cudaSuccess) return e;
     return launch_pdl(row4x3_kernel, dim3(static_cast<unsigned>(std::min<long long>(items, sms))), dim3(kThreads),
                       rp.smem_bytes, s, static_cast<const __half*>(x), static_cast<const __half*>(x_end), rp.tmU,

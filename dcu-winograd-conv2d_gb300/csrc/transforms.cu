@@ -1015,14 +1015,14 @@ InBlocking choose_in_blocking(const Geom& g) {
 
 template <class TF, class OutT, bool SCALED, bool XB = false, bool KEEP = false>
 cudaError_t input_launch(const InDesc& d, int smem, DevErr* err, cudaStream_t s) {
-    auto kern = input_transform_kernel<TF, OutT, SCALED, XB, KEEP>;
+    constexpr auto kern = input_transform_kernel<TF, OutT, SCALED, XB, KEEP>;
     // a third staging buffer where two CTAs of three still fit an SM: the
     // next item's copies then start two items ahead of the arithmetic
     const int buf = (smem - kInHeader - 2 * kInSlack) / 2;
     const int smem3 = kInHeader + 2 * kInSlack + 3 * buf;
     const int nbufs = in_ctas_per_sm(smem3) >= 2 ? 3 : 2;
     if (nbufs == 3) smem = smem3;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const long long total = d.gx * d.gy;
     const long long grid = std::min<long long>(total, static_cast<long long>(sm_count()) * in_ctas_per_sm(smem));
@@ -1032,8 +1032,8 @@ cudaError_t input_launch(const InDesc& d, int smem, DevErr* err, cudaStream_t s)
 template <class TF, class OutT, bool SCALED>
 cudaError_t input_grouped_launch(const InDesc* descs, int ndesc, long long total, int smem, DevErr* err,
                                  cudaStream_t s) {
-    auto kern = input_transform_grouped<TF, OutT, SCALED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr auto kern = input_transform_grouped<TF, OutT, SCALED>;
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const long long grid = std::min<long long>(total, static_cast<long long>(sm_count()) * in_ctas_per_sm(smem));
     return launch_pdl(kern, dim3(static_cast<unsigned>(grid)), dim3(kInThreads), smem, s, descs, ndesc, total,
@@ -1044,9 +1044,9 @@ template <class TF, class MT, bool YB = false>
 cudaError_t output_launch(const OutDesc& d, DevErr* err, cudaStream_t s) {
     const long long total = (d.P + kOsTiles - 1) / kOsTiles * d.KG;
     if (total <= 0) return cudaSuccess;
-    auto kern = output_transform_staged<TF, MT, YB>;
+    constexpr auto kern = output_transform_staged<TF, MT, YB>;
     constexpr int smem = os_smem_bytes<TF>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const int per_sm = std::max(1, std::min(4, 233472 / (smem + 1024)));
     const long long grid = std::min<long long>(total, static_cast<long long>(sm_count()) * per_sm);
@@ -1057,9 +1057,9 @@ template <class TF, bool YB = false, bool YNHWC = false>
 cudaError_t output_launch_m24(const OutDesc& d, DevErr* err, cudaStream_t s) {
     const long long total = (d.P + kOsTiles - 1) / kOsTiles * d.KG;
     if (total <= 0) return cudaSuccess;
-    auto kern = output_transform_staged_m24<TF, YB, YNHWC>;
+    constexpr auto kern = output_transform_staged_m24<TF, YB, YNHWC>;
     constexpr int smem = os24_smem_bytes<TF>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const int per_sm = std::max(1, std::min(2, 233472 / (smem + 1024)));
     const long long grid = std::min<long long>(total, static_cast<long long>(sm_count()) * per_sm);
@@ -1069,9 +1069,9 @@ cudaError_t output_launch_m24(const OutDesc& d, DevErr* err, cudaStream_t s) {
 template <class TF>
 cudaError_t output_grouped_launch_m24(const OutDesc* descs, int ndesc, long long blocks, DevErr* err, cudaStream_t s) {
     if (blocks <= 0) return cudaSuccess;
-    auto kern = output_transform_staged_m24_grouped<TF>;
+    constexpr auto kern = output_transform_staged_m24_grouped<TF>;
     constexpr int smem = os24_smem_bytes<TF>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const int per_sm = std::max(1, std::min(2, 233472 / (smem + 1024)));
     const long long grid = std::min<long long>(blocks, static_cast<long long>(sm_count()) * per_sm);
@@ -1081,9 +1081,9 @@ cudaError_t output_grouped_launch_m24(const OutDesc* descs, int ndesc, long long
 template <class TF, class MT>
 cudaError_t output_grouped_launch(const OutDesc* descs, int ndesc, long long blocks, DevErr* err, cudaStream_t s) {
     if (blocks <= 0) return cudaSuccess;
-    auto kern = output_transform_staged_grouped<TF, MT>;
+    constexpr auto kern = output_transform_staged_grouped<TF, MT>;
     constexpr int smem = os_smem_bytes<TF>();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem<kern>(smem);
     if (e != cudaSuccess) return e;
     const int per_sm = std::max(1, std::min(4, 233472 / (smem + 1024)));
     const long long grid = std::min<long long>(blocks, static_cast<long long>(sm_count()) * per_sm);

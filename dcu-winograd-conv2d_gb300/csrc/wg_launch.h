@@ -7,6 +7,7 @@
 // launches; only the launch gap and prologue overlap.  WG_CONV2D_PDL=0 turns
 // it off (plain launches).
 #pragma once
+#include <atomic>
 #include <cstdlib>
 #include <utility>
 
@@ -20,6 +21,22 @@ inline bool pdl_enabled() {
         return !(v && v[0] == '0');
     }();
     return on;
+}
+
+// Raises the kernel's dynamic shared memory limit to `bytes` on the current
+// device, once (the limit stays until the process ends): asking the runtime on
+// every launch cost 0.3-0.4 us of host time (a call of one kernel 3.58 -> 3.18 us
+// to submit, of three 7.6 -> 6.7).
+template <auto Kernel>
+cudaError_t allow_smem(int bytes) {
+    constexpr int kDevices = 64;
+    static std::atomic<int> allowed[kDevices] = {};
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+    if (dev < kDevices && allowed[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess && dev < kDevices) allowed[dev].store(bytes, std::memory_order_relaxed);
+    return e;
 }
 
 template <class... KArgs, class... Args>
