@@ -445,7 +445,9 @@ int Plan::run(cudaStream_t s) {
 // overlap each other.  The host link bounds this call for large inputs (on
 // the GB300 measured: 206 GB/s in, 190 GB/s out, 312 GB/s for both at once,
 // whether copy engines or SM loads and stores move the bytes).  Chunks hold at
-// least 6 MB of copies and there are at most 8 of them: on the 32 x 256 x 56^2
+// least 6 MB of copies (two chunks from 4 MB in all: 16x128x28^2 -> 128, 6.4 MB,
+// 60 us in two, 66 in one, 77 in four; 8x64x28^2 -> 64, 1.6 MB, 39 in two, 33 in
+// one) and there are at most 8 of them: on the 32 x 256 x 56^2
 // layer (103 MB of copies) 8 chunks took 402-411 us per call, 6 took 420,
 // 4 took 439, 12 and 16 took 450; chunks ramping from 1 image up to 4 and
 // back measured 418-428 us against 415 for 8 x 4.  WG_CONV2D_HOST_CHUNKS sets
@@ -484,8 +486,9 @@ int host_schedule(int n, long long img_copy_bytes, int* sizes) {
     const long long total = static_cast<long long>(n) * img_copy_bytes;
     long long max_chunks = 8;
     if (const char* e = std::getenv("WG_CONV2D_HOST_CHUNKS")) max_chunks = std::max(1, std::min(std::atoi(e), Plan::kMaxHostChunks));
-    const int chunks = static_cast<int>(
-        std::max(1LL, std::min<long long>({static_cast<long long>(n), max_chunks, total / (6LL << 20)})));
+    // two from 4 MB on: there the overlap outweighs the events between the streams
+    const long long wanted = std::max(total / (6LL << 20), total >= (4LL << 20) ? 2LL : 1LL);
+    const int chunks = static_cast<int>(std::max(1LL, std::min<long long>({static_cast<long long>(n), max_chunks, wanted})));
     const int per = (n + chunks - 1) / chunks;
     int cnt = 0;
     for (int done = 0; done < n; done += per) sizes[cnt++] = std::min(per, n - done);
@@ -596,6 +599,25 @@ int Plan::enqueue_host(const void* const* host_in, void* const* host_out, int st
     // the non-fused workspace holds chunk_n images: a host chunk runs as
     // ranges of at most that many
     const int cap = single_kernel() ? n : chunk_n;
+    auto compute = [&](int n0, int images) {
+        for (int r0 = n0; r0 < n0 + images; r0 += cap) {
+            const int nc = std::min(cap, n0 + images - r0);
+            const GemmPlan* gp = nullptr;
+            if (!single_kernel() && !(gp = host_gemm_for(nc))) return fail(CONV2D_ERR_CUDA, "GEMM plan (host chunks) failed");
+            if (const int rs = run_range(r0, nc, gp, s)) return rs;
+        }
+        return static_cast<int>(CONV2D_OK);
+    };
+    // one batch in one chunk: nothing overlaps, so the copies go to the compute
+    // stream and no event is waited for (16x128x28^2 -> 128 in one chunk: 72 us
+    // instead of 75)
+    if (nch == 1 && steps == 1) {
+        cudaError_t ce = cudaMemcpyAsync(prob.in, host_in[0], n * in_img_b, cudaMemcpyHostToDevice, s);
+        if (ce != cudaSuccess) return cuda_fail(ce, "input copy");
+        if (const int rs = compute(0, n)) return rs;
+        ce = cudaMemcpyAsync(host_out[0], prob.out, n * out_img_b, cudaMemcpyDeviceToHost, s);
+        return ce == cudaSuccess ? CONV2D_OK : cuda_fail(ce, "output copy");
+    }
     cudaEvent_t* ev_in = host_ev;                         // [kMaxHostChunks]
     cudaEvent_t* ev_done = host_ev + kMaxHostChunks;      // [kMaxHostChunks]
     cudaEvent_t* ev_out = host_ev + 2 * kMaxHostChunks;   // [kMaxHostChunks]
@@ -629,13 +651,7 @@ int Plan::enqueue_host(const void* const* host_in, void* const* host_out, int st
         if (ce != cudaSuccess) return cuda_fail(ce, "input copy");
         cudaStreamWaitEvent(s, ev_in[i], 0);
         if (st > 0) cudaStreamWaitEvent(s, ev_out[i], 0);   // step st-1's output copy read these rows
-        for (int r0 = n0; r0 < n0 + sizes[i]; r0 += cap) {
-            const int nc = std::min(cap, n0 + sizes[i] - r0);
-            const GemmPlan* gp = nullptr;
-            if (!single_kernel() && !(gp = host_gemm_for(nc))) return fail(CONV2D_ERR_CUDA, "GEMM plan (host chunks) failed");
-            const int rs = run_range(r0, nc, gp, s);
-            if (rs) return rs;
-        }
+        if (const int rs = compute(n0, sizes[i])) return rs;
         cudaEventRecord(ev_done[i], s);
         cudaStreamWaitEvent(host_out_stream, ev_done[i], 0);
         ce = cudaMemcpyAsync(static_cast<char*>(host_out[st]) + n0 * out_img_b,

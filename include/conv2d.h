@@ -158,7 +158,7 @@ int conv2d_fp16_ex(const void* param_ptr, void* stream);
 /* End-to-end call with HOST buffers: copies host_in (n*c*h*w fp16) to the
  * problem's device input, runs, copies the output to host_out and waits for
  * the stream.  The batch is cut into up to 8 image chunks (at least 6 MB of
- * copies each; WG_CONV2D_HOST_CHUNKS / WG_CONV2D_HOST_SIZES override) whose
+ * copies each, or two of at least 2 MB; WG_CONV2D_HOST_CHUNKS / WG_CONV2D_HOST_SIZES override) whose
  * input copies, compute and output copies overlap (two internal copy
  * streams); with pinned host memory the copies run at full link speed. */
 int conv2d_fp16_host(const void* param_ptr, const void* host_in, void* host_out, void* stream);
