@@ -8,7 +8,8 @@
 // the same choice without measuring.  The reference selection wins unless
 // another candidate is more than 3% faster, so noise between nearly equal
 // candidates cannot flip the choice from run to run.  The direct kernel is
-// timed as well: where it is faster than the winner, calls run it.
+// timed as well: where it is faster than the winner, calls run it.  Times are
+// weighed by accuracy (accuracy_weight).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -35,13 +36,21 @@ struct Choice {
     bool direct;   // the direct kernel ran faster
 };
 
-// Direct-convolution operations per second the direct kernel holds under the
-// board's power cap: 32 x 256 x 56^2 -> 256 takes 70 us in the first
-// milliseconds, as it is timed here, and 82.5 us (1,435 TFLOP/s) once calls
+// Operations per second, padding included, that the direct kernel holds under
+// the board's power cap: 32 x 256 x 56^2 -> 256 takes 70 us in the first
+// milliseconds, as it is timed here, and 82.5 us (1,487 TFLOP/s) once calls
 // have run back to back for some tenths of a second; the Winograd paths, with
 // 0.25-0.5 of its products, keep their times (101.7 us).  32 x 512 x 28^2 ->
-// 512, 70.5 us here against F(4x3)'s 71.1, would be 80 us in earnest.
-constexpr double kSustainedFlops = 1.43e15;
+// 512, 70.5 us here against F(4x3)'s 65.5, would be 80 us in earnest.
+constexpr double kSustainedFlops = 1.48e15;
+
+// Candidates within a few percent of one another change places with every
+// measurement; the more accurate one then wins.  Relative errors against 64
+// bits (fp16 tensors): direct 2.1e-4, F(2x3) 6.4e-4, row F(4x3) 9.5e-4, F(4x3)
+// 2.0e-3.
+float accuracy_weight(int algo) {
+    return algo == CONV2D_ALGO_4X3_NON_FUSED ? 1.08f : algo == CONV2D_ALGO_4X3_ROW ? 1.04f : 1.f;
+}
 
 // In the tune file the algorithm's number carries the direct kernel's flag.
 constexpr int kDirectFlag = 16;
@@ -162,20 +171,23 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
     for (const Cand& cd : cands) {
         const float ms = time_candidate(pr, opt, cd.algo, cd.bn, scratch, s);
         if (ms < 0.f) continue;
-        if (cd.algo == fallback && (ref_ms < 0.f || ms < ref_ms)) {
-            ref_ms = ms;
+        const float weighed = ms * accuracy_weight(cd.algo);
+        if (cd.algo == fallback && (ref_ms < 0.f || weighed < ref_ms)) {
+            ref_ms = weighed;
             ref_bn = cd.bn;
         }
-        if (best.ms < 0.f || ms < best.ms) best = Choice{cd.algo, cd.bn, ms, false};
+        if (best.ms < 0.f || weighed < best.ms) best = Choice{cd.algo, cd.bn, weighed, false};
     }
     const float direct_ms = best.ms < 0.f ? -1.f : time_candidate(pr, opt, CONV2D_ALGO_DIRECT, 0, scratch, s);
     cudaStreamDestroy(s);
     cudaFree(scratch);
     if (ref_ms > 0.f && best.ms > 0.f && best.ms > ref_ms / 1.03f) best = Choice{fallback, ref_bn, ref_ms, false};
     if (best.ms < 0.f) best = Choice{fallback, 0, 0.f, false};
-    // no margin: its result is the more accurate one
-    const double flops = 18.0 * pr.n * pr.c * pr.k * (pr.h + 2.0 * pr.p - 2) * (pr.w + 2.0 * pr.q - 2);
+    // the kernel multiplies whole rows with their padding, 16 channels and 32 filters at a time
+    const double positions = pr.n * (pr.h + std::max<double>(pr.p, 2.0 * pr.p - 2)) * (pr.w + std::max<double>(pr.q, 2.0 * pr.q - 2));
+    const double flops = 18.0 * positions * ((pr.c + 15) / 16 * 16) * ((pr.k + 31) / 32 * 32);
     best.direct = direct_ms > 0.f && std::max(static_cast<double>(direct_ms), flops / kSustainedFlops * 1e3) < best.ms;
+    best.ms /= accuracy_weight(best.algo);
     {
         std::lock_guard<std::mutex> lk(g_mu);
         if (g_cache.find(kk) == g_cache.end()) {
