@@ -298,7 +298,7 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
             info_grid = static_cast<unsigned>(
                 2 * std::min(direct_parts(direct, pr->in, pr->out, static_cast<int>(pr->n), parts), direct.max_pairs));
         }
-        info_threads = static_cast<unsigned>(direct_threads());
+        info_threads = static_cast<unsigned>(direct_threads(nhwc));
         info_smem = direct.ring.smem_bytes;
     } else if (algo == CONV2D_ALGO_2X3_FUSED) {
         ce = plan_fused2x3(fused, op, g, U);

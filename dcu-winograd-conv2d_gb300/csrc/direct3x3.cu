@@ -61,7 +61,10 @@ constexpr int kGroups = 3, kGroupWarps = 4;       // producer groups
 constexpr int kProdWarps = kGroups * kGroupWarps;
 constexpr int kEpiWarps = 4, kEpiHalves = kEpiWarps / 4;
 constexpr int kTmaWarp = kProdWarps + kEpiWarps, kMmaWarpD = kTmaWarp + 1;
-constexpr int kDirectThreads = 32 * (kMmaWarpD + 1);
+constexpr int kTables = 2, kTableWarp = kMmaWarpD + 1;   // channels-last: item tables, each filled by a warp of its own
+// more warps than 20 would leave fewer than 96 registers per thread
+template <bool NHWC>
+constexpr int kDirectThreads = 32 * (NHWC ? kTableWarp + kTables : kTableWarp);
 constexpr int kMaxRingA = 12, kMaxRingB = 12;
 constexpr int kHeader = 512;                      // barriers
 constexpr int kMaxSmem = 227 * 1024;
@@ -128,6 +131,39 @@ __device__ __forceinline__ DItem locate_direct(const DirectDesc* __restrict__ de
 constexpr int kGroupThreads = 32 * kGroupWarps;
 constexpr int kMaxPadBits = 32;      // pairs: positions per thread the pad mask covers
 
+// Channels-last: where the pixels of an item's window lie in the input, worked
+// out once per item by warps that do nothing else (items take the two tables in
+// turn; all warps share the first item).  Worked out by the threads of each
+// producer group, and kept in 12 of their registers, it stood in the way of
+// their loads: 32x256x56^2 -> 256 75.4 -> 69.9 us, 32x128x56^2 -> 128 28.0 -> 26.7,
+// 32x256x14^2 -> 256 12.3 -> 11.2.  (NCHW gains nothing, 16x64x128^2 -> 64 30.6 ->
+// 30.4 and 32x256x28^2 -> 256 23.1 -> 24.2: a table of pixel pairs and padding takes
+// a warp three times as long.)
+struct ItemTable {
+    const uint16_t* xi;   // image of the window's first position
+    int chunks, win, channels;
+    // then the element offset of each position from xi, or -1; whole blocks of 128
+};
+__host__ __device__ __forceinline__ int table_bytes(int win) {
+    return static_cast<int>(sizeof(ItemTable)) + 4 * ((win + 127) / 128 * 128);
+}
+// longest window that a stage of a_bytes holds
+__host__ __device__ __forceinline__ int max_window(int a_bytes) { return a_bytes / 32; }
+
+// by `threads` threads
+__device__ __forceinline__ void build_table(const DirectDesc& d, const DItem& it, uint32_t rank, ItemTable* tab, int tid,
+                                            int threads) {
+    const int z0 = d.pos0 + (2 * it.tile + static_cast<int>(rank)) * d.cta_rows;
+    const int n0 = min(static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z0))), d.n - 1), win = d.win;
+    if (tid == 0) {
+        tab->xi = static_cast<const uint16_t*>(d.x) + static_cast<long long>(n0) * d.c * d.h * d.w;
+        tab->chunks = d.c_chunks;
+        tab->win = win;
+        tab->channels = d.c;
+    }
+    for (int p = tid; p < (win + 127) / 128 * 128; p += threads) reinterpret_cast<int*>(tab + 1)[p] = p < win ? pixel_offset<true>(d, z0 + p, n0) : -1;
+}
+
 struct Step {
     uint32_t r[16];
     int p;             // pairs, single: position of the first granule; NHWC: of the block's first
@@ -152,13 +188,19 @@ struct Producer {
     int pairs;
     uint32_t plane;
     const uint16_t* xi;
-    // the item's first blocks: element offset from xi (-1: nothing to load) and
-    // position; NHWC: the first positions, 32 apart
-    static constexpr int kKeep = NHWC ? 12 : 4;
+    // the item's first blocks: element offset from xi (-1: nothing to load) and position
+    static constexpr int kKeep = 4;
     int off[kKeep];
     uint32_t pos2[2];   // positions of blocks 0, 1 and 2, 3 as 16-bit halves (-1 as 0xffff)
     uint32_t pads;
-    int far_n, far_ij, wn, wi, wj;   // NHWC: image, padded row and column of the first position past the kept ones; walk()
+    // NHWC: the tables, the item of this CTA and its table
+    unsigned char* tables;
+    int table_size, k;
+    const int* table;
+    uint64_t *tabfull, *tabempty;
+    volatile int* abort_flag;
+    DevErr* err;
+    bool failed;
 
     // pairs: pair number gt + 128 i of the window, decoded from scratch (blocks past kKeep)
     __device__ __forceinline__ void locate_pair(const DirectDesc& d, int i, int& o, int& p) const {
@@ -181,16 +223,7 @@ struct Producer {
     }
 
     __device__ __forceinline__ void decode(const DirectDesc& d) {
-        if constexpr (NHWC) {
-#pragma unroll
-            for (int i = 0; i < kKeep; ++i) off[i] = pixel_offset<true>(d, z0 + i * 32 + (gt >> 2), n0);
-            if (win > 32 * kKeep) {
-                const int z = z0 + 32 * kKeep + (gt >> 2);
-                far_n = static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z)));
-                const int rem = z - far_n * d.img, i = static_cast<int>(fast_div(d.fd_pw, static_cast<uint32_t>(rem)));
-                far_ij = (i << 16) | (rem - i * d.pw);
-            }
-        } else if (pairs) {
+        if (pairs) {
             // pairs 128 apart: a step of qy rows and rx columns
             const int hw = d.h * d.w, w = d.w, h = d.h, chw = d.c * hw;
             const int g = d_first(d) + 2 * gt;
@@ -233,22 +266,6 @@ struct Producer {
         }
     }
 
-    // NHWC: the pixel offset of the next position past the kept blocks, 32 on
-    // from the one before (`restart`: of the first)
-    __device__ __forceinline__ int walk(bool restart) {
-        const DirectDesc& d = descs[pi];
-        if (restart) wn = far_n, wi = far_ij >> 16, wj = far_ij & 0xffff;
-        const int y = wi - d.pad_h, x = wj - d.pad_w;
-        const bool in = wn < d.n && static_cast<unsigned>(y) < static_cast<unsigned>(d.h) &&
-                        static_cast<unsigned>(x) < static_cast<unsigned>(d.w);
-        const int o = in ? ((wn - n0) * d.h * d.w + y * d.w + x) * d.c : -1;
-        wj += d.walk_j;
-        wi += d.walk_i;
-        if (wj >= d.pw) wj -= d.pw, ++wi;
-        while (wi >= d.ph) wi -= d.ph, ++wn;
-        return o;
-    }
-
     // the current item's chunks, or pairs of them
     __device__ __forceinline__ int units() const { return NHWC ? (chunks + 1) / 2 : chunks; }
 
@@ -263,15 +280,35 @@ struct Producer {
     // moves to the first step in the items that follow; false when there is none
     __device__ __forceinline__ bool next_item() {
         while (c >= units()) {
+            if (NHWC && k >= 0) {   // its table is read
+                __syncwarp();
+                if ((gt & 31) == 0) mbar_arrive(&tabempty[k % kTables]);
+            }
             gu0 += units();
             gc0 += chunks;
             chunks = 0;
             t += step;
             if (t >= total_items) return false;
+            if constexpr (NHWC) {
+                ++k;
+                if (!mbar_wait(&tabfull[k % kTables], (k / kTables) & 1, abort_flag, err, ERR_SITE_FULL)) {
+                    failed = true;
+                    return false;
+                }
+                const ItemTable& tab = *reinterpret_cast<const ItemTable*>(tables + (k % kTables) * table_size);
+                chunks = tab.chunks;
+                c = (grp - gu0 % kGroups + kGroups) % kGroups;
+                table = reinterpret_cast<const int*>(&tab + 1);
+                xi = tab.xi;
+                win = tab.win;
+                channels = tab.channels;
+                blocks = (win + 127) / 128;
+                continue;
+            }
             const DItem it = locate_direct(descs, ndesc, t, pi);
             const DirectDesc& d = descs[pi];
             chunks = d.c_chunks;
-            c = (grp - (NHWC ? gu0 : gc0) % kGroups + kGroups) % kGroups;
+            c = (grp - gc0 % kGroups + kGroups) % kGroups;
             if (c >= units()) continue;
             z0 = d.pos0 + (2 * it.tile + static_cast<int>(rank)) * d.cta_rows;
             n0 = min(static_cast<int>(fast_div(d.fd_img, static_cast<uint32_t>(z0))), d.n - 1);
@@ -281,8 +318,7 @@ struct Producer {
             plane = static_cast<uint32_t>(d.h * d.w);
             xi = static_cast<const uint16_t*>(d.x) + static_cast<long long>(n0) * channels * plane;
             // blocks that reach into the window, for this warp's part of them
-            blocks = NHWC ? (win + 127) / 128
-                          : max(((pairs ? win / 2 + 1 : win) - (gt & ~31) + kGroupThreads - 1) / kGroupThreads, 1);
+            blocks = max(((pairs ? win / 2 + 1 : win) - (gt & ~31) + kGroupThreads - 1) / kGroupThreads, 1);
             pads = 0;
             decode(d);
         }
@@ -299,8 +335,7 @@ struct Producer {
             s.p = blk * 128 + (gt >> 2);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                int o = blk == 0 ? off[k] : blk == 1 ? off[4 + k] : off[8 + k];
-                if (blk > 2) o = walk(blk == 3 && k == 0);
+                int o = table[s.p + 32 * k];
                 if (o < 0 || !cin) {
                     o = 0;
                     s.flags |= 16u << k;
@@ -471,13 +506,17 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
     uint64_t* bempty = bfull + kMaxRingB;          // MMAs done with the filter rows
     uint64_t* tfull = bempty + kMaxRingB;          // [2] accumulator ready
     uint64_t* tempty = tfull + 2;                  // [2] even CTA: accumulator drained in both CTAs
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty + 2);
+    uint64_t* tabfull = tempty + 2;                // item table written
+    uint64_t* tabempty = tabfull + kTables;        // read by every producer warp
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tabempty + kTables);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int first = blockIdx.x >> 1, step = gridDim.x >> 1;
     const int na = ring.na, nb = ring.nb;
+    unsigned char* tables = reinterpret_cast<unsigned char*>(bars) + kHeader;
+    const int table_size = table_bytes(max_window(ring.a_bytes));
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxRingA; ++i) {
@@ -492,11 +531,21 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
             mbar_init(&tfull[i], 1);
             mbar_init(&tempty[i], 2 * kEpiWarps);
         }
+        for (int i = 0; i < kTables; ++i) {
+            mbar_init(&tabfull[i], 1);
+            mbar_init(&tabempty[i], kProdWarps);
+        }
         *abort_flag = 0;
         fence_barrier_init();
     }
     if constexpr (!LATE) pdl_wait();
     if (warp == kMmaWarpD) tmem_alloc_pair(tmem_slot, 512);
+    if (NHWC && first < total_items) {
+        int pi = 0;
+        const DItem it = locate_direct(descs, ndesc, first, pi);
+        build_table(descs[pi], it, rank, reinterpret_cast<ItemTable*>(tables), static_cast<int>(threadIdx.x),
+                    kDirectThreads<NHWC>);
+    }
     tc_fence_before();
     __syncthreads();
     cluster_sync();
@@ -517,6 +566,14 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
         pr.grp = warp / kGroupWarps;
         pr.gt = static_cast<int>(threadIdx.x) - pr.grp * kGroupThreads;
         pr.rank = rank;
+        pr.tables = tables;
+        pr.table_size = table_size;
+        pr.k = -1;
+        pr.tabfull = tabfull;
+        pr.tabempty = tabempty;
+        pr.abort_flag = abort_flag;
+        pr.err = err;
+        pr.failed = false;
         pr.t = first - step;
         pr.pi = pr.c = pr.chunks = pr.gc0 = pr.gu0 = pr.blk = pr.blocks = 0;
         int sa = pr.grp;             // this group's next window stage and its phase
@@ -570,7 +627,7 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
             }
         }
         // the last commits on this CTA's window barriers must land before it exits
-        if (ok && warp == 0 && lane == 0)
+        if (ok && !pr.failed && warp == 0 && lane == 0)
             for (int k = max(0, pr.gc0 - na); k < pr.gc0; ++k)
                 if (!mbar_wait(&aempty[k % na], (k / na) & 1, abort_flag, err, ERR_SITE_DRAIN)) break;
     } else if (warp == kTmaWarp) {
@@ -659,6 +716,20 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
                 if (ok && elected) tc_commit_pair(&tfull[acc]);
                 __syncwarp();
             }
+        }
+    } else if (NHWC && warp >= kTableWarp) {
+        // ---- item tables; the first is written
+        int pi = 0, k = warp - kTableWarp;
+        if (k == 0) {
+            if (lane == 0) mbar_arrive(&tabfull[0]);
+            k = kTables;
+        }
+        for (int t = first + k * step; t < total_items; t += kTables * step, k += kTables) {
+            const DItem it = locate_direct(descs, ndesc, t, pi);
+            if (!mbar_wait_warp(&tabempty[k % kTables], ((k / kTables) & 1) ^ 1, abort_flag, err, ERR_SITE_EMPTY)) break;
+            build_table(descs[pi], it, rank, reinterpret_cast<ItemTable*>(tables + (k % kTables) * table_size), lane, 32);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tabfull[k % kTables]);
         }
     } else {
         // ---- epilogue: kEpiHalves warps per TMEM lane quarter, taking blocks
@@ -755,13 +826,13 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
 }
 
 template <bool NHWC, bool BF16>
-__global__ void __launch_bounds__(kDirectThreads, 1)
+__global__ void __launch_bounds__(kDirectThreads<NHWC>, 1)
     direct3x3_kernel(const __grid_constant__ DirectParts parts, const __grid_constant__ DirectRing ring, DevErr* err) {
     direct_body<NHWC, BF16, true>(parts.d, parts.count, parts.items, ring, err);
 }
 
 // Many problems (fp16 NCHW) as one work queue; descs device-resident, sorted by item_begin.
-__global__ void __launch_bounds__(kDirectThreads, 1)
+__global__ void __launch_bounds__(kDirectThreads<false>, 1)
     direct3x3_grouped(const DirectDesc* __restrict__ descs, int ndesc, int items, const __grid_constant__ DirectRing ring,
                       DevErr* err) {
     direct_body<false, false, false>(descs, ndesc, items, ring, err);
@@ -818,8 +889,8 @@ int b_stage_bytes(int bn) { return kTaps9 * bn * 16; }
 
 // Ring depths for one window size and channel tile; false when two stages of
 // each do not fit.
-bool size_ring(DirectRing& r, int a_bytes, int b_bytes) {
-    const int room = kMaxSmem - 1024 - kHeader;
+bool size_ring(DirectRing& r, int a_bytes, int b_bytes, bool nhwc) {
+    const int fixed = 1024 + kHeader + (nhwc ? kTables * table_bytes(max_window(a_bytes)) : 0), room = kMaxSmem - fixed;
     r.a_bytes = a_bytes;
     r.b_bytes = b_bytes;
     // as many chunks ahead on both sides; what is left over goes to the windows
@@ -828,7 +899,7 @@ bool size_ring(DirectRing& r, int a_bytes, int b_bytes) {
         if (na >= 2) {
             r.nb = nb;
             r.na = na;
-            r.smem_bytes = std::max(kMinSmem, nb * b_bytes + na * a_bytes + kHeader + 1024);
+            r.smem_bytes = std::max(kMinSmem, nb * b_bytes + na * a_bytes + fixed);
             return true;
         }
     }
@@ -847,9 +918,9 @@ double item_cycles(int bn, int mb, int pw, int chunks) {
 }
 
 template <auto Kernel, class... Args>
-cudaError_t launch_cluster(int pairs, int smem, cudaStream_t s, const Args&... args) {
+cudaError_t launch_cluster(int pairs, int threads, int smem, cudaStream_t s, const Args&... args) {
     const cudaError_t e = allow_smem<Kernel>(kMaxSmem);
-    return e == cudaSuccess ? launch_pairs(Kernel, pairs, kDirectThreads, smem, s, args...) : e;
+    return e == cudaSuccess ? launch_pairs(Kernel, pairs, threads, smem, s, args...) : e;
 }
 
 // CTA pairs that run at once (one CTA per SM; a cluster stays within a GPC)
@@ -858,7 +929,7 @@ int max_pairs(int num_sms) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem) != cudaSuccess) return num_sms / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (num_sms / 2));
-    cfg.blockDim = dim3(kDirectThreads);
+    cfg.blockDim = dim3(kDirectThreads<false>);
     cfg.dynamicSmemBytes = kMaxSmem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -877,7 +948,7 @@ int max_pairs(int num_sms) {
 
 }  // namespace
 
-int direct_threads() { return kDirectThreads; }
+int direct_threads(bool nhwc) { return nhwc ? kDirectThreads<true> : kDirectThreads<false>; }
 
 long long direct_filter_bytes(int K, int C) {
     return static_cast<long long>(kTaps9) * ((C + 7) / 8 * 8) * ((K + 7) / 8 * 8) * 2;
@@ -894,11 +965,11 @@ struct Split {
     double cycles = 0;
 };
 
-bool tile_fits(int bn, int mb, int pw, DirectRing* ring) {
+bool tile_fits(int bn, int mb, int pw, DirectRing* ring, bool nhwc) {
     if (bn * mb > 256) return false;
     const int a = window_bytes(window_of(mb, pw));
     DirectRing r;
-    if (!size_ring(r, a, b_stage_bytes(bn))) return false;
+    if (!size_ring(r, a, b_stage_bytes(bn), nhwc)) return false;
     if (ring) *ring = r;
     return true;
 }
@@ -906,11 +977,11 @@ bool tile_fits(int bn, int mb, int pw, DirectRing* ring) {
 // Cycles of every item shape that fits (0: does not), by log2 mb and bn / 32 - 1.
 struct TileCosts {
     double one[4][8];
-    TileCosts(int pw, int chunks, int only_bn, int only_mb) {
+    TileCosts(int pw, int chunks, int only_bn, int only_mb, bool nhwc) {
         for (int i = 0; i < 4; ++i)
             for (int j = 0; j < 8; ++j) {
                 const int mb = 1 << i, bn = 32 * (j + 1);
-                const bool out = (only_mb && mb != only_mb) || (only_bn && bn != only_bn) || !tile_fits(bn, mb, pw, nullptr);
+                const bool out = (only_mb && mb != only_mb) || (only_bn && bn != only_bn) || !tile_fits(bn, mb, pw, nullptr, nhwc);
                 one[i][j] = out ? 0 : item_cycles(bn, mb, pw, chunks);
             }
     }
@@ -997,10 +1068,6 @@ cudaError_t describe_direct(DirectDesc& d, const Geom& g, bool nhwc) {
     d.step_x = (2 * kGroupThreads) % g.w;
     d.pad_step_i = kGroupThreads / d.pw;
     d.pad_step_j = kGroupThreads % d.pw;
-    d.walk_i = 32 / d.pw;
-    d.walk_j = 32 % d.pw;
-    // rows and columns of positions in 16 bits each
-    if (nhwc && (d.ph > 0x7fff || d.pw > 0xffff)) return cudaErrorNotSupported;
     d.fd_img = make_fastdiv(static_cast<uint32_t>(d.img));
     d.fd_pw = make_fastdiv(static_cast<uint32_t>(d.pw));
     d.fd_hw = make_fastdiv(static_cast<uint32_t>(static_cast<long long>(g.h) * g.w));
@@ -1031,7 +1098,7 @@ int direct_max_pairs(int num_sms) {
 
 bool direct_supported(const Geom& g, bool nhwc) {
     DirectDesc d;
-    return describe_direct(d, g, nhwc) == cudaSuccess && tile_fits(32, 1, d.pw, nullptr);
+    return describe_direct(d, g, nhwc) == cudaSuccess && tile_fits(32, 1, d.pw, nullptr, nhwc);
 }
 
 cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, const void* U, int tile, int num_sms) {
@@ -1039,9 +1106,9 @@ cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, con
     if (cudaError_t e = describe_direct(d, g, nhwc); e != cudaSuccess) return e;
     dp.max_pairs = direct_max_pairs(num_sms);
     const int bn = tile & 0x1ff, mb = tile >> 9;
-    const TileCosts any(d.pw, d.c_chunks, 0, 0), asked(d.pw, d.c_chunks, bn, mb);
+    const TileCosts any(d.pw, d.c_chunks, 0, 0, nhwc), asked(d.pw, d.c_chunks, bn, mb, nhwc);
     const Split s = best_split(positions(d, g.n), g.k, dp.max_pairs, asked, &any);
-    if (s.bn == 0 || !tile_fits(s.bn, s.mb, d.pw, &dp.ring)) return cudaErrorNotSupported;
+    if (s.bn == 0 || !tile_fits(s.bn, s.mb, d.pw, &dp.ring, nhwc)) return cudaErrorNotSupported;
     set_tile(d, s.bn, s.mb);
     dp.main = d;
     dp.tail = d;
@@ -1051,7 +1118,7 @@ cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, con
         DirectRing r;
         // one ring serves both parts: the larger stages
         const int a = std::max(window_bytes(d.win), window_bytes(dp.tail.win));
-        if (size_ring(r, a, std::max(b_stage_bytes(d.bn), b_stage_bytes(dp.tail.bn))))
+        if (size_ring(r, a, std::max(b_stage_bytes(d.bn), b_stage_bytes(dp.tail.bn)), nhwc))
             dp.ring = r;
         else
             dp.has_tail = false;
@@ -1116,7 +1183,7 @@ cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDe
     // stages small enough for four of each
     auto fits = [](int bn, int mb, int pw) {
         DirectRing r;
-        return tile_fits(bn, mb, pw, &r) && (mb == 1 || r.a_bytes <= 18 * 1024);
+        return tile_fits(bn, mb, pw, &r, false) && (mb == 1 || r.a_bytes <= 18 * 1024);
     };
     auto choose = [&](Pick& k, double longest) {
         const long long pos = positions(k.d, k.d.n);
@@ -1155,7 +1222,7 @@ cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDe
         a = std::max(a, window_bytes(k.d.win));
         b = std::max(b, b_stage_bytes(k.d.bn));
     }
-    if (!size_ring(ring, a, b)) return cudaErrorNotSupported;
+    if (!size_ring(ring, a, b, false)) return cudaErrorNotSupported;
     std::stable_sort(picks.begin(), picks.end(), [](const Pick& x, const Pick& y) { return x.one > y.one; });
     long long begin = 0;
     for (int i = 0; i < n; ++i) {
@@ -1174,17 +1241,19 @@ cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDe
 
 cudaError_t launch_direct_grouped(const DirectDesc* descs, int ndesc, int items, const DirectRing& ring, int pairs, DevErr* err,
                                   cudaStream_t stream) {
-    return launch_cluster<direct3x3_grouped>(std::min(items, pairs), ring.smem_bytes, stream, descs, ndesc, items, ring, err);
+    return launch_cluster<direct3x3_grouped>(std::min(items, pairs), kDirectThreads<false>, ring.smem_bytes, stream, descs, ndesc,
+                                             items, ring, err);
 }
 
 cudaError_t launch_direct(const DirectPlan& dp, const void* x, void* y, int n_images, DevErr* err, cudaStream_t stream) {
     DirectParts p;
     const int pairs = std::min(direct_parts(dp, x, y, n_images, p), dp.max_pairs);
+    const int threads = direct_threads(dp.nhwc), smem = dp.ring.smem_bytes;
     if (dp.nhwc)
-        return dp.bf16 ? launch_cluster<direct3x3_kernel<true, true>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
-                       : launch_cluster<direct3x3_kernel<true, false>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
-    return dp.bf16 ? launch_cluster<direct3x3_kernel<false, true>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err)
-                   : launch_cluster<direct3x3_kernel<false, false>>(pairs, dp.ring.smem_bytes, stream, p, dp.ring, err);
+        return dp.bf16 ? launch_cluster<direct3x3_kernel<true, true>>(pairs, threads, smem, stream, p, dp.ring, err)
+                       : launch_cluster<direct3x3_kernel<true, false>>(pairs, threads, smem, stream, p, dp.ring, err);
+    return dp.bf16 ? launch_cluster<direct3x3_kernel<false, true>>(pairs, threads, smem, stream, p, dp.ring, err)
+                   : launch_cluster<direct3x3_kernel<false, false>>(pairs, threads, smem, stream, p, dp.ring, err);
 }
 
 }  // namespace wg

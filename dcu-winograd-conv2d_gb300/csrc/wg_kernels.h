@@ -324,7 +324,6 @@ struct alignas(64) DirectDesc {
     int pairs;           // NCHW: input read as pixel pairs
     int step_y, step_x;          // 256 pixels as rows and columns of the input
     int pad_step_i, pad_step_j;  // 128 positions as rows and columns of positions
-    int walk_i, walk_j;          // 32 positions likewise
     int pos0;            // first position of item_begin's item
     int item_begin, items;
     FastDiv fd_nb, fd_img, fd_pw, fd_hw, fd_w;
@@ -376,7 +375,7 @@ cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDe
 cudaError_t launch_direct_grouped(const DirectDesc* descs, int ndesc, int items, const DirectRing& ring, int pairs, DevErr* err,
                                   cudaStream_t stream);
 long long direct_filter_bytes(int K, int C);
-int direct_threads();
+int direct_threads(bool nhwc);
 // U9[tap][Cp/8][Kp][8] from KCRS weights (16-bit values copied as they are)
 cudaError_t launch_direct_filter(const void* weight, void* U, int K, int C, cudaStream_t stream);
 // and back

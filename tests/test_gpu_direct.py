@@ -75,6 +75,15 @@ def test_channels_last(wg, shape, pad):
     _run(wg, *shape, pad, nhwc=True)
 
 
+@pytest.mark.parametrize("shape,tile", [((200, 16, 28, 28, 256), 0), ((300, 24, 14, 14, 40), 32 + 512), ((5, 40, 90, 90, 64), 32 + 512),
+                                        ((64, 8, 30, 30, 32), 32 + 1024)])
+def test_channels_last_many_items(wg, shape, tile):
+    # 3 to 13 items per CTA pair: both item tables are filled again and again, by
+    # items of one chunk (fewer than the producer groups) to three
+    _run(wg, *shape, (1, 1), nhwc=True, bn=tile)
+    _run(wg, *shape, (1, 1), nhwc=True, bf16=True, bn=tile)
+
+
 @pytest.mark.parametrize("shape", [(1, 3, 8, 8, 5), (4, 72, 28, 28, 130)])
 def test_bf16(wg, shape):
     _run(wg, *shape, (1, 1), bf16=True)
