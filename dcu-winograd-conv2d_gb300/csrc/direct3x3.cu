@@ -1250,8 +1250,7 @@ cudaError_t launch_direct(const DirectPlan& dp, const void* x, void* y, int n_im
     const int pairs = std::min(direct_parts(dp, x, y, n_images, p), dp.max_pairs);
     const int threads = direct_threads(dp.nhwc), smem = dp.ring.smem_bytes;
     if (dp.nhwc)
-        return dp.bf16 ? launch_cluster<direct3x3_kernel<true, true>>(pairs, threads, smem, stream, p, dp.ring, err)
-                       : launch_cluster<direct3x3_kernel<true, false>>(pairs, threads, smem, stream, p, dp.ring, err);
+        return launch_cluster<direct3x3_kernel<true, false>>(pairs, threads, smem, stream, p, dp.ring, err);
     return dp.bf16 ? launch_cluster<direct3x3_kernel<false, true>>(pairs, threads, smem, stream, p, dp.ring, err)
                    : launch_cluster<direct3x3_kernel<false, false>>(pairs, threads, smem, stream, p, dp.ring, err);
 }

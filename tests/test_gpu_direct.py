@@ -81,7 +81,6 @@ def test_channels_last_many_items(wg, shape, tile):
     # 3 to 13 items per CTA pair: both item tables are filled again and again, by
     # items of one chunk (fewer than the producer groups) to three
     _run(wg, *shape, (1, 1), nhwc=True, bn=tile)
-    _run(wg, *shape, (1, 1), nhwc=True, bf16=True, bn=tile)
 
 
 @pytest.mark.parametrize("shape", [(1, 3, 8, 8, 5), (4, 72, 28, 28, 130)])
