@@ -35,10 +35,11 @@
 // same (the window is read nine times for few columns), so they take several
 // blocks of 128 positions per item, which share the filter rows and the
 // window's halo.  Measured, back to back with rotating buffers, against the
-// tuner's choice without this kernel: 32x256x56^2 -> 256 70 us (1,700 TFLOP/s;
-// 82 under the power cap) against 102; 32x256x28^2 -> 256 24.2 against 35;
-// 32x256x14^2 -> 256 13 against 18.7; 1x64x56^2 -> 64 6.8 against 9.5; bf16
-// 32x256x28^2 -> 256 23.8 against 52.7.
+// tuner's choice without this kernel: 32x256x56^2 -> 256 70 us (1,690 TFLOP/s;
+// 82 under the power cap) against 102; 32x256x28^2 -> 256 22.8 against 35;
+// 32x256x14^2 -> 256 11.6 against 18.7; 16x64x128^2 -> 64 30.7 against 36.6;
+// 1x64x56^2 -> 64 5.1 against 9.5; bf16 32x256x28^2 -> 256 22.9 against 52.8;
+// channels-last 32x128x56^2 -> 128 26.7 against 42.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

@@ -224,7 +224,7 @@ struct Server {
     // The direct kernel holds about 1,430 TFLOP/s of direct-convolution work
     // under the power cap whatever the channels; F(4x3), whose traffic per
     // product falls as they grow, passes it from about 512 x 512 channels on
-    // (32 x 28^2: 70.9 against 80 us; at 256 x 256 101.6 against 82.5 on 56^2).
+    // (32 x 28^2: 65.5 against 80 us; at 256 x 256 101 against 82 on 56^2).
     bool choose_direct(const Layer& L, unsigned n) const {
         if (cfg.algo != CONV2D_ALGO_AUTO || !L.U9) return false;
         if (std::min(L.c, L.k) >= 512 && L.h >= 14 && L.w >= 14) return false;

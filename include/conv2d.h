@@ -109,11 +109,12 @@ enum {
  * times the candidates (the reference's three algorithms and the row F(4x3)
  * kernel) on the device, reading the problem's input and weights and writing
  * a scratch output, and keeps the reference rule's pick unless another is
- * more than 3% faster; the choice is cached per shape (and in
- * WG_CONV2D_TUNE_FILE).  It also times the direct kernel, which calls run
- * where it is faster than that pick (conv2d_get_direct).  On GB300 the reference rule's fused F(2x3) pick is
- * several times slower than the alternatives for wide K (e.g. 392 against
- * 115 us on 32x256x56^2 -> 256).  algo = CONV2D_ALGO_REFERENCE, or
+ * more than 3% faster, times weighed by accuracy; the choice is cached per
+ * shape (and in WG_CONV2D_TUNE_FILE).  It also times the direct kernel, which
+ * calls run where it is faster than that pick (conv2d_get_direct).  On GB300
+ * the reference rule's fused F(2x3) pick is several times slower than the
+ * alternatives for wide K (e.g. 390 against 101 us for F(4x3) and 82 for the
+ * direct kernel on 32x256x56^2 -> 256).  algo = CONV2D_ALGO_REFERENCE, or
  * WG_CONV2D_ALGO=ref, applies the reference rule (src/conv2d.cpp:83-114)
  * exactly; conv2d_get_algo reports what was chosen. */
 typedef struct
