@@ -224,10 +224,15 @@ struct Server {
     // The direct kernel holds about 1,430 TFLOP/s of direct-convolution work
     // under the power cap whatever the channels; F(4x3), whose traffic per
     // product falls as they grow, passes it from about 512 x 512 channels on
-    // (32 x 28^2: 65.5 against 80 us; at 256 x 256 101 against 82 on 56^2).
+    // (32 x 28^2: 65.5 against 80.6 us; at 256 x 256 101 against 82 on 56^2),
+    // unless its 4 x 4 tiles reach past the output (64 x 512 x 14^2: 59.2 against
+    // 44.7; 16 x 30^2 53.7 against 48.9; 32 x 20^2 42.0 against 44.8) or the request
+    // is small (1 x 56^2: 18.9 against 17.2; 8 x 28^2 26.9 against 28.5).
     bool choose_direct(const Layer& L, unsigned n) const {
         if (cfg.algo != CONV2D_ALGO_AUTO || !L.U9) return false;
-        if (std::min(L.c, L.k) >= 512 && L.h >= 14 && L.w >= 14) return false;
+        const long long oh = L.h + 2LL * L.p - 2, ow = L.w + 2LL * L.q - 2;
+        const long long tiled = (oh + 3) / 4 * ((ow + 3) / 4) * 16;
+        if (std::min(L.c, L.k) >= 512 && L.h >= 14 && L.w >= 14 && 20 * tiled <= 21 * oh * ow && n * oh * ow >= 4096) return false;
         return direct_supported(make_geom(static_cast<int>(n), L.c, L.h, L.w, L.k, L.p, L.q, 2), false);
     }
 

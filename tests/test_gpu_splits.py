@@ -81,3 +81,22 @@ def test_host_chunks_around_the_threshold(wg, algo, n):
         hout.zero_()
         op.host(hin.data_ptr(), hout.data_ptr(), s)
         assert torch.equal(hout.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("n,h,algo", [(40, 13, 5), (21, 14, 5), (10, 20, 5), (11, 20, 0), (4, 29, 5), (5, 28, 5), (6, 28, 0)])
+def test_server_picks_per_request(wg, n, h, algo):
+    """512 -> 512 channels: F(4x3) where its tiles fit the output and there are
+    4,096 output pixels, else direct; the bits are those of a call by name."""
+    c = k = 512
+    g = torch.Generator().manual_seed(n + h)
+    x = (torch.rand((n, c, h, h), generator=g) * 2 - 1).half().cuda()
+    f = (torch.randn((k, c, 3, 3), generator=g) / 68).half().cuda()
+    want, op = wg.conv2d_torch(x, f, 1, 1, opts_for(wg, algo))
+    assert op.algo == algo
+    y = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    server = wg.Server(hbm_budget_bytes=1 << 30)
+    layer = server.add_layer(c, k, h, h, f.data_ptr())
+    server.replay([layer], [n], [0.0], [x.data_ptr()], [y.data_ptr()])
+    torch.cuda.synchronize()
+    assert torch.equal(y.view(torch.int16), want.view(torch.int16))
