@@ -27,6 +27,8 @@
 // they run in stream order they share one workspace region.  Completion is
 // observed the same way in both modes (an event per request or batch, polled
 // by the scheduler thread).
+#include <sys/prctl.h>
+
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -435,6 +437,11 @@ struct Server {
 
     void loop() {
         cudaSetDevice(device);
+        // the sleeps below are of 5 us; the default timer slack makes them 55, which
+        // every completion, and a request that arrives just after a batch was
+        // launched, then wait for (13 requests on three layers in one burst: 173 us,
+        // now 91; 24 on 16 layers 488 -> 466)
+        prctl(PR_SET_TIMERSLACK, 1ul, 0ul, 0ul, 0ul);
         while (true) {
             std::unique_lock<std::mutex> lk(mu);
             // completions
