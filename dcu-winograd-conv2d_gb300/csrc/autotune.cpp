@@ -97,8 +97,9 @@ void append_file_locked(const Key& kk, const Choice& ch) {
     std::fclose(fp);
 }
 
-// Device time of one call of a candidate plan (best of 3 after a warm-up), or
-// a negative value when the candidate cannot be planned.
+// Device time of one call of a candidate plan (best of 8 after a warm-up; with
+// the best of 3 a choice now and then took a GEMM tile a fifth slower), or a
+// negative value when the candidate cannot be planned.
 float time_candidate(const problem_t& pr, conv2d_options_t opt, int algo, int bn, void* scratch_out,
                      cudaStream_t s) {
     problem_t p = pr;
@@ -112,7 +113,7 @@ float time_candidate(const problem_t& pr, conv2d_options_t opt, int algo, int bn
     cudaEventCreate(&a);
     cudaEventCreate(&b);
     float best = -1.f;
-    for (int rep = 0; rep < 3; ++rep) {
+    for (int rep = 0; rep < 8; ++rep) {
         cudaEventRecord(a, s);
         if (pl.run(s) != CONV2D_OK) break;
         cudaEventRecord(b, s);
