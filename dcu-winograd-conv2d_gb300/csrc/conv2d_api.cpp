@@ -447,6 +447,7 @@ int Plan::run(cudaStream_t s) {
 // whether copy engines or SM loads and stores move the bytes).  Chunks hold at
 // least 6 MB of copies (two chunks from 4 MB in all: 16x128x28^2 -> 128, 6.4 MB,
 // 60 us in two, 66 in one, 77 in four; 8x64x28^2 -> 64, 1.6 MB, 39 in two, 33 in
+// one; but 16x10x12^2 -> 960, 4.4 MB, nearly all of them out, 57 in two, 50 in
 // one) and there are at most 8 of them: on the 32 x 256 x 56^2
 // layer (103 MB of copies) 8 chunks took 402-411 us per call, 6 took 420,
 // 4 took 439, 12 and 16 took 450; chunks ramping from 1 image up to 4 and
@@ -481,13 +482,15 @@ int host_sizes_env(int n, int* sizes) {
     return (sum == n && distinct <= Plan::kMaxHostPlans) ? cnt : 0;
 }
 
-int host_schedule(int n, long long img_copy_bytes, int* sizes) {
+int host_schedule(int n, long long img_in_bytes, long long img_out_bytes, int* sizes) {
     if (const int cnt = host_sizes_env(n, sizes)) return cnt;
-    const long long total = static_cast<long long>(n) * img_copy_bytes;
+    const long long in = n * img_in_bytes, out = n * img_out_bytes, total = in + out;
     long long max_chunks = 8;
     if (const char* e = std::getenv("WG_CONV2D_HOST_CHUNKS")) max_chunks = std::max(1, std::min(std::atoi(e), Plan::kMaxHostChunks));
-    // two from 4 MB on: there the overlap outweighs the events between the streams
-    const long long wanted = std::max(total / (6LL << 20), total >= (4LL << 20) ? 2LL : 1LL);
+    // two from 4 MB on, where the copies of both directions are of a size: there
+    // their overlap outweighs the events between the streams
+    const bool two = total >= (4LL << 20) && 3 * std::min(in, out) >= total;
+    const long long wanted = std::max(total / (6LL << 20), two ? 2LL : 1LL);
     const int chunks = static_cast<int>(std::max(1LL, std::min<long long>({static_cast<long long>(n), max_chunks, wanted})));
     const int per = (n + chunks - 1) / chunks;
     int cnt = 0;
@@ -595,7 +598,7 @@ int Plan::enqueue_host(const void* const* host_in, void* const* host_out, int st
     const long long in_img_b = static_cast<long long>(g.c) * g.h * g.w * 2;
     const long long out_img_b = static_cast<long long>(g.k) * g.oh * g.ow * 2;
     int sizes[kMaxHostChunks];
-    const int nch = host_schedule(n, in_img_b + out_img_b, sizes);
+    const int nch = host_schedule(n, in_img_b, out_img_b, sizes);
     // the non-fused workspace holds chunk_n images: a host chunk runs as
     // ranges of at most that many
     const int cap = single_kernel() ? n : chunk_n;

@@ -63,11 +63,12 @@ def test_input_transform_blocks(wg, monkeypatch, n, c, h, w):
 
 
 @pytest.mark.parametrize("algo", [0, 1, 5])
-@pytest.mark.parametrize("n", [1, 10, 11, 13])
-def test_host_chunks_around_the_threshold(wg, algo, n):
+@pytest.mark.parametrize("n,k", [(1, 64), (10, 64), (11, 64), (13, 64), (13, 136)])
+def test_host_chunks_around_the_threshold(wg, algo, n, k):
     """409,600 bytes of copies per image: one chunk below 4 MB (10 images), two
-    from there on; the result of each is that of the device call, bit for bit."""
-    c, h, k = 64, 40, 64
+    from there on unless one direction (k = 136: the output) has more than two
+    thirds; the result of each is that of the device call, bit for bit."""
+    c, h = 64, 40
     x, wt = O.uniform_inputs(n, n, c, h, h, k)
     xt, wtt = torch.from_numpy(x).cuda(), torch.from_numpy(wt).cuda()
     y = torch.empty((n, k, h, h), dtype=torch.float16, device="cuda")
