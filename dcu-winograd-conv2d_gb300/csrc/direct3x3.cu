@@ -888,8 +888,17 @@ int window_bytes(int win) { return (2 * granule_bytes(win) + 127) / 128 * 128 + 
 
 int b_stage_bytes(int bn) { return kTaps9 * bn * 16; }
 
-// Ring depths for one window size and channel tile; false when two stages of
-// each do not fit.
+// Fewest window stages.  A producer group waits for the release of a stage by
+// the parity of its use, which tells one use from the next but not from the one
+// after: when the group comes to its next chunk, the use before last of that
+// chunk's stage has to be over.  What it knows to be over is the use that freed
+// the stage of its last chunk, na chunks before that one.  So na may not be less
+// than the chunks it moves on by: three, or channels-last, by pairs of chunks,
+// five from the second of one pair to the first of the next.
+constexpr int least_stages(bool nhwc) { return nhwc ? 2 * kGroups - 1 : kGroups; }
+
+// Ring depths for one window size and channel tile; false when the fewest
+// window stages and two of the filter do not fit.
 bool size_ring(DirectRing& r, int a_bytes, int b_bytes, bool nhwc) {
     const int fixed = 1024 + kHeader + (nhwc ? kTables * table_bytes(max_window(a_bytes)) : 0), room = kMaxSmem - fixed;
     r.a_bytes = a_bytes;
@@ -897,7 +906,7 @@ bool size_ring(DirectRing& r, int a_bytes, int b_bytes, bool nhwc) {
     // as many chunks ahead on both sides; what is left over goes to the windows
     for (int nb = std::min(kMaxRingB, room / (a_bytes + b_bytes)); nb >= 2; --nb) {
         const int na = std::min(kMaxRingA, (room - nb * b_bytes) / a_bytes);
-        if (na >= 2) {
+        if (na >= least_stages(nhwc)) {
             r.nb = nb;
             r.na = na;
             r.smem_bytes = std::max(kMinSmem, nb * b_bytes + na * a_bytes + fixed);

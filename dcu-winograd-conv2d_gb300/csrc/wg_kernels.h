@@ -352,7 +352,7 @@ struct DirectPlan {
 // tile: output channels per item (a multiple of 32 up to 256) + 512 x blocks
 // of 128 positions per CTA (1, 2, 4 or 8, with at most 256 channels x blocks);
 // either part 0 = chosen from the sizes.  cudaErrorNotSupported when the
-// window of one CTA does not fit in shared memory (rows beyond about 1,600
+// window of one CTA does not fit in shared memory (rows beyond about 1,080
 // columns), for sizes beyond 32-bit positions, and for channels-last C not a
 // multiple of 8.  U may be null (a size probe).
 cudaError_t plan_direct(DirectPlan& dp, const Geom& g, bool nhwc, bool bf16, const void* U, int tile, int num_sms);

@@ -83,6 +83,15 @@ def test_channels_last_many_items(wg, shape, tile):
     _run(wg, *shape, (1, 1), nhwc=True, bn=tile)
 
 
+@pytest.mark.parametrize("shape,nhwc,tile", [
+    ((2, 64, 6, 1000, 40), False, 0), ((1, 80, 4, 1080, 40), False, 0), ((12, 96, 40, 40, 256), True, 256 + 512),
+    ((19, 296, 32, 32, 280), True, 0), ((5, 312, 56, 56, 720), True, 0), ((1, 80, 12, 400, 70), True, 0),
+    ((8, 200, 64, 64, 64), True, 64 + 512 * 2)])
+def test_fewest_stages(wg, shape, nhwc, tile):
+    # windows or filter tiles that leave the rings little more than their fewest stages
+    _run(wg, *shape, (1, 1), nhwc=nhwc, bn=tile)
+
+
 @pytest.mark.parametrize("shape", [(1, 3, 8, 8, 5), (4, 72, 28, 28, 130)])
 def test_bf16(wg, shape):
     _run(wg, *shape, (1, 1), bf16=True)
