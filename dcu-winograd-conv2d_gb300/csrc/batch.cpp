@@ -8,7 +8,8 @@
 //     per (channel tile, M type) whose work queue holds every (problem,
 //     element, tile block, channel block) item, the output transforms in one
 //     launch per family, the problems that run the direct kernel in one
-//     launch over all their items -- captured once into a CUDA graph and
+//     launch over all their items (one more for rows so wide that their windows
+//     and the others' filter tiles do not fit one ring) -- captured once into a CUDA graph and
 //     replayed; or
 //   * per call: each problem's own launches, one problem after another
 //     (the comparison the grouped run is measured against).
@@ -65,11 +66,11 @@ struct Batch {
     std::vector<InGroup> in_groups;
     std::vector<GemmGroup> gemm_groups;
     std::vector<OutGroup> out_groups;
-    // problems that run the direct kernel: one launch over all of them
+    // problems that run the direct kernel: one launch per queue of them
     struct DirectGroup {
         const DirectDesc* descs = nullptr;
-        int n = 0, items = 0, pairs = 0;
-        DirectRing ring{};
+        int pairs = 0;
+        std::vector<DirectQueue> queues;
     } direct;
     std::vector<int> fused;      // problems run by their own fused kernel
     std::vector<int> scaled;     // problems whose tile scale is computed per problem
@@ -99,7 +100,7 @@ struct Batch {
     cudaEvent_t fork = nullptr, join[kSides] = {};
     struct Unit {
         Xform xf;      // chain: transform and GEMM tile
-        int bn;
+        int bn;        // (kDirectUnit: the queue)
         int single;    // or the problem run by its own kernel (>= 0), or kDirectUnit
         double flops;  // direct-convolution work
         int stream;    // 0: the caller's stream, k: side[k - 1]
@@ -133,7 +134,7 @@ struct Batch {
 
     cudaError_t launch_unit(const Unit& u, cudaStream_t s) {
         if (u.single == kDirectUnit)
-            return launch_direct_grouped(direct.descs, direct.n, direct.items, direct.ring, direct.pairs, err, s);
+            return launch_direct_grouped(direct.descs, direct.queues[u.bn], direct.pairs, err, s);
         return u.single >= 0 ? launch_single(u.single, s) : launch_chain(u.xf, u.bn, s);
     }
 
@@ -199,12 +200,10 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     const bool split_bn = sb && sb[0] == '1';
     std::map<std::tuple<int, int, int, int>, std::vector<int>> gemm_keys;     // (shape, M type, op, xform) -> problems
     std::vector<DirectProblem> direct_probs;
-    double direct_flops = 0;
     for (int i = 0; i < count; ++i) {
         Plan& p = *b->plans[i];
         if (p.run_direct) {
             direct_probs.push_back({p.g, p.prob.in, p.prob.out, p.U});
-            direct_flops += 18.0 * p.prob.n * p.prob.k * p.g.oh * p.g.ow * p.prob.c;
             continue;
         }
         if (p.single_kernel()) {
@@ -275,10 +274,9 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     }
     std::vector<DirectDesc> direct_descs(direct_probs.size());
     if (!direct_probs.empty()) {
-        b->direct.n = static_cast<int>(direct_probs.size());
         b->direct.pairs = direct_max_pairs(b->plans[0]->num_sms);
-        if (make_direct_group(direct_probs.data(), b->direct.n, b->direct.pairs, direct_descs.data(), b->direct.ring,
-                              b->direct.items) != cudaSuccess)
+        if (make_direct_queues(direct_probs.data(), static_cast<int>(direct_probs.size()), b->direct.pairs,
+                               direct_descs.data(), b->direct.queues) != cudaSuccess)
             return batch_fail(CONV2D_ERR_CUDA, "direct kernel descriptors");
     }
     // one device block: error word | GemmDesc[] and DirectDesc[] (64-byte aligned) | InDesc[] | OutDesc[]
@@ -317,7 +315,7 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
     int single = 0;   // launches of the problems run by their own kernels
     for (int i : b->fused) single += b->plans[i]->launches;
     b->grouped_launches = static_cast<int>(b->scaled.size() + b->in_groups.size() + b->gemm_groups.size() +
-                                           b->out_groups.size()) + single + (b->direct.n ? 1 : 0);
+                                           b->out_groups.size() + b->direct.queues.size()) + single;
     if (cudaDeviceSynchronize() != cudaSuccess) return batch_fail(CONV2D_ERR_CUDA, "batch setup failed");
     // work units (chains and single-kernel problems), largest first, each to
     // the stream with the least direct-convolution work so far
@@ -337,7 +335,14 @@ int batch_create(const problem_t* problems, int count, const conv2d_options_t* o
         b->units.push_back(u);
     }
     for (int i : b->fused) b->units.push_back({Xform::F2, 0, i, flops(i), 0});
-    if (b->direct.n) b->units.push_back({Xform::F2, 0, Batch::kDirectUnit, direct_flops, 0});
+    for (size_t q = 0; q < b->direct.queues.size(); ++q) {
+        Batch::Unit u{Xform::F2, static_cast<int>(q), Batch::kDirectUnit, 0.0, 0};
+        for (int i = 0; i < b->direct.queues[q].n; ++i) {
+            const DirectDesc& d = direct_descs[b->direct.queues[q].first + i];
+            u.flops += 18.0 * d.n * d.k * d.oh * d.ow * d.c;
+        }
+        b->units.push_back(u);
+    }
     std::stable_sort(b->units.begin(), b->units.end(),
                      [](const Batch::Unit& x, const Batch::Unit& y) { return x.flops > y.flops; });
     {

@@ -1179,15 +1179,21 @@ int direct_parts(const DirectPlan& dp, const void* x, void* y, int n_images, Dir
     return out.items;
 }
 
-// Item shapes for a queue of many problems: throughput decides (items x
+// Item shapes for queues of many problems: throughput decides (items x
 // cycles), not rounds, as the problems fill each other's; but no item longer
 // than a third of the queue's time where a shorter one is to be had.  Longest
 // items first, so that the pairs, which take the items in turn, end together.
-cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDesc* out, DirectRing& ring, int& items) {
+//
+// One queue where one ring has room for the widest window and the widest filter
+// tile of all; otherwise the problems with the wider windows get queues of
+// their own (a row of 751 columns beside 256 output channels: three window
+// stages of 52 KB and two filter stages of 37 KB do not fit).  Each problem's
+// own stages fit (choose), so every set of problems has its queues.
+cudaError_t make_direct_queues(const DirectProblem* p, int n, int pairs, DirectDesc* out, std::vector<DirectQueue>& queues) {
     struct Pick {
         DirectDesc d;
         double one;
-        int i;
+        int i, queue;
     };
     std::vector<Pick> picks(n);
     // stages small enough for four of each
@@ -1226,33 +1232,52 @@ cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDe
         total += t;
     }
     const double longest = total / pairs / 3;
-    int a = 0, b = 0;
-    for (Pick& k : picks) {
+    for (Pick& k : picks)
         if (k.one > longest) choose(k, longest);
-        a = std::max(a, window_bytes(k.d.win));
-        b = std::max(b, b_stage_bytes(k.d.bn));
+    // narrower windows first, each problem into the first queue whose ring has room for it
+    std::stable_sort(picks.begin(), picks.end(), [](const Pick& x, const Pick& y) { return x.d.win < y.d.win; });
+    queues.clear();
+    for (Pick& k : picks) {
+        const int a = window_bytes(k.d.win), b = b_stage_bytes(k.d.bn);
+        for (k.queue = 0;; ++k.queue) {
+            if (k.queue == static_cast<int>(queues.size())) queues.push_back(DirectQueue{});
+            DirectQueue& q = queues[k.queue];
+            DirectRing r;
+            if (!size_ring(r, std::max(a, q.ring.a_bytes), std::max(b, q.ring.b_bytes), false)) {
+                if (q.n == 0) return cudaErrorNotSupported;   // (its own stages fit)
+                continue;
+            }
+            q.ring = r;
+            ++q.n;
+            break;
+        }
     }
-    if (!size_ring(ring, a, b, false)) return cudaErrorNotSupported;
-    std::stable_sort(picks.begin(), picks.end(), [](const Pick& x, const Pick& y) { return x.one > y.one; });
-    long long begin = 0;
-    for (int i = 0; i < n; ++i) {
-        DirectDesc& d = picks[i].d;
-        const DirectProblem& q = p[picks[i].i];
-        if (cudaError_t e = encode_filter(d, q.U, false); e != cudaSuccess) return e;
-        const long long rows = 2LL * d.cta_rows;
-        place(d, q.x, q.y, false, 0, (positions(d, d.n) + rows - 1) / rows, static_cast<int>(begin));
-        begin += d.items;
-        if (begin >= (1LL << 31)) return cudaErrorNotSupported;
-        out[i] = d;
+    std::sort(picks.begin(), picks.end(), [](const Pick& x, const Pick& y) {
+        return x.queue != y.queue ? x.queue < y.queue : x.one != y.one ? x.one > y.one : x.i < y.i;
+    });
+    int next = 0;
+    for (DirectQueue& q : queues) {
+        q.first = next;
+        long long begin = 0;
+        for (; next < q.first + q.n; ++next) {
+            DirectDesc& d = picks[next].d;
+            const DirectProblem& pr = p[picks[next].i];
+            if (pr.U)
+                if (cudaError_t e = encode_filter(d, pr.U, false); e != cudaSuccess) return e;
+            const long long rows = 2LL * d.cta_rows;
+            place(d, pr.x, pr.y, false, 0, (positions(d, d.n) + rows - 1) / rows, static_cast<int>(begin));
+            begin += d.items;
+            if (begin >= (1LL << 31)) return cudaErrorNotSupported;
+            out[next] = d;
+        }
+        q.items = static_cast<int>(begin);
     }
-    items = static_cast<int>(begin);
     return cudaSuccess;
 }
 
-cudaError_t launch_direct_grouped(const DirectDesc* descs, int ndesc, int items, const DirectRing& ring, int pairs, DevErr* err,
-                                  cudaStream_t stream) {
-    return launch_cluster<direct3x3_grouped>(std::min(items, pairs), kDirectThreads<false>, ring.smem_bytes, stream, descs, ndesc,
-                                             items, ring, err);
+cudaError_t launch_direct_grouped(const DirectDesc* descs, const DirectQueue& q, int pairs, DevErr* err, cudaStream_t stream) {
+    return launch_cluster<direct3x3_grouped>(std::min(q.items, pairs), kDirectThreads<false>, q.ring.smem_bytes, stream,
+                                             descs + q.first, q.n, q.items, q.ring, err);
 }
 
 cudaError_t launch_direct(const DirectPlan& dp, const void* x, void* y, int n_images, DevErr* err, cudaStream_t stream) {

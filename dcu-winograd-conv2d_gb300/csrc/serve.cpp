@@ -13,7 +13,8 @@
 // slot: one input-transform launch per transform family, one persistent GEMM
 // launch per (channel tile, M type) over every request's tiles, one
 // output-transform launch per family, and one launch over the items of every
-// request that runs the direct kernel.  Requests that arrive while other
+// request that runs the direct kernel (a second one where very wide rows and
+// many output channels do not fit the same ring).  Requests that arrive while other
 // batches are on the GPU are admitted as soon as a slot and workspace free
 // up, and their batch runs concurrently with the ones still in flight.
 // A request's arithmetic does not depend on what else is in its batch, so its
@@ -307,11 +308,10 @@ struct Server {
             off += kv.second.size() * sizeof(GemmDesc);
         }
         std::vector<DirectDesc> dd(direct.size());
-        DirectRing ring{};
-        int direct_items = 0;
+        std::vector<DirectQueue> queues;
         const int pairs = direct.empty() ? 0 : direct_max_pairs(num_sms);
-        if (!direct.empty() && make_direct_group(direct.data(), static_cast<int>(direct.size()), pairs, dd.data(), ring,
-                                                 direct_items) != cudaSuccess)
+        if (!direct.empty() &&
+            make_direct_queues(direct.data(), static_cast<int>(direct.size()), pairs, dd.data(), queues) != cudaSuccess)
             return set_last_error(CONV2D_ERR_CUDA, "direct kernel descriptors");
         const size_t o_direct = off;
         std::memcpy(h + off, dd.data(), dd.size() * sizeof(DirectDesc));
@@ -342,9 +342,9 @@ struct Server {
         if (both) {
             if ((e = cudaEventRecord(slot.fork, s)) == cudaSuccess) e = cudaStreamWaitEvent(s2, slot.fork, 0);
         }
-        if (!dd.empty() && e == cudaSuccess)
-            e = launch_direct_grouped(reinterpret_cast<const DirectDesc*>(d + o_direct), static_cast<int>(dd.size()),
-                                      direct_items, ring, pairs, err, in4.empty() ? s : s2);
+        for (const DirectQueue& q : queues)
+            if (e == cudaSuccess)
+                e = launch_direct_grouped(reinterpret_cast<const DirectDesc*>(d + o_direct), q, pairs, err, in4.empty() ? s : s2);
         if (!in2.empty() && e == cudaSuccess)
             e = launch_input_transform_grouped(Xform::F2, OpType::F16, reinterpret_cast<const InDesc*>(d + o_in2),
                                                static_cast<int>(in2.size()), blk_in2, smem2, false, err, s2);

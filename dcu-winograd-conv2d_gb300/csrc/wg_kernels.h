@@ -4,6 +4,8 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <vector>
+
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -365,15 +367,24 @@ struct DirectProblem {
     void* y;
     const void* U;       // U9
 };
+
+// One launch over problems: descriptors [first, first + n), whose item_begin
+// count from the queue's start.
+struct DirectQueue {
+    int first, n, items;
+    DirectRing ring;
+};
 // Whether the direct kernel takes these sizes.
 bool direct_supported(const Geom& g, bool nhwc);
 // CTA pairs the device runs at once.
 int direct_max_pairs(int num_sms);
-// Descriptors (out[n], sorted by item_begin, to be copied to the device) and
-// ring of one launch over n problems.
-cudaError_t make_direct_group(const DirectProblem* p, int n, int pairs, DirectDesc* out, DirectRing& ring, int& items);
-cudaError_t launch_direct_grouped(const DirectDesc* descs, int ndesc, int items, const DirectRing& ring, int pairs, DevErr* err,
-                                  cudaStream_t stream);
+// Descriptors (out[n], by queue and item_begin, to be copied to the device) and
+// queues of n problems, each of which direct_supported takes: mostly one queue,
+// more where the stages of all do not fit one ring.  U may be null (the
+// descriptors then lack its tensor map).
+cudaError_t make_direct_queues(const DirectProblem* p, int n, int pairs, DirectDesc* out, std::vector<DirectQueue>& queues);
+// descs: those of all queues, on the device
+cudaError_t launch_direct_grouped(const DirectDesc* descs, const DirectQueue& q, int pairs, DevErr* err, cudaStream_t stream);
 long long direct_filter_bytes(int K, int C);
 int direct_threads(bool nhwc);
 // U9[tap][Cp/8][Kp][8] from KCRS weights (16-bit values copied as they are)
