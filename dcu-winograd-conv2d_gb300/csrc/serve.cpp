@@ -126,6 +126,7 @@ struct Request {
     bool direct;        // runs the direct kernel
     size_t ws_off = 0, ws_bytes = 0;
     bool done = false;
+    int status = CONV2D_OK;   // of its launch: otherwise its output is not written
 };
 
 struct Slot {
@@ -141,6 +142,8 @@ struct Slot {
     std::vector<long long> reqs;
     bool busy = false;
 };
+
+constexpr char kFailedRequest[] = "the launch of a request failed: its output is not written";
 
 constexpr size_t kDescBytesPerRequest = sizeof(GemmDesc) + sizeof(InDesc) + sizeof(OutDesc) + sizeof(DirectDesc) + 256;
 
@@ -163,6 +166,7 @@ struct Server {
     long long next_id = 1;
     std::atomic<bool> stop{false};
     std::thread sched;
+    std::vector<long long> failed;   // requests whose launch failed, not yet reported by wait_all or replay
     long long completed = 0;
     double flops_done = 0;
     int batches = 0, batch_requests = 0, max_inflight = 0;
@@ -433,6 +437,48 @@ struct Server {
         ++completed;
     }
 
+    // A batch whose launch failed: its requests one at a time, so that those
+    // that can be launched are.  What the failed launch queued has ended when
+    // this returns; the slot is left with the requests now in flight.
+    void launch_singly(Slot& slot) {
+        std::vector<long long> batch;
+        batch.swap(slot.reqs);
+        std::vector<long long> queued;
+        auto settle = [&] {   // the descriptors and workspaces of what was queued are free again
+            cudaStreamSynchronize(slot.stream);
+            cudaStreamSynchronize(slot.stream2);
+            cudaGetLastError();
+        };
+        for (long long id : batch) {
+            settle();
+            Request& r = reqs[id];
+            slot.reqs.assign(1, id);
+            const int st = launch(slot);
+            if (st == CONV2D_OK) {
+                queued.push_back(id);
+                continue;
+            }
+            settle();
+            arena.release(r.ws_off, r.ws_bytes);
+            r.status = st;
+            r.t_done = now_us();
+            r.done = true;
+            failed.push_back(id);
+        }
+        slot.reqs.swap(queued);
+        slot.busy = !slot.reqs.empty();
+        // the event of the last launch that succeeded stands for those before it
+        if (slot.busy) cudaEventRecord(slot.done, slot.stream);
+        cv.notify_all();
+    }
+
+    bool idle() const {
+        if (!pending.empty() || !plain_inflight.empty()) return false;
+        for (const Slot& s : slots)
+            if (s.busy) return false;
+        return true;
+    }
+
     bool per_request() const { return cfg.per_request != 0; }
 
     void loop() {
@@ -499,16 +545,7 @@ struct Server {
                     free_slot->busy = true;
                     ++batches;
                     batch_requests += static_cast<int>(batch.size());
-                    if (launch(*free_slot) != CONV2D_OK) {
-                        // a launch that fails completes its requests at once
-                        for (long long id : batch) {
-                            reqs[id].done = true;
-                            reqs[id].t_done = now_us();
-                            arena.release(reqs[id].ws_off, reqs[id].ws_bytes);
-                        }
-                        free_slot->reqs.clear();
-                        free_slot->busy = false;
-                    }
+                    if (launch(*free_slot) != CONV2D_OK) launch_singly(*free_slot);
                     max_inflight = std::max(max_inflight, inflight + 1);
                     continue;
                 }
@@ -656,20 +693,19 @@ int conv2d_server_poll(conv2d_server_t* server, long long request, double* laten
     if (it == sv->reqs.end()) return -1;
     if (!it->second.done) return 0;
     if (latency_us) *latency_us = it->second.t_done - it->second.t_arrive;
-    return 1;
+    return it->second.status == CONV2D_OK ? 1 : -2;
 }
 
 int conv2d_server_wait_all(conv2d_server_t* server) {
     Server* sv = reinterpret_cast<Server*>(server);
     if (!sv) return set_last_error(CONV2D_ERR_INVALID, "null server");
     std::unique_lock<std::mutex> lk(sv->mu);
-    sv->cv.wait(lk, [sv] {
-        if (!sv->pending.empty() || !sv->plain_inflight.empty()) return false;
-        for (const Slot& s : sv->slots)
-            if (s.busy) return false;
-        return true;
-    });
-    return CONV2D_OK;
+    sv->cv.wait(lk, [sv] { return sv->idle(); });
+    if (sv->failed.empty()) return CONV2D_OK;
+    const auto it = sv->reqs.find(sv->failed.front());
+    const int st = it != sv->reqs.end() ? it->second.status : CONV2D_ERR_CUDA;
+    sv->failed.clear();
+    return set_last_error(st, kFailedRequest);
 }
 
 int conv2d_server_replay(conv2d_server_t* server, int count, const int* layer, const unsigned* n,
@@ -686,15 +722,19 @@ int conv2d_server_replay(conv2d_server_t* server, int count, const int* layer, c
         const int st = conv2d_server_submit(server, layer[i], n[i], in[i], out[i], &ids[i]);
         if (st) return st;
     }
-    conv2d_server_wait_all(server);
+    std::unique_lock<std::mutex> lk(sv->mu);
+    sv->cv.wait(lk, [sv] { return sv->idle(); });
     if (wall_us) *wall_us = now_us() - t0;
-    std::lock_guard<std::mutex> lk(sv->mu);
+    int st = CONV2D_OK;
     for (int i = 0; i < count; ++i) {
         const Request& r = sv->reqs[ids[i]];
         latency_us[i] = r.t_done - r.t_arrive;
+        if (r.status == CONV2D_OK) continue;
+        if (st == CONV2D_OK) st = r.status;
+        sv->failed.erase(std::remove(sv->failed.begin(), sv->failed.end(), ids[i]), sv->failed.end());
     }
     for (int i = 0; i < count; ++i) sv->reqs.erase(ids[i]);
-    return CONV2D_OK;
+    return st == CONV2D_OK ? CONV2D_OK : set_last_error(st, kFailedRequest);
 }
 
 int conv2d_server_stats(conv2d_server_t* server, conv2d_server_stats_t* st) {

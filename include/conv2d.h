@@ -282,11 +282,15 @@ int conv2d_server_add_layer(conv2d_server_t* server, unsigned c, unsigned k, uns
  * CONV2D_ERR_BUSY when its workspace alone exceeds the budget. */
 int conv2d_server_submit(conv2d_server_t* server, int layer, unsigned n, const void* in, void* out,
                          long long* request);
-/* 1 when done (latency in microseconds, arrival to completion), 0 pending, -1 unknown. */
+/* 1 when done (latency in microseconds, arrival to completion), 0 pending, -1 unknown,
+ * -2 when its launch failed: it is over, but its output is not written. */
 int conv2d_server_poll(conv2d_server_t* server, long long request, double* latency_us);
+/* Waits for every request; a failing status when the launch of one of them
+ * failed since the last call (poll says which). */
 int conv2d_server_wait_all(conv2d_server_t* server);
 /* Submits `count` requests at their arrival times (microseconds from the call),
- * waits for all, returns each latency and the wall time. */
+ * waits for all, returns each latency and the wall time; a failing status when
+ * the launch of one of them failed. */
 int conv2d_server_replay(conv2d_server_t* server, int count, const int* layer, const unsigned* n,
                          const double* arrival_us, const void* const* in, void* const* out, double* latency_us,
                          double* wall_us);
