@@ -9,6 +9,7 @@
 #pragma once
 #include <atomic>
 #include <cstdlib>
+#include <mutex>
 #include <utility>
 
 #include <cuda_runtime.h>
@@ -26,16 +27,21 @@ inline bool pdl_enabled() {
 // Raises the kernel's dynamic shared memory limit to `bytes` on the current
 // device, once (the limit stays until the process ends): asking the runtime on
 // every launch cost 0.3-0.4 us of host time (a call of one kernel 3.58 -> 3.18 us
-// to submit, of three 7.6 -> 6.7).
+// to submit, of three 7.6 -> 6.7).  Limit and cached value are raised under one
+// lock and never lowered: of two threads that raise a kernel's limit at once, by
+// unlike sizes, neither may leave a cached value above the limit in force.
 template <auto Kernel>
 cudaError_t allow_smem(int bytes) {
     constexpr int kDevices = 64;
     static std::atomic<int> allowed[kDevices] = {};
+    static std::mutex raising;
     int dev = 0;
     if (cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return e;
+    if (dev < kDevices && allowed[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+    std::lock_guard<std::mutex> lock(raising);
     if (dev < kDevices && allowed[dev].load(std::memory_order_relaxed) >= bytes) return cudaSuccess;
     const cudaError_t e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess && dev < kDevices) allowed[dev].store(bytes, std::memory_order_relaxed);
+    if (e == cudaSuccess && dev < kDevices) allowed[dev].store(bytes, std::memory_order_release);
     return e;
 }
 
