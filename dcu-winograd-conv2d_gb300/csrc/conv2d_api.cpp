@@ -146,6 +146,7 @@ void Plan::release() {
     for (cudaEvent_t& e : host_ev)
         if (e) cudaEventDestroy(e);
     host_in_stream = host_out_stream = nullptr;
+    delete loaded.exchange(nullptr);
     if (ws) cudaFree(ws);
     ws = nullptr;
     U = V = Mw = nullptr;
@@ -153,7 +154,7 @@ void Plan::release() {
     err = nullptr;
 }
 
-int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
+int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in, bool filter_only) {
     int st = validate_problem(pr);
     if (st) return st;
     prob = *pr;
@@ -244,7 +245,7 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
     g = make_geom(pr->n, pr->c, pr->h, pr->w, pr->k, pr->p, pr->q, m);
     const int E = g.alpha * g.alpha;
     const long long op_bytes = 2;
-    if (!single_kernel() && !nhwc) {
+    if (!filter_only && !single_kernel() && !nhwc) {
         // the input transform stages whole input rows of 8 channels, twice
         int in_smem = 0;
         make_in_desc(g, pr->in, pr->in, nullptr, nullptr, &in_smem);
@@ -267,7 +268,7 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
                                             : static_cast<long long>(E) * g.kp * g.cp * op_bytes;
     const long long bU = al(u_bytes);
     long long bV = 0, bM = 0, bS = 0;
-    if (!single_kernel()) {
+    if (!filter_only && !single_kernel()) {
         bV = al(static_cast<long long>(E) * round_rows(Pc) * g.cp * op_bytes);
         bM = al(m_bytes(mt, E, Pc, g.kp));
         if (scaling) bS = al(Pc * 4);
@@ -288,6 +289,7 @@ int Plan::build(const problem_t* pr, const conv2d_options_t* opt_in) {
     err = reinterpret_cast<DevErr*>(b + bU + bV + bM + bS);
     ce = cudaMemset(err, 0, sizeof(DevErr));
     if (ce != cudaSuccess) return cuda_fail(ce, "cudaMemset");
+    if (filter_only) return CONV2D_OK;
 
     if (run_direct) {
         ce = plan_direct(direct, g, nhwc, opt.io_bf16 != 0, U, algo == CONV2D_ALGO_DIRECT ? direct_tile(opt) : 0, num_sms);
@@ -670,11 +672,17 @@ int Plan::enqueue_host(const void* const* host_in, void* const* host_out, int st
 
 int set_last_error(int status, const char* msg) { return fail(status, msg); }
 
-Plan* plan_of(const void* param) {
+Plan* blob_plan(const void* param) {
     if (!param) return nullptr;
     const ParamBlob* pb = static_cast<const ParamBlob*>(param);
     if (pb->magic != kParamMagic || !pb->plan) return nullptr;
     return static_cast<Plan*>(pb->plan);
+}
+
+Plan* plan_of(const void* param) {
+    Plan* pl = blob_plan(param);
+    Plan* loaded = pl ? pl->loaded.load(std::memory_order_acquire) : nullptr;
+    return loaded ? loaded : pl;
 }
 
 void fill_blob(ParamBlob* pb, Plan* pl) {
@@ -695,10 +703,13 @@ void fill_blob(ParamBlob* pb, Plan* pl) {
     pb->plan = pl;
 }
 
-void replace_plan(void* param, Plan* plan) {
-    Plan* old = plan_of(param);
-    fill_blob(static_cast<ParamBlob*>(param), plan);
-    delete old;
+void set_loaded(void* param, Plan* plan) {
+    Plan* owner = blob_plan(param);
+    ParamBlob* pb = static_cast<ParamBlob*>(param);
+    pb->U_d = plan->U;
+    pb->V_d = plan->V;
+    pb->M_d = plan->Mw;
+    owner->loaded.store(plan, std::memory_order_release);
 }
 
 }  // namespace wg
@@ -794,11 +805,15 @@ int conv2d_refresh_filter(const void* param_ptr, void* stream) {
     Plan* pl = plan_of(param_ptr);
     if (!pl) return fail(CONV2D_ERR_INVALID, "param blob not set up by getkernelInfo");
     DeviceGuard dg(pl->device);
+    // graphs captured before a filter file was loaded run the plan the blob was set up with
+    Plan* first = blob_plan(param_ptr);
+    if (first != pl)
+        if (const int st = first->filter(static_cast<cudaStream_t>(stream))) return st;
     return pl->filter(static_cast<cudaStream_t>(stream));
 }
 
 int conv2d_destroy(void* param_ptr) {
-    Plan* pl = plan_of(param_ptr);
+    Plan* pl = blob_plan(param_ptr);
     if (!pl) return fail(CONV2D_ERR_INVALID, "param blob not set up by getkernelInfo");
     {
         DeviceGuard dg(pl->device);
@@ -820,8 +835,8 @@ int conv2d_get_direct(const void* param_ptr) {
 }
 
 long long conv2d_workspace_bytes(const void* param_ptr) {
-    Plan* pl = plan_of(param_ptr);
-    return pl ? pl->ws_bytes : -1;
+    Plan *pl = plan_of(param_ptr), *first = blob_plan(param_ptr);
+    return pl ? pl->ws_bytes + (first != pl ? first->ws_bytes : 0) : -1;
 }
 
 int conv2d_launches_per_call(const void* param_ptr) {
@@ -835,15 +850,18 @@ int conv2d_check_device(const void* param_ptr, int* site) {
     DeviceGuard dg(pl->device);
     cudaError_t ce = cudaDeviceSynchronize();
     if (ce != cudaSuccess) return cuda_fail(ce, "device synchronize");
-    DevErr h{};
-    ce = cudaMemcpy(&h, pl->err, sizeof(h), cudaMemcpyDeviceToHost);
-    if (ce != cudaSuccess) return cuda_fail(ce, "error word copy");
-    if (site) *site = static_cast<int>(h.code);
-    if (h.code) {
-        cudaMemset(pl->err, 0, sizeof(DevErr));
-        return fail(CONV2D_ERR_TIMEOUT, "a kernel gave up a bounded wait");
+    // graphs captured before a filter file was loaded report to the plan the blob was set up with
+    Plan* const plans[2] = {pl, blob_plan(param_ptr)};
+    unsigned code = 0;
+    for (int i = 0; i < (plans[1] != pl ? 2 : 1); ++i) {
+        DevErr h{};
+        ce = cudaMemcpy(&h, plans[i]->err, sizeof(h), cudaMemcpyDeviceToHost);
+        if (ce != cudaSuccess) return cuda_fail(ce, "error word copy");
+        if (h.code) cudaMemset(plans[i]->err, 0, sizeof(DevErr));
+        if (!code) code = h.code;
     }
-    return CONV2D_OK;
+    if (site) *site = static_cast<int>(code);
+    return code ? fail(CONV2D_ERR_TIMEOUT, "a kernel gave up a bounded wait") : CONV2D_OK;
 }
 
 int conv2d_last_error(void) { return t_last_status; }

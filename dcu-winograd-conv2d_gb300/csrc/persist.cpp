@@ -14,6 +14,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -77,13 +78,12 @@ PlanFileHeader header_of(const Plan& pl) {
 
 // The plan of the Winograd algorithm that a tuned plan running the direct
 // kernel stands for: its filter files are that algorithm's, as they are where
-// the direct kernel is not the faster.  Null when it cannot be made.
-std::unique_ptr<Plan> winograd_plan(const Plan& pl) {
+// the direct kernel is not the faster.
+int winograd_plan(const Plan& pl, bool filter_only, std::unique_ptr<Plan>& out) {
     conv2d_options_t o = pl.opt;
     o.algo = pl.algo;
-    std::unique_ptr<Plan> np(new Plan());
-    if (np->build(&pl.prob, &o) != CONV2D_OK) return nullptr;
-    return np;
+    out.reset(new Plan());
+    return out->build(&pl.prob, &o, filter_only);
 }
 
 }  // namespace
@@ -106,8 +106,11 @@ int conv2d_plan_save(const void* param, const char* path) {
     if (pl->run_direct && pl->algo != CONV2D_ALGO_DIRECT) {
         // from the plan's own copy of the filter: the caller's may have changed or be gone
         void* w = nullptr;
-        if (!(winograd = winograd_plan(*pl)) || cudaMalloc(&w, static_cast<size_t>(pl->prob.k) * pl->prob.c * 18) != cudaSuccess)
+        if (const int st = winograd_plan(*pl, true, winograd)) return st;
+        if (cudaMalloc(&w, static_cast<size_t>(pl->prob.k) * pl->prob.c * 18) != cudaSuccess) {
+            cudaGetLastError();
             return set_last_error(CONV2D_ERR_NOMEM, "workspace of the filter transform");
+        }
         winograd->prob.weight = w;
         const bool ok = launch_direct_unfilter(pl->U, w, pl->g.k, pl->g.c, nullptr) == cudaSuccess &&
                         winograd->filter(nullptr) == CONV2D_OK && cudaDeviceSynchronize() == cudaSuccess;
@@ -128,21 +131,26 @@ int conv2d_plan_save(const void* param, const char* path) {
 }
 
 int conv2d_plan_load(const void* param, const char* path) {
+    Plan* owner = blob_plan(param);
+    if (!owner || !path) return set_last_error(CONV2D_ERR_INVALID, "param blob not set up, or null path");
+    std::lock_guard<std::mutex> lock(owner->loading);
     Plan* pl = plan_of(param);
-    if (!pl || !path) return set_last_error(CONV2D_ERR_INVALID, "param blob not set up, or null path");
     FILE* f = std::fopen(path, "rb");
     if (!f) return set_last_error(CONV2D_ERR_INVALID, "cannot open the plan file");
     PlanFileHeader h;
     std::vector<unsigned char> u;
     bool ok = std::fread(&h, sizeof(h), 1, f) == 1;
     DeviceGuard dg(pl->device);
+    // a tuned plan that runs the direct kernel: the file's filter is that of the
+    // Winograd algorithm, which gets a plan of its own once the file is read
+    const bool tuned = pl->run_direct && pl->algo != CONV2D_ALGO_DIRECT;
     std::unique_ptr<Plan> winograd;
-    if (pl->run_direct && pl->algo != CONV2D_ALGO_DIRECT && !(winograd = winograd_plan(*pl))) {
-        std::fclose(f);
-        return set_last_error(CONV2D_ERR_NOMEM, "workspace of the plan file's algorithm");
-    }
-    Plan* to = winograd ? winograd.get() : pl;   // the plan the file's filter feeds from now on
-    const PlanFileHeader want = header_of(*to);
+    if (tuned)
+        if (const int st = winograd_plan(*pl, true, winograd)) {
+            std::fclose(f);
+            return st;
+        }
+    const PlanFileHeader want = header_of(tuned ? *winograd : *pl);
     if (ok && (std::memcmp(h.magic, kPlanMagic, 8) != 0 || h.version != 1)) {
         std::fclose(f);
         return set_last_error(CONV2D_ERR_INVALID, "not a plan file");
@@ -159,11 +167,14 @@ int conv2d_plan_load(const void* param, const char* path) {
     std::fclose(f);
     if (!ok) return set_last_error(CONV2D_ERR_INVALID, "plan file truncated");
     if (fnv1a(u.data(), u.size()) != h.checksum) return set_last_error(CONV2D_ERR_INVALID, "plan file checksum mismatch");
+    if (tuned)
+        if (const int st = winograd_plan(*pl, false, winograd)) return st;
+    Plan* to = tuned ? winograd.get() : pl;
     // U may still be read by work queued earlier on any stream
     if (cudaDeviceSynchronize() != cudaSuccess || cudaMemcpy(to->U, u.data(), u.size(), cudaMemcpyHostToDevice) != cudaSuccess)
         return set_last_error(CONV2D_ERR_CUDA, "copy of the transformed filter failed");
     to->filter_ready = true;
-    if (winograd) replace_plan(const_cast<void*>(param), winograd.release());
+    if (tuned) set_loaded(const_cast<void*>(param), winograd.release());
     return CONV2D_OK;
 }
 

@@ -1,6 +1,8 @@
 // Plan object behind the opaque param blob of the C ABI.
 #pragma once
+#include <atomic>
 #include <cstdint>
+#include <mutex>
 
 #include "../../include/conv2d.h"
 #include "wg_kernels.h"
@@ -63,6 +65,14 @@ struct Plan {
     unsigned info_grid = 0, info_threads = 0;
     int info_smem = 0;
 
+    // A plan that runs the direct kernel beside the Winograd algorithm it stands
+    // for, once a filter file of that algorithm was loaded into it: the plan
+    // that calls run from then on (plan_of), owned.  This plan and its memory
+    // stay as they are: graphs captured from its calls, copies of the param
+    // blob and calls on other threads may still use them.
+    std::atomic<Plan*> loaded{nullptr};
+    std::mutex loading;
+
     // when set, run() records an event on the stream after every launch
     cudaEvent_t* marks = nullptr;
     int n_marks = 0, max_marks = 0;
@@ -90,7 +100,8 @@ struct Plan {
     bool m_row() const { return nhwc && mt != MType::F24; }
 
     ~Plan();
-    int build(const problem_t* pr, const conv2d_options_t* opt);
+    // filter_only: just what filter() needs (U), no workspace of calls
+    int build(const problem_t* pr, const conv2d_options_t* opt, bool filter_only = false);
     int filter(cudaStream_t s);
     int run(cudaStream_t s);
     // images [n0, n0 + nc) with the given GEMM plan (sized for nc images)
@@ -135,9 +146,13 @@ int default_bn(int K);
 int select_reference64(unsigned long long n, unsigned long long c, unsigned long long h, unsigned long long w,
                        unsigned long long k, unsigned long long r, unsigned long long s, unsigned long long oh,
                        unsigned long long ow);
+// The plan that calls of the blob run, and the one the blob was set up with,
+// which owns it (the same one unless a filter file was loaded, Plan::loaded).
 Plan* plan_of(const void* param);
-// Puts `plan` in place of the blob's plan, which is deleted.
-void replace_plan(void* param, Plan* plan);
+Plan* blob_plan(const void* param);
+// Makes `plan` the one that calls of the blob run; the blob's plan, which has
+// none yet, owns it.
+void set_loaded(void* param, Plan* plan);
 
 // Records the status and message conv2d_last_error / _message report.
 int set_last_error(int status, const char* msg);

@@ -188,11 +188,12 @@ int conv2d_get_algo(const void* param_ptr);
 /* 1 when conv2d calls of this blob run the direct kernel: asked for as
  * CONV2D_ALGO_DIRECT, or, under CONV2D_ALGO_AUTO, measured faster than the
  * selected algorithm (which conv2d_get_algo still reports, and whose filter
- * files conv2d_plan_save and _load still use; after a load the blob runs that
- * algorithm, from the file's filter).  0 otherwise, -1 for a bad blob. */
+ * files conv2d_plan_save and _load still use; after a load calls of the blob run
+ * that algorithm, from the file's filter).  0 otherwise, -1 for a bad blob. */
 int conv2d_get_direct(const void* param_ptr);
 
-/* Device workspace bytes held by the blob. */
+/* Device workspace bytes held by the blob (after conv2d_plan_load into a blob
+ * that ran the direct kernel: those of both plans). */
 long long conv2d_workspace_bytes(const void* param_ptr);
 
 /* Kernel launches one conv2d_fp16 call makes (with the filter already transformed). */
@@ -304,7 +305,16 @@ int conv2d_server_destroy(conv2d_server_t* server);
  * file; loading it into a plan of the same layer skips the filter transform
  * (a restarted process pairs this with WG_CONV2D_TUNE_FILE for the autotuner's
  * choices).  Load fails with CONV2D_ERR_INVALID when the file was made for
- * another layer, transform or operand type, or is damaged. */
+ * another layer, transform or operand type, or is damaged.
+ * A blob that runs the direct kernel by the autotuner's choice: save allocates
+ * device memory for the two forms of the filter while it works; load allocates
+ * the Winograd algorithm's workspace (CONV2D_ERR_NOMEM when there is none),
+ * which the blob keeps beside its own, and calls then run that algorithm (the
+ * file does not hold the direct kernel's filter), which is the slower one here.
+ * Addresses that the caller holds stay valid until conv2d_destroy; a graph
+ * captured from the blob before the load keeps running the direct kernel with
+ * the filter that it had (or conv2d_refresh_filter gives it): capture again to
+ * run the loaded one. */
 int conv2d_plan_save(const void* param, const char* path);
 int conv2d_plan_load(const void* param, const char* path);
 /* A server's resident layers (both transformed filters of each) to a file,
