@@ -725,6 +725,10 @@ __device__ __forceinline__ void direct_body(const DirectDesc* __restrict__ descs
             if (lane == 0) mbar_arrive(&tabfull[0]);
             k = kTables;
         }
+        // nothing here needs the kernel ahead, but the bounded waits below end only
+        // after the producers, who do, have read a table: its remaining time must
+        // not count against them
+        start();
         for (int t = first + k * step; t < total_items; t += kTables * step, k += kTables) {
             const DItem it = locate_direct(descs, ndesc, t, pi);
             if (!mbar_wait_warp(&tabempty[k % kTables], ((k / kTables) & 1) ^ 1, abort_flag, err, ERR_SITE_EMPTY)) break;
