@@ -228,6 +228,27 @@ struct Server {
         return (std::min(L.c, L.k) >= 128 && L.h >= 14 && L.w >= 14) ? 4 : 2;
     }
 
+    // Rows so wide that the direct kernel is the slower.  A window holds its 128
+    // positions and two padded rows, so what an item loads per product grows with
+    // the row, and the rings get fewer stages; the Winograd paths' cost per row
+    // does not.  Against F(4x3) it is the producers' time against the products':
+    // the wider the channels, the sooner the Winograd path wins.  Against F(2x3)
+    // the input channels count (they are the length of an item).  Odd rows are
+    // read pixel by pixel.  Direct / Winograd, us, single calls:
+    //   F(4x3)  128 -> 128, 64 x 560: 24 / 26, 64 x 640: 38 / 29, 1000^2: 2094 / 570
+    //           256 -> 256, 300^2: 78 / 94, 64 x 320: 1.14 of F(4x3), 64 x 400: 41 / 36, 64 x 1000: 528 / 69
+    //           512 -> 256, 64 x 200: 32 / 33, 256^2: 1.02 of F(4x3), 400^2: 306 / 257, 64 x 161: 1.03
+    //   F(2x3)  64 -> 64, 800^2: 128 / 231, 64 x 800: 25 / 26, 64 x 900: 31 / 28, 1000^2: 615 / 367
+    //           256 -> 64, 64 x 600: 0.88 of F(2x3), 64 x 640: 48 / 42, 64 x 301: 1.10, 64 x 401: 1.22
+    bool wide_rows(const Layer& L) const {
+        const bool odd = L.w % 2 != 0;
+        if (choose_m(L) == 4) {
+            const double w = odd ? L.w * 4.0 / 3 : L.w;
+            return w * w * L.c * L.k > 6e9;   // 300 columns at 256 x 256 channels
+        }
+        return L.w > (odd ? (L.c <= 128 ? 560u : 300u) : (L.c <= 64 ? 800u : 600u));
+    }
+
     // The direct kernel holds about 1,430 TFLOP/s of direct-convolution work
     // under the power cap whatever the channels; F(4x3), whose traffic per
     // product falls as they grow, passes it from about 512 x 512 channels on
@@ -236,7 +257,7 @@ struct Server {
     // 44.7; 16 x 30^2 53.7 against 48.9; 32 x 20^2 42.0 against 44.8) or the request
     // is small (1 x 56^2: 18.9 against 17.2; 8 x 28^2 26.9 against 28.5).
     bool choose_direct(const Layer& L, unsigned n) const {
-        if (cfg.algo != CONV2D_ALGO_AUTO || !L.U9) return false;
+        if (cfg.algo != CONV2D_ALGO_AUTO || !L.U9 || wide_rows(L)) return false;
         const long long oh = L.h + 2LL * L.p - 2, ow = L.w + 2LL * L.q - 2;
         const long long tiled = (oh + 3) / 4 * ((ow + 3) / 4) * 16;
         if (std::min(L.c, L.k) >= 512 && L.h >= 14 && L.w >= 14 && 20 * tiled <= 21 * oh * ow && n * oh * ow >= 4096) return false;
