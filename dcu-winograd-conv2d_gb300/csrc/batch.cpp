@@ -8,8 +8,8 @@
 //     per (channel tile, M type) whose work queue holds every (problem,
 //     element, tile block, channel block) item, the output transforms in one
 //     launch per family, the problems that run the direct kernel in one
-//     launch over all their items (one more for rows so wide that their windows
-//     and the others' filter tiles do not fit one ring) -- captured once into a CUDA graph and
+//     launch over all their items (another for rows so wide that their windows
+//     and the others' filter tiles do not share a ring) -- captured once into a CUDA graph and
 //     replayed; or
 //   * per call: each problem's own launches, one problem after another
 //     (the comparison the grouped run is measured against).

@@ -45,6 +45,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <utility>
 #include <vector>
 
 #include "wg_kernels.h"
@@ -1188,11 +1189,15 @@ int direct_parts(const DirectPlan& dp, const void* x, void* y, int n_images, Dir
 // than a third of the queue's time where a shorter one is to be had.  Longest
 // items first, so that the pairs, which take the items in turn, end together.
 //
-// One queue where one ring has room for the widest window and the widest filter
-// tile of all; otherwise the problems with the wider windows get queues of
-// their own (a row of 751 columns beside 256 output channels: three window
-// stages of 52 KB and two filter stages of 37 KB do not fit).  Each problem's
-// own stages fit (choose), so every set of problems has its queues.
+// Problems share a queue where one ring has room for the widest window and the
+// widest filter tile of all, three stages of each (or as many as a problem's own
+// ring has): up to rows of about 220 columns always.  The problems with wider
+// windows get queues of their own.  32x256x56^2 -> 256, 16x128x28^2 -> 128 and
+// 8x512x14^2 -> 512 take 84-88 us together; with 64x560^2 -> 64, 56 us by itself,
+// they took 199 in one queue of two filter stages and take 138 in two; with
+// 64x760^2 -> 64 (108) 323 when its items were held to one block of positions, now
+// 181; with 64x300^2 -> 64 (20) 102-104 in one.  Each problem's own stages fit
+// (choose), so every set of problems has its queues.
 cudaError_t make_direct_queues(const DirectProblem* p, int n, int pairs, DirectDesc* out, std::vector<DirectQueue>& queues) {
     struct Pick {
         DirectDesc d;
@@ -1200,10 +1205,13 @@ cudaError_t make_direct_queues(const DirectProblem* p, int n, int pairs, DirectD
         int i, queue;
     };
     std::vector<Pick> picks(n);
-    // stages small enough for four of each
+    // stages small enough for four of each; of wide rows, whose windows are too
+    // long for that anyway, any that fit (several blocks share the window's halo)
     auto fits = [](int bn, int mb, int pw) {
         DirectRing r;
-        return tile_fits(bn, mb, pw, &r, false) && (mb == 1 || r.a_bytes <= 18 * 1024);
+        constexpr int kShared = 18 * 1024;
+        return tile_fits(bn, mb, pw, &r, false) &&
+               (mb == 1 || r.a_bytes <= kShared || window_bytes(window_of(1, pw)) > kShared);
     };
     auto choose = [&](Pick& k, double longest) {
         const long long pos = positions(k.d, k.d.n);
@@ -1241,19 +1249,26 @@ cudaError_t make_direct_queues(const DirectProblem* p, int n, int pairs, DirectD
     // narrower windows first, each problem into the first queue whose ring has room for it
     std::stable_sort(picks.begin(), picks.end(), [](const Pick& x, const Pick& y) { return x.d.win < y.d.win; });
     queues.clear();
+    constexpr int kEnough = 3;
+    std::vector<std::pair<int, int>> least;   // stages that a queue's ring keeps
     for (Pick& k : picks) {
         const int a = window_bytes(k.d.win), b = b_stage_bytes(k.d.bn);
+        DirectRing own, r;
+        if (!size_ring(own, a, b, false)) return cudaErrorNotSupported;
         for (k.queue = 0;; ++k.queue) {
-            if (k.queue == static_cast<int>(queues.size())) queues.push_back(DirectQueue{});
-            DirectQueue& q = queues[k.queue];
-            DirectRing r;
-            if (!size_ring(r, std::max(a, q.ring.a_bytes), std::max(b, q.ring.b_bytes), false)) {
-                if (q.n == 0) return cudaErrorNotSupported;   // (its own stages fit)
-                continue;
+            if (k.queue == static_cast<int>(queues.size())) {
+                queues.push_back(DirectQueue{});
+                least.push_back({0, 0});
             }
-            q.ring = r;
-            ++q.n;
-            break;
+            DirectQueue& q = queues[k.queue];
+            const int na = std::max(least[k.queue].first, std::min(kEnough, own.na));
+            const int nb = std::max(least[k.queue].second, std::min(kEnough, own.nb));
+            if (size_ring(r, std::max(a, q.ring.a_bytes), std::max(b, q.ring.b_bytes), false) && r.na >= na && r.nb >= nb) {
+                q.ring = r;
+                least[k.queue] = {na, nb};
+                ++q.n;
+                break;
+            }
         }
     }
     std::sort(picks.begin(), picks.end(), [](const Pick& x, const Pick& y) {

@@ -14,7 +14,7 @@
 // launch per (channel tile, M type) over every request's tiles, one
 // output-transform launch per family, and one launch over the items of every
 // request that runs the direct kernel (a second one where very wide rows and
-// many output channels do not fit the same ring).  Requests that arrive while other
+// many output channels do not share a ring).  Requests that arrive while other
 // batches are on the GPU are admitted as soon as a slot and workspace free
 // up, and their batch runs concurrently with the ones still in flight.
 // A request's arithmetic does not depend on what else is in its batch, so its

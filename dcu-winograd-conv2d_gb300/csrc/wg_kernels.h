@@ -380,7 +380,7 @@ bool direct_supported(const Geom& g, bool nhwc);
 int direct_max_pairs(int num_sms);
 // Descriptors (out[n], by queue and item_begin, to be copied to the device) and
 // queues of n problems, each of which direct_supported takes: mostly one queue,
-// more where the stages of all do not fit one ring.  U may be null (the
+// more where one ring has too few stages for all.  U may be null (the
 // descriptors then lack its tensor map).
 cudaError_t make_direct_queues(const DirectProblem* p, int n, int pairs, DirectDesc* out, std::vector<DirectQueue>& queues);
 // descs: those of all queues, on the device

@@ -68,6 +68,17 @@ def planner(wg, tmp_path_factory):
     return plan
 
 
+def own_stages(a, b):
+    """Window and filter stages of a ring for these sizes: as many of the
+    filter as of both, the rest to the windows, three of those and two at least."""
+    room = 227 * 1024 - 1536
+    for nb in range(min(12, room // (a + b)), 1, -1):
+        na = min(12, (room - nb * b) // a)
+        if na >= 3:
+            return na, nb
+    raise AssertionError((a, b))
+
+
 def check(shapes, got):
     assert got["status"] == 0, shapes
     seen, first = [], 0
@@ -77,6 +88,11 @@ def check(shapes, got):
         # the rings: fewest stages, all of shared memory at most (barriers and alignment 1,536 bytes)
         assert q["na"] >= 3 and q["nb"] >= 2 and q["smem"] <= 227 * 1024
         assert q["na"] * q["a"] + q["nb"] * q["b"] + 1536 <= q["smem"]
+        if len(q["problems"]) > 1:
+            # as deep as a problem alone would have it, or three of each
+            for p in q["problems"]:
+                own = own_stages((2 * p["gran"] + 127) // 128 * 128 + 32, 9 * 16 * p["bn"])
+                assert q["na"] >= min(3, own[0]) and q["nb"] >= min(3, own[1])
         begin = 0
         for p in q["problems"]:
             n, c, h, w, k = shapes[p["i"]]
@@ -94,17 +110,16 @@ def check(shapes, got):
 
 def test_wide_rows_beside_many_channels(planner):
     """Every width that the kernel takes beside every filter tile, both ways
-    round, and several of each: all are planned, in one queue where one ring
-    holds the stages of all."""
+    round, and several of each: all are planned, the narrow ones together."""
     sets = []
-    for w in (300, 500, 640, 750, 751, 847, 943, 1000, 1079, 1080):
+    for w in (222, 300, 500, 640, 750, 751, 847, 943, 1000, 1079, 1080):
         for k in (8, 64, 96, 128, 192, 256, 512):
             wide, many = (1, 64, 200, w, 64), (8, 256, 14, 14, k)
             sets += [[wide, many], [many, wide], [many, (3, 8, 9, w, 300), (32, 256, 28, 28, k), wide, (1, 3, 1, 1, 1)]]
     for shapes, got in zip(sets, planner(sets)):
         check(shapes, got)
-        if max(s[3] for s in shapes) <= 500:
-            assert len(got["queues"]) == 1
+        narrow = {i for i, s in enumerate(shapes) if s[3] <= 220}
+        assert narrow == set(p["i"] for p in got["queues"][0]["problems"]) & narrow
     split = [[(1, 64, 800, 800, 64), (8, 256, 14, 14, 256)]]
     got = planner(split)[0]
     assert [[p["i"] for p in q["problems"]] for q in got["queues"]] == [[1], [0]]
