@@ -228,25 +228,27 @@ struct Server {
         return (std::min(L.c, L.k) >= 128 && L.h >= 14 && L.w >= 14) ? 4 : 2;
     }
 
-    // Rows so wide that the direct kernel is the slower.  A window holds its 128
-    // positions and two padded rows, so what an item loads per product grows with
-    // the row, and the rings get fewer stages; the Winograd paths' cost per row
-    // does not.  Against F(4x3) it is the producers' time against the products':
-    // the wider the channels, the sooner the Winograd path wins.  Against F(2x3)
-    // the input channels count (they are the length of an item).  Odd rows are
-    // read pixel by pixel.  Direct / Winograd, us, single calls:
-    //   F(4x3)  128 -> 128, 64 x 560: 24 / 26, 64 x 640: 38 / 29, 1000^2: 2094 / 570
-    //           256 -> 256, 300^2: 78 / 94, 64 x 320: 1.14 of F(4x3), 64 x 400: 41 / 36, 64 x 1000: 528 / 69
-    //           512 -> 256, 64 x 200: 32 / 33, 256^2: 1.02 of F(4x3), 400^2: 306 / 257, 64 x 161: 1.03
-    //   F(2x3)  64 -> 64, 800^2: 128 / 231, 64 x 800: 25 / 26, 64 x 900: 31 / 28, 1000^2: 615 / 367
-    //           256 -> 64, 64 x 600: 0.88 of F(2x3), 64 x 640: 48 / 42, 64 x 301: 1.10, 64 x 401: 1.22
+    // Rows so wide that the direct kernel is the slower.  A window holds two padded
+    // rows beside its positions, so what an item loads per product grows with the
+    // row, and the rings get fewer stages; the Winograd paths' cost per row does
+    // not.  Against F(4x3), which saves more products the more channels there are,
+    // channels bring the line down; odd rows are read pixel by pixel.  Direct /
+    // Winograd time of one request of 64 rows, of one of 200 rows, of 8 of 64 rows:
+    //   F(4x3)  128 -> 128  640: 1.06 / 0.85 / 0.70    751: 1.23 / 0.99 / 0.93
+    //           256 -> 256  560: 0.95 / 0.92 / 0.84    640: 1.25 / 1.00 / 0.92
+    //                       301: 0.86 / 0.90 / 0.75    401: 1.30 / 1.15 / 0.99
+    //           512 -> 256  400: 1.23 / 1.03 / 0.82    480: 1.25 / 1.06 / 1.33
+    //                       201: 1.00 / 1.00 / 0.82    257: 1.09 / 1.06 / 0.96
+    //          1024 -> 256  300: 0.80 / 1.03 / 0.83    400: 1.29 / 1.15 / 1.28
+    //   F(2x3)   32 ->  32 1080: 1.07 / 1.09 / 0.95
+    //           256 ->  64  900: 1.07 / 0.90 / 0.78   1000: 1.62 / 1.49 / 1.41
+    //                       801: 1.17 / 1.06 / 0.84   1080: 2.62 / 2.68 / 2.78
+    // (nearly equal: the more accurate one).
     bool wide_rows(const Layer& L) const {
         const bool odd = L.w % 2 != 0;
-        if (choose_m(L) == 4) {
-            const double w = odd ? L.w * 4.0 / 3 : L.w;
-            return w * w * L.c * L.k > 6e9;   // 300 columns at 256 x 256 channels
-        }
-        return L.w > (odd ? (L.c <= 128 ? 560u : 300u) : (L.c <= 64 ? 800u : 600u));
+        if (choose_m(L) == 4)
+            return L.w > 640 || static_cast<double>(L.w) * L.w * L.c * L.k > (odd ? 8e9 : 2.4e10);
+        return L.c > 32 && L.w > (odd ? 801u : 900u);
     }
 
     // The direct kernel holds about 1,430 TFLOP/s of direct-convolution work

@@ -10,11 +10,11 @@ DIRECT, F2, F4 = 5, 1, 0
 
 
 @pytest.mark.parametrize("c,k,h,w,algo", [
-    (64, 64, 9, 800, DIRECT), (64, 64, 9, 802, F2), (64, 32, 5, 1080, F2), (128, 100, 9, 600, DIRECT), (136, 64, 9, 602, F2),
-    (128, 64, 9, 559, DIRECT), (128, 64, 9, 561, F2), (136, 64, 9, 299, DIRECT), (136, 64, 9, 301, F2), (256, 256, 10, 560, DIRECT),
-    (128, 128, 14, 604, DIRECT), (128, 128, 14, 606, F4), (128, 128, 15, 453, DIRECT), (128, 128, 15, 455, F4),
-    (256, 256, 16, 302, DIRECT), (256, 256, 16, 304, F4), (256, 256, 16, 225, DIRECT), (256, 256, 16, 229, F4),
-    (40, 24, 6, 1400, F2)])
+    (64, 64, 9, 900, DIRECT), (64, 64, 9, 902, F2), (40, 32, 5, 1080, F2), (32, 40, 5, 1080, DIRECT), (8, 8, 5, 1079, DIRECT),
+    (256, 64, 9, 801, DIRECT), (256, 64, 9, 803, F2), (256, 256, 10, 900, DIRECT), (128, 128, 14, 640, DIRECT),
+    (128, 128, 14, 642, F4), (128, 128, 15, 639, DIRECT), (128, 128, 15, 641, F4), (256, 256, 16, 604, DIRECT),
+    (256, 256, 16, 606, F4), (256, 256, 16, 349, DIRECT), (256, 256, 16, 351, F4), (256, 512, 14, 426, DIRECT),
+    (256, 512, 14, 428, F4), (40, 24, 6, 1400, F2)])
 def test_rows(wg, c, k, h, w, algo):
     g = torch.Generator().manual_seed(w)
     x = (torch.rand((2, c, h, w), generator=g) * 2 - 1).half().cuda()
