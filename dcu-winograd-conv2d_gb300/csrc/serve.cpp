@@ -258,6 +258,7 @@ struct Server {
     // unless its 4 x 4 tiles reach past the output (64 x 512 x 14^2: 59.2 against
     // 44.7; 16 x 30^2 53.7 against 48.9; 32 x 20^2 42.0 against 44.8) or the request
     // is small (1 x 56^2: 18.9 against 17.2; 8 x 28^2 26.9 against 28.5).
+    // (So the bits of an image of such a layer depend on its request's size.)
     bool choose_direct(const Layer& L, unsigned n) const {
         if (cfg.algo != CONV2D_ALGO_AUTO || !L.U9 || wide_rows(L)) return false;
         const long long oh = L.h + 2LL * L.p - 2, ow = L.w + 2LL * L.q - 2;

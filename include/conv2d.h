@@ -109,8 +109,10 @@ enum {
  * times the candidates (the reference's three algorithms and the row F(4x3)
  * kernel) on the device, reading the problem's input and weights and writing
  * a scratch output, and keeps the reference rule's pick unless another is
- * more than 3% faster, times weighed by accuracy; the choice is cached per
- * shape (and in WG_CONV2D_TUNE_FILE).  It also times the direct kernel, which
+ * more than 3% faster, times weighed by accuracy (row F(4x3) by 1.04, F(4x3) by
+ * 1.08: of nearly equal candidates the more accurate one; an algorithm asked for
+ * by name runs whatever its time); the choice is cached per shape (and in
+ * WG_CONV2D_TUNE_FILE).  It also times the direct kernel, which
  * calls run where it is faster than that pick (conv2d_get_direct).  On GB300
  * the reference rule's fused F(2x3) pick is several times slower than the
  * alternatives for wide K (e.g. 390 against 101 us for F(4x3) and 82 for the
@@ -124,12 +126,14 @@ typedef struct
     int tile_scaling;    /* F(4x3): per-tile power-of-two scaling of the input transform */
     int f4_points;       /* F(4x3) interpolation points: 0 = {0,+-1,1/2,-2}, 1 = reference {0,+-1,+-2} */
     int filter_policy;   /* 0: transform the filter on the first call, then reuse; 1: every call */
-    int gemm_bn;         /* GEMM output-channel tile: 0 = automatic, else 32/64/128/256 */
+    int gemm_bn;         /* GEMM output-channel tile: 0 = automatic, else 32/64/128/256 (the direct kernel by
+                            name: channels per item, a multiple of 32, + 512 x blocks of 128 positions) */
     long long l2_chunk_bytes; /* non-fused: process images in chunks whose V+M fit this many bytes (0 = one pass) */
     int io_bf16;         /* 1: input, filter and output tensors are bf16 (end to end); F(2x3) then uses bf16
                             operands, F(4x3) fp16 operands with per-tile scaling, both an fp32 M */
     int layout_nhwc;     /* 1: input and output tensors are NHWC (channels last; filter stays KCRS);
-                            non-fused F(2x3)/F(4x3), fp16 tensors, images up to ~250 columns */
+                            non-fused F(2x3)/F(4x3), fp16 tensors, images up to ~250 columns (the direct
+                            kernel up to ~590) */
     int m_fp32;          /* F(4x3) non-fused: 1 stores the GEMM result M in fp32; 0 (default) in 24 bits
                             (each fp32 accumulator rounded to its upper 24 bits: relative rounding
                             2^-17, 3/4 of the fp32 bytes), for NCHW and NHWC tensors alike */
@@ -158,10 +162,12 @@ int conv2d_fp16_ex(const void* param_ptr, void* stream);
 
 /* End-to-end call with HOST buffers: copies host_in (n*c*h*w fp16) to the
  * problem's device input, runs, copies the output to host_out and waits for
- * the stream.  The batch is cut into up to 8 image chunks (at least 6 MB of
- * copies each, or two of at least 2 MB; WG_CONV2D_HOST_CHUNKS / WG_CONV2D_HOST_SIZES override) whose
- * input copies, compute and output copies overlap (two internal copy
- * streams); with pinned host memory the copies run at full link speed. */
+ * the stream.  The batch is cut into up to 8 image chunks of at least 6 MB of
+ * copies each, or two from 4 MB of copies in all where neither direction has
+ * more than two thirds of them (WG_CONV2D_HOST_CHUNKS / WG_CONV2D_HOST_SIZES
+ * override), whose input copies, compute and output copies overlap (two internal
+ * copy streams); a call of one chunk copies on the caller's stream.  With pinned
+ * host memory the copies run at full link speed. */
 int conv2d_fp16_host(const void* param_ptr, const void* host_in, void* host_out, void* stream);
 
 /* `steps` end-to-end calls of the same layer on consecutive host batches
@@ -182,14 +188,19 @@ int conv2d_refresh_filter(const void* param_ptr, void* stream);
 int conv2d_destroy(void* param_ptr);
 
 /* Selected algorithm (CONV2D_ALGO_4X3_NON_FUSED .. CONV2D_ALGO_2X3_FUSED,
- * CONV2D_ALGO_4X3_ROW, or CONV2D_ALGO_DIRECT when asked for by name), or -1. */
+ * CONV2D_ALGO_4X3_ROW, or CONV2D_ALGO_DIRECT when asked for by name), or -1.
+ * Under CONV2D_ALGO_AUTO it and the blob's `kernel` field name the pick among the
+ * Winograd algorithms also where calls run the direct kernel: ask
+ * conv2d_get_direct. */
 int conv2d_get_algo(const void* param_ptr);
 
 /* 1 when conv2d calls of this blob run the direct kernel: asked for as
  * CONV2D_ALGO_DIRECT, or, under CONV2D_ALGO_AUTO, measured faster than the
  * selected algorithm (which conv2d_get_algo still reports, and whose filter
  * files conv2d_plan_save and _load still use; after a load calls of the blob run
- * that algorithm, from the file's filter).  0 otherwise, -1 for a bad blob. */
+ * that algorithm, from the file's filter).  0 otherwise, -1 for a bad blob.
+ * The blob's U_d is then the direct kernel's filter and V_d and M_d are null;
+ * WG_CONV2D_KEEP_WORKSPACE=1 has the selected algorithm run. */
 int conv2d_get_direct(const void* param_ptr);
 
 /* Device workspace bytes held by the blob (after conv2d_plan_load into a blob
@@ -224,8 +235,10 @@ void conv2d_autotune_clear(void);
 
 /* Many convolutions of different shapes run together: one grouped launch per
  * kernel family covers every problem (the GEMM as one persistent work queue of
- * (problem, element, tile block, channel block) items), captured once into a
- * CUDA graph and replayed.  Each problem's algorithm and GEMM tile follow
+ * (problem, element, tile block, channel block) items, the problems that run the
+ * direct kernel as one queue of theirs, or more where very wide rows and many
+ * output channels do not share a ring), captured once into a CUDA graph and
+ * replayed.  Each problem's algorithm and GEMM tile follow
  * `opt->algo` (CONV2D_ALGO_AUTO: per-shape autotuner).  Workspaces and
  * transformed filters stay resident until conv2d_batch_destroy. */
 typedef struct conv2d_batch conv2d_batch_t;
@@ -234,6 +247,8 @@ int conv2d_batch_create(const problem_t* problems, int count, const conv2d_optio
 int conv2d_batch_run(conv2d_batch_t* batch, void* stream);
 /* The same problems, one conv2d call after another (for comparison). */
 int conv2d_batch_run_percall(conv2d_batch_t* batch, void* stream);
+/* A problem's algorithm, as conv2d_get_algo reports it, and the output-channel
+ * tile that its plan runs with: the direct kernel's where the plan runs that. */
 int conv2d_batch_info(const conv2d_batch_t* batch, int index, int* algo, int* gemm_bn);
 /* Kernel launches of one grouped (grouped != 0) or per-call run. */
 int conv2d_batch_launches(const conv2d_batch_t* batch, int grouped);
@@ -242,13 +257,19 @@ int conv2d_batch_destroy(conv2d_batch_t* batch);
 
 /* ---- serving (no counterpart in the reference) ---------------------------- */
 
-/* A request loop over resident layers: filters transformed once (F(2x3) and
- * F(4x3)) and kept on the device; requests admitted in arrival order while
- * their Winograd-domain workspace fits in an arena of `hbm_budget_bytes`;
+/* A request loop over resident layers: filters kept on the device in the forms
+ * of the direct kernel, F(2x3) and F(4x3); requests admitted in arrival order
+ * while the Winograd-domain workspace of their layer and size (reserved also where
+ * they run the direct kernel) fits in an arena of `hbm_budget_bytes`;
  * admitted requests packed into batches of at most `max_batch` and launched
  * as grouped kernels on one of `slots` streams, so batches overlap on the
  * device (continuous batching).  A request's result does not depend on what
- * else is in its batch.  per_request = 1 gives the plain per-call path: each
+ * else is in its batch.  It may depend on its own number of images: under
+ * CONV2D_ALGO_AUTO a layer of 512 or more channels in and out, of images of 14^2
+ * or more into which 4x4 tiles fit within 5%, runs the direct kernel for requests
+ * below 4,096 output pixels and F(4x3) from there on (2.1e-4 and 2.0e-3 relative
+ * error); an `algo` other than AUTO runs the same kernels for
+ * every size.  per_request = 1 gives the plain per-call path: each
  * request's own kernels queued at submission on one stream. */
 typedef struct conv2d_server conv2d_server_t;
 typedef struct
@@ -317,7 +338,7 @@ int conv2d_server_destroy(conv2d_server_t* server);
  * run the loaded one. */
 int conv2d_plan_save(const void* param, const char* path);
 int conv2d_plan_load(const void* param, const char* path);
-/* A server's resident layers (both transformed filters of each) to a file,
+/* A server's resident layers (the filters of each in every form) to a file,
  * and back into a server: the loaded layers get indices first_layer ..
  * first_layer + count - 1, in the saved order. */
 int conv2d_server_save_layers(conv2d_server_t* server, const char* path);
