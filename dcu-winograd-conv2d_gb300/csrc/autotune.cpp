@@ -6,10 +6,11 @@
 // scratch output memory and timed on the device the first time a shape is seen; the winner is cached per shape and, when
 // WG_CONV2D_TUNE_FILE names a file, persisted there so later processes make
 // the same choice without measuring.  The reference selection wins unless
-// another candidate is more than 3% faster, so noise between nearly equal
-// candidates cannot flip the choice from run to run.  The direct kernel is
-// timed as well: where it is faster than the winner, calls run it.  Times are
-// weighed by accuracy (accuracy_weight).
+// another candidate is more than 3% faster, and of candidates that the
+// measurement does not tell apart the more accurate one (pick_tuned), so noise
+// between nearly equal candidates seldom flips the choice from run to run.  The
+// direct kernel is timed as well: where it is faster than the winner, calls run
+// it.  Times are weighed by accuracy (accuracy_weight).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -18,6 +19,7 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <numeric>
 #include <tuple>
 #include <vector>
 
@@ -51,6 +53,14 @@ constexpr double kSustainedFlops = 1.48e15;
 float accuracy_weight(int algo) {
     return algo == CONV2D_ALGO_4X3_NON_FUSED ? 1.08f : algo == CONV2D_ALGO_4X3_ROW ? 1.04f : 1.f;
 }
+
+// A candidate this close, in ms, to the fastest one counts as equal to it: what
+// the measurement of single calls does not tell apart.  4x512x28^2 -> 256 (direct
+// 22.1 us, F(4x3) 20.3, weighed 21.9) ran the direct kernel in 6 of 10 plans and
+// F(4x3), ten times its error, in 4; 2x512x28^2 -> 128 (F(2x3) 18.8, F(4x3) 18.0,
+// weighed 19.4) F(2x3) in 2 and F(4x3) in 8.  Now the first runs
+// direct in 10 of 10, the second F(2x3).
+constexpr float kTimingStepMs = 1.05e-3f;
 
 // In the tune file the algorithm's number carries the direct kernel's flag.
 constexpr int kDirectFlag = 16;
@@ -97,9 +107,11 @@ void append_file_locked(const Key& kk, const Choice& ch) {
     std::fclose(fp);
 }
 
-// Device time of one call of a candidate plan (best of 8 after a warm-up; with
-// the best of 3 a choice now and then took a GEMM tile a fifth slower), or a
-// negative value when the candidate cannot be planned.
+// Device time of one call of a candidate plan, or a negative value when the
+// candidate cannot be planned: the mean of the lower 5 in 8 of 16 calls after a
+// warm-up (of 8 that take over 5 ms in all).  Event times go in steps of about 1
+// us: the best of 8 calls of 20 us came out up to 2 us apart from one measurement
+// to the next, this mean 0.3.
 float time_candidate(const problem_t& pr, conv2d_options_t opt, int algo, int bn, void* scratch_out,
                      cudaStream_t s) {
     problem_t p = pr;
@@ -112,23 +124,52 @@ float time_candidate(const problem_t& pr, conv2d_options_t opt, int algo, int bn
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
-    float best = -1.f;
-    for (int rep = 0; rep < 8; ++rep) {
+    std::vector<float> times;
+    float total = 0.f;
+    for (int rep = 0; rep < 16 && !(rep >= 8 && total > 5.f); ++rep) {
         cudaEventRecord(a, s);
         if (pl.run(s) != CONV2D_OK) break;
         cudaEventRecord(b, s);
         if (cudaEventSynchronize(b) != cudaSuccess) break;
         float ms = 0.f;
         cudaEventElapsedTime(&ms, a, b);
-        if (best < 0.f || ms < best) best = ms;
+        times.push_back(ms);
+        total += ms;
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     cudaStreamSynchronize(s);
-    return best;
+    if (times.empty()) return -1.f;
+    std::sort(times.begin(), times.end());
+    times.resize((times.size() * 5 + 7) / 8);
+    return std::accumulate(times.begin(), times.end(), 0.f) / static_cast<float>(times.size());
 }
 
 }  // namespace
+
+void pick_tuned(const TunedTime* t, int n, int fallback, float direct_ms, double direct_flops, TunedTime* best, bool* direct) {
+    *best = TunedTime{fallback, 0, -1.f};
+    *direct = false;
+    TunedTime ref{fallback, 0, -1.f};
+    float least = -1.f;   // of the weighed times
+    const auto weighed = [](const TunedTime& x) { return x.ms * accuracy_weight(x.algo); };
+    for (int i = 0; i < n; ++i) {
+        if (least < 0.f || weighed(t[i]) < least) least = weighed(t[i]);
+        if (t[i].algo == fallback && (ref.ms < 0.f || t[i].ms < ref.ms)) ref = t[i];
+    }
+    if (n == 0) return;
+    // the most accurate of those as fast as the fastest, the fastest of these
+    for (int i = 0; i < n; ++i) {
+        if (weighed(t[i]) > least + kTimingStepMs) continue;
+        const float wi = accuracy_weight(t[i].algo), wb = accuracy_weight(best->algo);
+        if (best->ms < 0.f || wi < wb || (wi == wb && t[i].ms < best->ms)) *best = t[i];
+    }
+    // the reference rule's pick unless it is more than 3% slower or the less accurate
+    if (ref.ms > 0.f && accuracy_weight(fallback) <= accuracy_weight(best->algo) && weighed(*best) > weighed(ref) / 1.03f) *best = ref;
+    if (direct_ms <= 0.f) return;
+    const double sustained_ms = direct_flops / kSustainedFlops * 1e3;
+    *direct = std::max(static_cast<double>(direct_ms), sustained_ms) < std::max(least + kTimingStepMs, weighed(*best));
+}
 
 int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallback, int* algo_out, int* bn_out,
                     bool* direct_out) {
@@ -166,29 +207,21 @@ int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallba
         cands.push_back({a, bn0});
         if (pr.k > 128) cands.push_back({a, bn0 == 256 ? 128 : 256});
     }
-    Choice best{fallback, 0, -1.f, false};
-    float ref_ms = -1.f;
-    int ref_bn = 0;
+    std::vector<TunedTime> times;
     for (const Cand& cd : cands) {
         const float ms = time_candidate(pr, opt, cd.algo, cd.bn, scratch, s);
-        if (ms < 0.f) continue;
-        const float weighed = ms * accuracy_weight(cd.algo);
-        if (cd.algo == fallback && (ref_ms < 0.f || weighed < ref_ms)) {
-            ref_ms = weighed;
-            ref_bn = cd.bn;
-        }
-        if (best.ms < 0.f || weighed < best.ms) best = Choice{cd.algo, cd.bn, weighed, false};
+        if (ms >= 0.f) times.push_back({cd.algo, cd.bn, ms});
     }
-    const float direct_ms = best.ms < 0.f ? -1.f : time_candidate(pr, opt, CONV2D_ALGO_DIRECT, 0, scratch, s);
+    const float direct_ms = times.empty() ? -1.f : time_candidate(pr, opt, CONV2D_ALGO_DIRECT, 0, scratch, s);
     cudaStreamDestroy(s);
     cudaFree(scratch);
-    if (ref_ms > 0.f && best.ms > 0.f && best.ms > ref_ms / 1.03f) best = Choice{fallback, ref_bn, ref_ms, false};
-    if (best.ms < 0.f) best = Choice{fallback, 0, 0.f, false};
     // the kernel multiplies whole rows with their padding, 16 channels and 32 filters at a time
     const double positions = pr.n * (pr.h + std::max<double>(pr.p, 2.0 * pr.p - 2)) * (pr.w + std::max<double>(pr.q, 2.0 * pr.q - 2));
     const double flops = 18.0 * positions * ((pr.c + 15) / 16 * 16) * ((pr.k + 31) / 32 * 32);
-    best.direct = direct_ms > 0.f && std::max(static_cast<double>(direct_ms), flops / kSustainedFlops * 1e3) < best.ms;
-    best.ms /= accuracy_weight(best.algo);
+    TunedTime pick;
+    bool direct = false;
+    pick_tuned(times.data(), static_cast<int>(times.size()), fallback, direct_ms, flops, &pick, &direct);
+    const Choice best{pick.algo, pick.bn, std::max(pick.ms, 0.f), direct};
     {
         std::lock_guard<std::mutex> lk(g_mu);
         if (g_cache.find(kk) == g_cache.end()) {

@@ -162,5 +162,14 @@ int set_last_error(int status, const char* msg);
 // *direct: the direct kernel ran faster than that choice.
 int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallback, int* algo, int* bn, bool* direct);
 void autotune_clear();
+// The tuner's choice from measured times: *best among the n Winograd candidates
+// that could be planned (ms < 0, the fallback, with none), *direct whether calls
+// run the direct kernel (direct_ms <= 0: it cannot be planned; direct_flops: its
+// operations, padding included).
+struct TunedTime {
+    int algo, bn;
+    float ms;
+};
+void pick_tuned(const TunedTime* t, int n, int fallback, float direct_ms, double direct_flops, TunedTime* best, bool* direct);
 
 }  // namespace wg
