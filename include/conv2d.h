@@ -227,7 +227,8 @@ int conv2d_select_reference(const problem_t* problem);
  * CONV2D_ALGO_AUTO makes it: measured on the device the first time a shape is
  * seen (candidates run on scratch output memory, reading the problem's input
  * and weights), then cached; WG_CONV2D_TUNE_FILE persists the cache.  The
- * reference selection is kept unless another candidate is >3% faster. */
+ * reference selection is kept unless another candidate is >3% faster; of
+ * candidates that the measurement does not tell apart the most accurate runs. */
 int conv2d_autotune(const problem_t* problem, const conv2d_options_t* opt, int* algo, int* gemm_bn);
 void conv2d_autotune_clear(void);
 
