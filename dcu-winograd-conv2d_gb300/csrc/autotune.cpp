@@ -19,7 +19,6 @@
 #include <cstring>
 #include <map>
 #include <mutex>
-#include <numeric>
 #include <tuple>
 #include <vector>
 
@@ -54,13 +53,13 @@ float accuracy_weight(int algo) {
     return algo == CONV2D_ALGO_4X3_NON_FUSED ? 1.08f : algo == CONV2D_ALGO_4X3_ROW ? 1.04f : 1.f;
 }
 
-// A candidate this close, in ms, to the fastest one counts as equal to it: what
-// the measurement of single calls does not tell apart.  4x512x28^2 -> 256 (direct
-// 22.1 us, F(4x3) 20.3, weighed 21.9) ran the direct kernel in 6 of 10 plans and
-// F(4x3), ten times its error, in 4; 2x512x28^2 -> 128 (F(2x3) 18.8, F(4x3) 18.0,
-// weighed 19.4) F(2x3) in 2 and F(4x3) in 8.  Now the first runs
-// direct in 10 of 10, the second F(2x3).
-constexpr float kTimingStepMs = 1.05e-3f;
+// A candidate this close, in ms, to the fastest one counts as equal to it, so that
+// near ties go the same way in every plan.  By the best of 8 single calls
+// 4x512x28^2 -> 256 (direct 15.5 us, F(4x3) 14.2, weighed 15.3) ran the direct
+// kernel in 6 of 10 plans and F(4x3), ten times its error, in 4; 2x512x28^2 -> 128
+// (F(2x3) 12.8, F(4x3) 12.1, weighed 13.1) F(2x3) in 2 and F(4x3) in 8.  Now the
+// first runs direct in 10 of 10, the second F(2x3).
+constexpr float kTieMs = 0.7e-3f;
 
 // In the tune file the algorithm's number carries the direct kernel's flag.
 constexpr int kDirectFlag = 16;
@@ -108,10 +107,12 @@ void append_file_locked(const Key& kk, const Choice& ch) {
 }
 
 // Device time of one call of a candidate plan, or a negative value when the
-// candidate cannot be planned: the mean of the lower 5 in 8 of 16 calls after a
-// warm-up (of 8 that take over 5 ms in all).  Event times go in steps of about 1
-// us: the best of 8 calls of 20 us came out up to 2 us apart from one measurement
-// to the next, this mean 0.3.
+// candidate cannot be planned: after a warm-up four times 8 calls back to back
+// (once, if they take over 10 ms), the mean of the faster two.  Event times go in
+// steps of about 1 us: the best of 8 single calls of 20 us came out up to 2 us
+// apart from one plan to the next, and held the launch of the first kernel, which
+// calls in a program overlap (4x512x28^2 -> 256 direct 21-22 us by itself, 15.5 among
+// others; F(4x3), of three kernels, 19-20 and 14.2).
 float time_candidate(const problem_t& pr, conv2d_options_t opt, int algo, int bn, void* scratch_out,
                      cudaStream_t s) {
     problem_t p = pr;
@@ -124,25 +125,24 @@ float time_candidate(const problem_t& pr, conv2d_options_t opt, int algo, int bn
     cudaEvent_t a, b;
     cudaEventCreate(&a);
     cudaEventCreate(&b);
+    constexpr int kCalls = 8;
     std::vector<float> times;
-    float total = 0.f;
-    for (int rep = 0; rep < 16 && !(rep >= 8 && total > 5.f); ++rep) {
-        cudaEventRecord(a, s);
-        if (pl.run(s) != CONV2D_OK) break;
-        cudaEventRecord(b, s);
-        if (cudaEventSynchronize(b) != cudaSuccess) break;
+    bool ok = true;
+    for (int rep = 0; rep < 4 && ok; ++rep) {
+        ok = cudaEventRecord(a, s) == cudaSuccess;
+        for (int i = 0; i < kCalls && ok; ++i) ok = pl.run(s) == CONV2D_OK;
+        ok = ok && cudaEventRecord(b, s) == cudaSuccess && cudaEventSynchronize(b) == cudaSuccess;
         float ms = 0.f;
-        cudaEventElapsedTime(&ms, a, b);
-        times.push_back(ms);
-        total += ms;
+        ok = ok && cudaEventElapsedTime(&ms, a, b) == cudaSuccess;
+        if (ok) times.push_back(ms / kCalls);
+        if (ms > 10.f) break;
     }
     cudaEventDestroy(a);
     cudaEventDestroy(b);
     cudaStreamSynchronize(s);
     if (times.empty()) return -1.f;
     std::sort(times.begin(), times.end());
-    times.resize((times.size() * 5 + 7) / 8);
-    return std::accumulate(times.begin(), times.end(), 0.f) / static_cast<float>(times.size());
+    return times.size() == 1 ? times[0] : (times[0] + times[1]) / 2;
 }
 
 }  // namespace
@@ -160,7 +160,7 @@ void pick_tuned(const TunedTime* t, int n, int fallback, float direct_ms, double
     if (n == 0) return;
     // the most accurate of those as fast as the fastest, the fastest of these
     for (int i = 0; i < n; ++i) {
-        if (weighed(t[i]) > least + kTimingStepMs) continue;
+        if (weighed(t[i]) > least + kTieMs) continue;
         const float wi = accuracy_weight(t[i].algo), wb = accuracy_weight(best->algo);
         if (best->ms < 0.f || wi < wb || (wi == wb && t[i].ms < best->ms)) *best = t[i];
     }
@@ -168,7 +168,7 @@ void pick_tuned(const TunedTime* t, int n, int fallback, float direct_ms, double
     if (ref.ms > 0.f && accuracy_weight(fallback) <= accuracy_weight(best->algo) && weighed(*best) > weighed(ref) / 1.03f) *best = ref;
     if (direct_ms <= 0.f) return;
     const double sustained_ms = direct_flops / kSustainedFlops * 1e3;
-    *direct = std::max(static_cast<double>(direct_ms), sustained_ms) < std::max(least + kTimingStepMs, weighed(*best));
+    *direct = std::max(static_cast<double>(direct_ms), sustained_ms) < std::max(least + kTieMs, weighed(*best));
 }
 
 int autotune_choose(const problem_t& pr, const conv2d_options_t& opt, int fallback, int* algo_out, int* bn_out,

@@ -54,12 +54,13 @@ def pick(wg, tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("f4,direct", [(19.1, 21.1), (19.1, 21.5), (20.1, 21.1), (20.1, 22.1)])
-def test_direct_where_the_measurement_does_not_tell(pick, f4, direct):
-    assert pick(F4, direct, [(F4, 256, f4), (F2, 256, f4 + 2.1), (ROW, 0, 50.0)])[2]
+@pytest.mark.parametrize("f4,direct,runs", [(14.2, 15.5, True), (14.2, 16.0, True), (14.2, 16.1, False), (40.0, 43.8, True),
+                                            (40.0, 44.0, False)])
+def test_direct_in_a_near_tie(pick, f4, direct, runs):
+    assert pick(F4, direct, [(F4, 256, f4), (F2, 256, 1.5 * f4), (ROW, 0, 3 * f4)])[2] == runs
 
 
-@pytest.mark.parametrize("f2,f4,algo", [(17.4, 17.4, F2), (18.4, 17.4, F2), (17.4, 18.4, F2), (19.6, 17.4, F2), (21.0, 17.4, F4)])
+@pytest.mark.parametrize("f2,f4,algo", [(12.1, 12.1, F2), (12.8, 12.1, F2), (12.1, 12.8, F2), (13.7, 12.1, F2), (13.9, 12.1, F4)])
 def test_more_accurate_of_two_alike(pick, f2, f4, algo):
     # whichever of the two the reference rule names
     for fallback in (F4, F2):
